@@ -27,7 +27,7 @@
 //
 // Launch: a candidate pass (one thread per (OM, element), warp-aggregated
 // counts per (event, OM)), a scan into per-(event, OM) pair segments and a
-// list of 32-pair chunks, a second candidate pass listing the pairs, then a
+// list of pair chunks (up to 32 pairs), a second candidate pass listing the pairs, then a
 // persistent grid over the chunks: warp 0 forms each pair's frame, the CTA
 // lists the (pair, panel, piece) work, spreads (piece x wavelength node) over
 // its threads, accumulates bins in shared memory and the charge by a block
@@ -39,7 +39,14 @@
 
 namespace lh {
 
-constexpr int kO0Chunk = 32;
+constexpr int kO0Chunk = 32;  // most pairs per chunk
+// Pairs per chunk: as many as still give this many chunks (16 per SM), 1 to
+// kO0Chunk. A pair's cost varies by orders of magnitude (an OM near the track
+// has its arrivals cut at many bin edges), so chunks of 32 left one shower of
+// 2000 elements x 48 OMs on a few SMs: 2.95 ms against 0.35 ms with this rule;
+// eight showers of 500-50000 elements x 384 OMs: 2.38 against 1.72 ms (1.91 ms
+// with 8 or 64 chunks per SM: too uneven, too many chunk starts).
+constexpr int kO0ChunkTarget = 16 * 148;
 constexpr int kO0Threads = 256;
 constexpr int kO0MaxOrder = 64;
 constexpr int kO0MaxPanels = 128;
@@ -249,7 +256,7 @@ struct O0Work {
   int32_t* pairs;     // [pair capacity] global element index
   int2* chunks;       // [chunk capacity] (event * n_om + om, chunk)
   uint32_t* mask;     // [pair capacity / 32] candidate bits of the counting pass
-  int32_t* n_chunks;  // [2]: the chunk count, then the next chunk to take
+  int32_t* n_chunks;  // [3]: the chunk count, the next chunk to take, the pairs per chunk
   int64_t pair_capacity, chunk_capacity;
 };
 
@@ -296,20 +303,27 @@ __global__ void order0_candidates_kernel(const lh_order0_optics O, const lh_orde
   if (!fill && flags) atomicOr(reinterpret_cast<unsigned*>(B.status), flags);
 }
 
-// Single CTA: pair offsets per (event, OM) and the list of 32-pair chunks.
+// Single CTA: pair offsets per (event, OM), the chunk size and the chunk list.
 __global__ void __launch_bounds__(1024) order0_scan_kernel(int32_t n_keys, O0Work W) {
   __shared__ int32_t warp_sum[32], warp_chunks[32];
-  __shared__ int32_t carry, carry_chunks;
+  __shared__ int32_t carry, carry_chunks, all_pairs;
   if (threadIdx.x == 0) {
     carry = 0;
     carry_chunks = 0;
+    all_pairs = 0;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int32_t mine = 0;
+  for (int key = threadIdx.x; key < n_keys; key += blockDim.x) mine += W.counts[key];
+  for (int off = 16; off > 0; off >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, off);
+  if (lane == 0) atomicAdd(&all_pairs, mine);
+  __syncthreads();
+  const int32_t chunk = min(kO0Chunk, max(1, all_pairs / kO0ChunkTarget));
   for (int base = 0; base < n_keys; base += blockDim.x) {
     const int key = base + threadIdx.x;
     const int32_t c = key < n_keys ? W.counts[key] : 0;
-    const int32_t ch = (c + kO0Chunk - 1) / kO0Chunk;
+    const int32_t ch = (c + chunk - 1) / chunk;
     int32_t v = c, h = ch;
     for (int off = 1; off < 32; off <<= 1) {
       const int32_t a = __shfl_up_sync(0xffffffffu, v, off);
@@ -357,6 +371,7 @@ __global__ void __launch_bounds__(1024) order0_scan_kernel(int32_t n_keys, O0Wor
   if (threadIdx.x == 0) {
     W.n_chunks[0] = carry_chunks;
     W.n_chunks[1] = 0;
+    W.n_chunks[2] = chunk;
   }
 }
 
@@ -446,6 +461,7 @@ order0_kernel(const lh_order0_optics O, const lh_order0_batch B, const O0Work W,
   double pmin, pmax;
   o0_phase_range(O, pmin, pmax);
   const int total_chunks = min(*W.n_chunks, (int)W.chunk_capacity);
+  const int chunk_pairs = W.n_chunks[2];
   unsigned long long evaluations = 0;  // float32 integrand nodes of this thread
   // CTAs take chunks from a counter: one that drew a heavy chunk does not
   // hold back the chunks dealt to it after
@@ -458,8 +474,8 @@ order0_kernel(const lh_order0_optics O, const lh_order0_batch B, const O0Work W,
   const int2 entry = W.chunks[chunk];
   const int ev = entry.x / O.n_om;
   const int om = entry.x - ev * O.n_om;
-  const int p_begin = W.offsets[entry.x] + entry.y * kO0Chunk;
-  const int p_end = min(W.offsets[entry.x] + W.counts[entry.x], p_begin + kO0Chunk);
+  const int p_begin = W.offsets[entry.x] + entry.y * chunk_pairs;
+  const int p_end = min(W.offsets[entry.x] + W.counts[entry.x], p_begin + chunk_pairs);
   if (want_bins)
     for (int k = tid; k < nb; k += blockDim.x) sbins[k] = 0.0;
   if (tid == 0) S.n_combos = 0;
@@ -873,7 +889,9 @@ static O0Work o0_layout(const lh_order0_optics& O, const lh_order0_batch& B, uns
   O0Work W{};
   const int64_t keys = (int64_t)B.n_events * O.n_om;
   W.pair_capacity = B.n_elements * O.n_om;
-  W.chunk_capacity = W.pair_capacity / kO0Chunk + keys;
+  // chunks of fewer than kO0Chunk pairs come to at most 2 kO0ChunkTarget, and
+  // every (event, OM) adds at most one partly filled chunk
+  W.chunk_capacity = W.pair_capacity / kO0Chunk + 2 * kO0ChunkTarget + keys;
   size_t off = 0;
   auto take = [&](size_t n) {
     unsigned char* p = base ? base + off : nullptr;

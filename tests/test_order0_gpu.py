@@ -110,6 +110,30 @@ def test_batched_events_equal_alone_and_ragged():
                   g["rays8_charge"], g["rays8_bins"])
 
 
+@pytest.mark.parametrize("pairs", [1, 4735, 4736, 75776, 80000])
+def test_chunk_sizes(pairs):
+    """Chunks hold 1 pair below 2 x 2368 candidate pairs and 32 from 32 x 2368 on: the
+    same events on both sides of either edge (sums in float64, so to 1e-12)."""
+    from lighthit_b200.order0 import order0
+    g, el = fixture()
+    opt = optics_of(g, 2)
+    per_event = len(g["pair_om"])
+    whole = order0(opt, [el], g["origins_ns"][None], g["edges_ns"])
+    copies, rest = divmod(pairs, per_event)
+    # elements in order until their pairs reach the remainder
+    count = np.cumsum(np.bincount(g["pair_element"], minlength=len(el["beta"])))
+    part = {k: v[:int(np.searchsorted(count, rest)) + 1] for k, v in el.items()}
+    events = [part] + [el] * copies
+    out = order0(opt, events, np.repeat(g["origins_ns"][None], len(events), axis=0),
+                 g["edges_ns"])
+    alone = order0(opt, [part], g["origins_ns"][None], g["edges_ns"])
+    for key in ("charge", "bins"):
+        values = out[key].cpu().numpy()
+        for k, ref in enumerate([alone] + [whole] * copies):
+            ref = ref[key][0].cpu().numpy()
+            assert np.abs(values[k] - ref).max() <= 1e-12 * max(ref.max(), 1e-30)
+
+
 def test_fine_bins_and_shifted_clock_vs_oracle():
     """1 ns bins over a shifted window on a subset (many s and phi cuts)."""
     from lighthit_b200.order0 import order0
