@@ -75,10 +75,11 @@ LH_DEVICE unsigned long long global_ns() {
 }
 
 // Returns true when the phase with the given parity completed, false once
-// `limit_ns` of global time have passed (checked every 256 polls).
+// `limit_ns` of global time have passed. The global timer is read only from the
+// 256th poll on: a wait whose phase is complete costs one try_wait.
 LH_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit_ns = kWaitLimitNs) {
   const uint32_t addr = smem_addr(bar);
-  const unsigned long long start = global_ns();
+  unsigned long long start = 0;
   for (unsigned spin = 0; spin < 0x7fffffffu; ++spin) {
     uint32_t done;
     asm volatile(
@@ -89,7 +90,11 @@ LH_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit_ns = kW
         : "r"(addr), "r"(parity)
         : "memory");
     if (done) return true;
-    if ((spin & 255u) == 255u && global_ns() - start > (unsigned long long)limit_ns) return false;
+    if ((spin & 255u) == 255u) {
+      const unsigned long long now = global_ns();
+      if (start == 0) start = now;
+      else if (now - start > (unsigned long long)limit_ns) return false;
+    }
   }
   return false;
 }
@@ -188,6 +193,26 @@ LH_DEVICE void tmem_ld8(uint32_t addr, float (&v)[8]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Two loads of 32 lanes x 32 bits x 4 columns (at `a` and at `b`), one wait.
+LH_DEVICE void tmem_ld4x2(uint32_t a, uint32_t b, float (&va)[4], float (&vb)[4]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(b));
+  // the results pass through the wait, so that nothing reads them before it
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                 "+r"(r[6]), "+r"(r[7])::"memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    va[i] = __uint_as_float(r[i]);
+    vb[i] = __uint_as_float(r[4 + i]);
+  }
 }
 
 // ---------------------------------------------------------------- bf16 split

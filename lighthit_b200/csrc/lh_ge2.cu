@@ -490,57 +490,70 @@ int ge2_batch_launch(const lh_ge2_table& T, const lh_ge2_problem* P, int32_t n, 
 //
 // Layout: M = (band, w) rows in H <= 2 halves of 128 TMEM lanes, each half as
 // a real and an imaginary accumulator; N = channel row x pair columns
-// (column r * kTcSub + i for pair i of a sub-tile). Pairs are bucketed by
-// interval (counting sort); a CTA takes up to kTcPairs pairs of one interval,
-// streams A_jl with one bulk copy per degree (double-buffered) and keeps the
-// pairs' accumulators in registers across degrees.
-constexpr int kTcSub = 8;                   // pairs per MMA sub-tile
-constexpr int kTcSubs = 4;                  // sub-tiles per CTA tile
-constexpr int kTcPairs = kTcSub * kTcSubs;  // pairs per CTA tile
-constexpr int kTcThreads = 256;
+// (column r * P + i for pair i of a group of P pairs). Pairs are bucketed by
+// interval (counting sort); a CTA takes work items (tile of up to three groups
+// of one interval, half) and runs them as a pipeline of warp roles:
+//   MMA       one warp bulk-copies each degree's coefficients of the half into a
+//             ring of kTcAStages stages (48 KB each with three BF16 parts) and
+//             issues the products of (degree, group) into a ring of kTcSlots
+//             TMEM slots (real and imaginary accumulator, 2 x kTcCols columns);
+//   builders  form the B tile of (degree, group) from F and t, three parts, in
+//             a ring of kTcBStages tiles;
+//   epilogue  four warps (TMEM lane quarters) per group multiply its columns by
+//             the channels and keep its pairs' sums in registers across the
+//             degrees.
+// So the MMAs of one (degree, group), 24 of N = 80, run while others are drained
+// and the next coefficients arrive. Measured on 61k pairs (8 showers x 48 OMs,
+// degree 8): 0.77 ms against 2.83 ms for a CTA that built, multiplied and drained
+// sub-tiles of 8 pairs one after another (two such CTAs per SM: issue 26 %,
+// long-scoreboard 7.7 per issue). What bounds it: the epilogue alone takes 0.56 ms
+// (its channel loads 0.2 ms of that), the MMAs and their hand-over 0.5 ms (~50
+// cycles per MMA whatever its N, as each reads 4 KB of A from shared memory), the
+// pipeline without either 0.33 ms. Twenty warps of 96 registers (four groups) spilled in
+// the epilogue's row loop and took 1.1 ms; both halves in one CTA read twice the
+// coefficients (432 KB per work item now) and took 1.3 ms.
 constexpr int kTcK = 32;                                  // K columns (pairs x 4 <= 32)
 constexpr uint32_t kTcTileBytes = 128u * kTcK * 2u;       // one 128 x 32 BF16 operand tile
 constexpr int kTcParts = 3;                               // BF16 parts of a split operand
+constexpr int kTcCols = 80;         // columns of an accumulator: rows x pairs, padded to 16
+constexpr int kTcSlots = 3;         // TMEM slots of 2 x kTcCols columns (480 of 512)
+constexpr int kTcAStages = 3;
+constexpr int kTcBStages = 4;
+constexpr int kTcGroups = 3;                  // most pair groups per tile
+constexpr int kTcEpiWarps = 4 * kTcGroups;    // one warp per group and lane quarter
+constexpr int kTcBuildWarps = 3;
+constexpr int kTcThreads = 32 * (kTcEpiWarps + kTcBuildWarps + 1);  // 16 warps: 128 registers each
+
+// One (OM, point) pair in range.
+struct __align__(16) Ge2TcEntry {
+  const char* rows;      // the point's channel block: band 0, row 0, w 0
+  int64_t band_bytes;    // between bands
+  int32_t pair;          // global pair id
+  float t;               // offset in the interval
+  int32_t pad[2];
+};
 
 struct Ge2TcArgs {
-  const Ge2Slot* slots;
   Ge2Arrays A;
   const uint8_t* packed;        // [interval][degree] blocks: [hi, lo][half][re, im] tiles
-  const int32_t* sorted;        // global pair ids bucketed by interval
-  const int32_t* sorted_slot;   // their problems
-  const int32_t* bucket_start;  // [n_intervals + 1]
-  const int32_t* tile_start;    // [n_intervals + 1]
+  const Ge2TcEntry* entries;    // the pairs in range, bucketed by interval
+  const int4* tiles;            // interval, first entry, pairs, groups
+  const int32_t* n_tiles;
   float2* partial;              // [global pair][band * n_omega + w]
   int32_t* status;
   int passes;                   // 6 split-BF16, 1 BF16
   int halves;                   // H: ceil(bands x omega / 128)
-  int n_pad_max;                // widest sub-tile (16-column multiple)
-  int tmem_cols;                // 256 (two CTAs per SM) or 512
-  int a_buffers;                // 1 with two CTAs per SM, 2 (prefetch) with one
+  int row_bytes;                // between channel rows, the same in every problem
 };
 
-// (A part, B part) of each product of the split mode, largest first.
-__constant__ int kTcPassA[6] = {0, 0, 1, 0, 2, 1};
-__constant__ int kTcPassB[6] = {0, 1, 0, 2, 0, 1};
-
-struct Ge2TcPair {
-  const float2* channels;  // the point's channel block, band 0, channel row 0, w 0
-  int64_t band_stride;     // float2 elements between bands
-  int64_t scale_at;        // g_scale index of band 0
-  int64_t scale_stride;    // between bands
-  int32_t pair;            // global pair id, -1 for an empty place
-  int32_t omega_stride;    // float2 elements between channel rows
-  float t;
-  float pad;
-};
-
-// Whether a table takes the tensor-core path, and its widest sub-tile.
-bool ge2_tc_supported(const lh_ge2_table& T, int& halves, int& n_pad_max) {
+// Whether a table takes the tensor-core path; `pairs` per group: 16 where the
+// widest degree's rows x 16 fit an accumulator's columns, else 8 (up to 9 rows).
+bool ge2_tc_supported(const lh_ge2_table& T, int& halves, int& pairs) {
   const int M = T.n_bands * T.n_omega;
   const int rows_max = 2 * std::min(T.degree, T.max_m) + 1;
   halves = (M + 127) / 128;
-  n_pad_max = (rows_max * kTcSub + 15) & ~15;
-  return M <= 256 && 4 * T.n_pairs <= kTcK && 2 * halves * n_pad_max <= 512;
+  pairs = rows_max * 16 <= kTcCols ? 16 : 8;
+  return M <= 256 && 4 * T.n_pairs <= kTcK && ((rows_max * pairs + 15) & ~15) <= kTcCols;
 }
 
 size_t ge2_tc_block_bytes(const lh_ge2_table& T, int halves) {
@@ -554,6 +567,21 @@ LH_DEVICE void split3_bf16(float x, __nv_bfloat16& hi, __nv_bfloat16& mid, __nv_
   const float r = x - __bfloat162float(hi);
   mid = __float2bfloat16_rn(r);
   lo = __float2bfloat16_rn(r - __bfloat162float(mid));
+}
+
+// Two values' parts, packed (the first in the low half): split3_bf16 of each.
+LH_DEVICE void split3_bf16x2(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  auto pack = [](float x, float y) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  };
+  auto low = [](uint32_t v) { return __uint_as_float(v << 16); };
+  auto high = [](uint32_t v) { return __uint_as_float(v & 0xffff0000u); };
+  hi = pack(a, b);
+  a -= low(hi);
+  b -= high(hi);
+  mid = pack(a, b);
+  lo = pack(a - low(mid), b - high(mid));
 }
 
 // Packs the folded coefficients into the operand tiles (no swizzle, K-major
@@ -590,8 +618,8 @@ __global__ void ge2_tc_pack_kernel(const lh_ge2_table T, int halves, __nv_bfloat
 // Bucket pass 1 and 3 over every pair of every problem, points outermost so
 // that a bucket lists the OMs of one point together: count per interval, then
 // place (warp-aggregated atomics).
-__global__ void ge2_tc_bucket_kernel(const Ge2Slot* slots, Ge2Arrays A, int32_t* counts,
-                                     int32_t* sorted, int32_t* sorted_slot, int fill) {
+__global__ void ge2_tc_bucket_kernel(const Ge2Slot* slots, Ge2Arrays A, int nch, int32_t* counts,
+                                     Ge2TcEntry* entries) {
   const Ge2Slot& S = slots[blockIdx.y];
   const int64_t total = (int64_t)S.P.n_om * S.P.n_points;
   const int64_t rounded = (total + 31) & ~(int64_t)31;
@@ -599,10 +627,10 @@ __global__ void ge2_tc_bucket_kernel(const Ge2Slot* slots, Ge2Arrays A, int32_t*
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < rounded;
        t += (int64_t)gridDim.x * blockDim.x) {
     int j = -1;
-    int64_t idx = 0;
+    int64_t idx = 0, c = 0;
     if (t < total) {
-      const int64_t c = t / S.P.n_om, d = t % S.P.n_om;
-      idx = d * S.P.n_points + c;
+      c = t / S.P.n_om;
+      idx = (t - c * S.P.n_om) * S.P.n_points + c;
       j = A.g_j[S.pair_offset + idx];
     }
     const unsigned peers = __match_any_sync(0xffffffffu, j);
@@ -610,285 +638,537 @@ __global__ void ge2_tc_bucket_kernel(const Ge2Slot* slots, Ge2Arrays A, int32_t*
     int base = 0;
     if (lane == leader && j >= 0) base = atomicAdd(counts + j, __popc(peers));
     base = __shfl_sync(0xffffffffu, base, leader);
-    if (fill && j >= 0) {
-      const int pos = base + __popc(peers & ((1u << lane) - 1u));
-      sorted[pos] = (int32_t)(S.pair_offset + idx);
-      sorted_slot[pos] = (int32_t)blockIdx.y;
+    if (entries && j >= 0) {
+      Ge2TcEntry e;
+      const int64_t point_bytes = (int64_t)nch * S.P.n_omega_channels * (int64_t)sizeof(float2);
+      e.rows = reinterpret_cast<const char*>(S.P.channels) + c * point_bytes;
+      e.band_bytes = S.P.n_points * point_bytes;
+      e.pair = (int32_t)(S.pair_offset + idx);
+      e.t = A.g_t[S.pair_offset + idx];
+      e.pad[0] = e.pad[1] = 0;
+      entries[base + __popc(peers & ((1u << lane) - 1u))] = e;
     }
   }
 }
 
-// Bucket starts, tile starts (kTcPairs pairs per tile) and the fill cursors.
-__global__ void ge2_tc_scan_kernel(int n_intervals, int32_t* counts, int32_t* bucket_start,
-                                   int32_t* tile_start, unsigned long long* units) {
-  if (threadIdx.x != 0) return;
-  int32_t at = 0, tiles = 0;
-  for (int j = 0; j < n_intervals; ++j) {
-    const int32_t c = counts[j];
-    bucket_start[j] = at;
-    tile_start[j] = tiles;
-    counts[j] = at;  // the fill pass counts from the bucket's start
-    at += c;
-    tiles += (c + kTcPairs - 1) / kTcPairs;
+// One CTA: the fill cursors (bucket starts) and the tiles. A tile takes as many
+// groups as still leave every SM two work items (tile, half): more groups share
+// their coefficients, fewer spread a small problem over the SMs.
+__global__ void __launch_bounds__(256)
+ge2_tc_tiles_kernel(int n_intervals, int group_pairs, int halves, int32_t* counts, int4* tiles,
+                    int32_t* n_tiles, unsigned long long* units) {
+  extern __shared__ int32_t s_scan[];  // [n_intervals + 1] bucket starts, then tile starts
+  int32_t* s_start = s_scan;
+  int32_t* s_tile = s_scan + n_intervals + 1;
+  __shared__ int s_per;
+  for (int j = threadIdx.x; j < n_intervals; j += blockDim.x) s_start[j + 1] = counts[j];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int32_t at = 0, tile = 0;
+    for (int j = 0; j < n_intervals; ++j) {
+      const int32_t c = s_start[j + 1];
+      s_start[j] = at;
+      at += c;
+    }
+    s_start[n_intervals] = at;
+    int per = kTcGroups * group_pairs;
+    while (per > group_pairs && (int64_t)at * halves < 2 * 148 * (int64_t)per) per -= group_pairs;
+    for (int j = 0; j < n_intervals; ++j) {
+      s_tile[j] = tile;
+      tile += (s_start[j + 1] - s_start[j] + per - 1) / per;
+    }
+    s_tile[n_intervals] = tile;
+    s_per = per;
+    *n_tiles = tile;
+    if (units) atomicAdd(units, (unsigned long long)at);  // (OM, point) pairs in range
   }
-  bucket_start[n_intervals] = at;
-  tile_start[n_intervals] = tiles;
-  if (units) atomicAdd(units, (unsigned long long)at);  // (OM, point) pairs in range
+  __syncthreads();
+  const int per = s_per;
+  for (int j = threadIdx.x; j < n_intervals; j += blockDim.x) counts[j] = s_start[j];
+  for (int k = threadIdx.x; k < s_tile[n_intervals]; k += blockDim.x) {
+    int lo = 0, hi = n_intervals;  // the bucket: last j with s_tile[j] <= k
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (s_tile[mid] <= k) lo = mid; else hi = mid;
+    }
+    const int first = s_start[lo] + (k - s_tile[lo]) * per;
+    const int count = min(per, s_start[lo + 1] - first);
+    tiles[k] = make_int4(lo, first, count, (count + group_pairs - 1) / group_pairs);
+  }
 }
 
-__global__ void __launch_bounds__(kTcThreads, 2)
+// A work item: half h of a tile, the tile's interval and its entries (the same on
+// every caller).
+struct Ge2TcTile {
+  int h, j, first, count, groups;
+};
+
+LH_DEVICE Ge2TcTile ge2_tc_tile(const Ge2TcArgs& G, int item) {
+  const int tile = item / G.halves;
+  const int4 v = __ldg(G.tiles + tile);
+  return Ge2TcTile{item - tile * G.halves, v.x, v.y, v.z, v.w};
+}
+
+constexpr uint32_t kTcLboA = 128u * 16u, kTcLboB = (uint32_t)kTcCols * 16u;
+
+// The products of one step, the real and the imaginary accumulator in turn (two
+// chains of dependent MMAs instead of one). Descriptors of the parts and K steps
+// are the stage's plus constants (addresses in 16-byte units).
+template <int kPasses>
+LH_DEVICE void ge2_tc_issue(uint32_t d, uint64_t da0, uint64_t db0, uint32_t idesc) {
+  // (A part, B part) of each product of the split mode, largest first
+  constexpr int pass_a[6] = {0, 0, 1, 0, 2, 1}, pass_b[6] = {0, 1, 0, 2, 0, 1};
+#pragma unroll
+  for (int pass = 0; pass < kPasses; ++pass)
+#pragma unroll
+    for (int kk = 0; kk < kTcK / 16; ++kk)
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        const uint64_t da = da0 + (uint64_t)(((pass_a[pass] * 2 + part) * kTcTileBytes +
+                                              kk * 2 * kTcLboA) >> 4);
+        const uint64_t db = db0 + (uint64_t)((pass_b[pass] * kTcCols * kTcK * 2 +
+                                              kk * 2 * kTcLboB) >> 4);
+        tc_mma_bf16(d + (uint32_t)(part * kTcCols), da, db, idesc, pass + kk ? 1u : 0u);
+      }
+}
+
+// One lane of a converged warp (always the same one).
+LH_DEVICE bool elect_one() {
+  uint32_t mine;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(mine));
+  return mine != 0;
+}
+
+// mbar_wait of a whole warp, with one outcome for all its lanes.
+LH_DEVICE bool warp_wait(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
+// A barrier of the four warps of an epilogue group; true when `flag` holds on any.
+LH_DEVICE bool group_sync_or(int group, bool flag) {
+  int any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %2, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, 128, p;\n\t"
+      "selp.b32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(1 + group), "r"((int)flag)
+      : "memory");
+  return any != 0;
+}
+
+struct Ge2TcBars {
+  uint64_t a_full[kTcAStages], a_empty[kTcAStages];
+  uint64_t b_full[kTcBStages], b_empty[kTcBStages];
+  // per group, for even and odd steps: its columns are in TMEM / have been read.
+  // At most two steps of a group are in flight, so a parity names the phase.
+  uint64_t t_full[kTcGroups][2], t_empty[kTcGroups][2];
+  uint64_t drain;
+};
+
+// P pairs per group. Each role walks the same sequence of (work item, degree,
+// group) and counts its stages itself; a wait that runs into its time limit ends
+// that role, and the roles waiting for it then end the same way.
+template <int P>
+__global__ void __launch_bounds__(kTcThreads, 1)
 ge2_tc_kernel(const lh_ge2_table T, const Ge2TcArgs G) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int H = G.halves;
   const int parts = G.passes > 1 ? kTcParts : 1;
-  const uint32_t block_bytes = (uint32_t)kTcParts * H * 2u * kTcTileBytes;
-  const uint32_t load_bytes = (uint32_t)parts * H * 2u * kTcTileBytes;
-  uint8_t* s_a0 = smem;
-  uint8_t* s_a1 = smem + (G.a_buffers > 1 ? load_bytes : 0);
-  __nv_bfloat16* s_b = reinterpret_cast<__nv_bfloat16*>(smem + G.a_buffers * load_bytes);
-  const int b_elems = G.n_pad_max * kTcK;
-  Ge2TcPair* s_pair = reinterpret_cast<Ge2TcPair*>(smem + G.a_buffers * load_bytes +
-                                                   (size_t)parts * b_elems * 2);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_pair + kTcPairs);  // load[2], mma
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 3);
+  const uint32_t a_bytes = (uint32_t)parts * 2u * kTcTileBytes;  // one half's coefficients
+  constexpr int kBElems = kTcCols * kTcK;
+  const uint32_t b_bytes = (uint32_t)parts * kBElems * 2u;
+  uint8_t* s_a = smem;
+  uint8_t* s_b = s_a + kTcAStages * a_bytes;
+  // each pair's channel block per band: [group][band][pair]
+  const char** s_ch = reinterpret_cast<const char**>(s_b + kTcBStages * b_bytes);
+  Ge2TcBars* bars = reinterpret_cast<Ge2TcBars*>(s_ch + kTcGroups * P * T.n_bands);
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   if (tid == 0) {
-    mbar_init(bars + 0, 1);
-    mbar_init(bars + 1, 1);
-    mbar_init(bars + 2, 1);
+    for (int i = 0; i < kTcAStages; ++i) mbar_init(bars->a_full + i, 1), mbar_init(bars->a_empty + i, 1);
+    for (int i = 0; i < kTcBStages; ++i)
+      mbar_init(bars->b_full + i, kTcBuildWarps), mbar_init(bars->b_empty + i, 1);
+    for (int i = 0; i < 2 * kTcGroups; ++i)
+      mbar_init(&bars->t_full[0][0] + i, 1), mbar_init(&bars->t_empty[0][0] + i, 4);
+    mbar_init(&bars->drain, 1);
     fence_barrier_init();
   }
   if (warp == 0) {
-    tmem_alloc(s_tmem, (uint32_t)G.tmem_cols);
+    tmem_alloc(s_tmem, 512);
     tmem_relinquish();
   }
+  // K columns past 4 n_pairs stay zero in every B tile
+  for (int e = tid; e < kTcBStages * (int)b_bytes / 16; e += kTcThreads)
+    reinterpret_cast<uint4*>(s_b)[e] = make_uint4(0u, 0u, 0u, 0u);
+  fence_proxy_async();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  const int L1 = T.degree + 1, W = T.n_omega, M = T.n_bands * W;
-  const int h = warp >> 2, quarter = warp & 3;
-  const int m = h * 128 + quarter * 32 + lane;
-  const bool m_ok = m < M;
-  const int lam = m_ok ? m / W : 0, wq = m_ok ? m % W : 0;
-  const bool reads = h < H;  // warps of a missing half read no TMEM
-  const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
-  const int k_used = 4 * T.n_pairs;
-  const double omega = T.omega[wq];
-  const double inv_speed = 1.0 / T.speed[lam];
-  uint32_t ph_load[2] = {0u, 0u}, ph_mma = 0u;
-  bool failed = false, mma_pending = false;
-  const int n_tiles = G.tile_start[T.n_intervals];
+  const int L1 = T.degree + 1, W = T.n_omega, NB = T.n_bands, M = NB * W;
+  const int n_items = *G.n_tiles * H;
+  bool failed = false;
 
-  for (int tile = blockIdx.x; tile < n_tiles && !failed; tile += gridDim.x) {
-    int lo = 0, hi = T.n_intervals;  // the bucket: last j with tile_start[j] <= tile
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (G.tile_start[mid] <= tile) lo = mid; else hi = mid;
-    }
-    const int j = lo;
-    const int first = G.bucket_start[j] + (tile - G.tile_start[j]) * kTcPairs;
-    const int count = min(kTcPairs, G.bucket_start[j + 1] - first);
-    if (tid < kTcPairs) {
-      Ge2TcPair e{};
-      e.pair = -1;
-      if (tid < count) {
-        const int g = G.sorted[first + tid];
-        const Ge2Slot& S = G.slots[G.sorted_slot[first + tid]];
-        const int64_t idx = g - S.pair_offset;
-        const int c = (int)(idx % S.P.n_points);
-        const int64_t pairs = (int64_t)S.P.n_om * S.P.n_points;
-        e.pair = g;
-        e.t = G.A.g_t[g];
-        e.omega_stride = S.P.n_omega_channels;
-        e.band_stride = (int64_t)S.P.n_points * T.nch * S.P.n_omega_channels;
-        e.channels = reinterpret_cast<const float2*>(S.P.channels) +
-                     (int64_t)c * T.nch * S.P.n_omega_channels;
-        e.scale_at = S.pair_offset * T.n_bands + idx;
-        e.scale_stride = pairs;
-      }
-      s_pair[tid] = e;
-    }
-    if (tid == 0) {  // degree 0 of this interval
-      mbar_expect_tx(bars + 0, load_bytes);
-      bulk_g2s(s_a0, G.packed + (size_t)j * L1 * block_bytes, load_bytes, bars + 0);
-    }
-    __syncthreads();
-    float acc_re[kTcSubs][kTcSub], acc_im[kTcSubs][kTcSub];
-#pragma unroll
-    for (int s = 0; s < kTcSubs; ++s)
-#pragma unroll
-      for (int i = 0; i < kTcSub; ++i) acc_re[s][i] = acc_im[s][i] = 0.f;
-
-    for (int l = 0; l < L1 && !failed; ++l) {
-      const int buf = G.a_buffers > 1 ? (l & 1) : 0;
-      uint8_t* s_a = buf ? s_a1 : s_a0;
-      const int keep = min(l, T.max_m), nr = 2 * keep + 1, row0 = T.starts[l];
-      const int n_cols = nr * kTcSub, n_pad = (n_cols + 15) & ~15;
-      if (G.a_buffers > 1 && tid == 0 && l + 1 < L1) {
-        // the next degree into the other buffer (its MMAs are done)
-        mbar_expect_tx(bars + (buf ^ 1), load_bytes);
-        bulk_g2s(buf ? s_a0 : s_a1, G.packed + ((size_t)j * L1 + l + 1) * block_bytes,
-                 load_bytes, bars + (buf ^ 1));
-      }
-      bool ok = mbar_wait(bars + buf, ph_load[buf]);
-      ph_load[buf] ^= 1u;
-      if (__syncthreads_or(!ok)) { failed = true; break; }
-#pragma unroll
-      for (int s = 0; s < kTcSubs; ++s) {
-        if (failed) continue;
-        if (s * kTcSub >= count) continue;  // the same for the whole CTA
-        // B of sub-tile s: column n = r * kTcSub + i, K index k = 4 p + q
-        for (int e = tid; e < n_pad * kTcK; e += kTcThreads) {
-          const int n = e / kTcK, k = e % kTcK;
-          float v = 0.f;
-          if (n < n_cols && k < k_used) {
-            const Ge2TcPair& P = s_pair[s * kTcSub + n % kTcSub];
-            if (P.pair >= 0) {
-              const int r = n / kTcSub, pp = k >> 2, q = k & 3;
-              float power = 1.f;
-              for (int u = q; u < 3; ++u) power *= P.t;
-              v = G.A.g_F[((int64_t)P.pair * T.nch + row0 + r) * T.n_pairs + pp] * power;
-            }
-          }
-          __nv_bfloat16 bh, bm, bl;
-          split3_bf16(v, bh, bm, bl);
-          const int off = ((k >> 3) * n_pad + n) * 8 + (k & 7);
-          s_b[off] = bh;
-          if (parts > 1) {
-            s_b[b_elems + off] = bm;
-            s_b[2 * b_elems + off] = bl;
-          }
+  if (warp < kTcEpiWarps) {
+    // ---- epilogue: group g, TMEM lanes quarter * 32 + lane
+    const int quarter = warp & 3, g = warp >> 2;
+    const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+    const int rows = T.starts[T.degree] + 2 * min(T.degree, T.max_m) + 1;  // over all degrees
+    const char** table = s_ch + g * P * NB;
+    uint32_t before = 0;  // (degree, group) steps of the items before
+    uint32_t taken = 0;   // this group's steps so far
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+      const Ge2TcTile t = ge2_tc_tile(G, item);
+      const int cnt = min(P, t.count - g * P);
+      if (cnt > 0) {
+        const int m0 = t.h * 128 + quarter * 32, m = m0 + lane;
+        const bool m_ok = m < M;
+        const bool reads = m0 < M;  // warps without a row read no TMEM
+        const int lam = m_ok ? m / W : 0, wq = m_ok ? m % W : 0;
+        // the table of the item before has been read; a wait that gave up ends
+        // all four warps here
+        if (group_sync_or(g, failed)) { failed = true; break; }
+        for (int e = quarter * 32 + lane; e < P * NB; e += 128) {
+          // places past the last pair repeat the first: computed, not written
+          const int band = e / P, i = e - band * P;
+          const Ge2TcEntry& q = G.entries[t.first + g * P + (i < cnt ? i : 0)];
+          table[e] = q.rows + band * q.band_bytes;
         }
-        fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core
-        __syncthreads();
-        tc_fence_after();
-        if (tid == 0) {
-          const uint32_t idesc = instr_desc_bf16_f32(128, n_pad);
-          const uint32_t lbo_a = 128u * 16u, lbo_b = (uint32_t)n_pad * 16u;
-          for (int hh = 0; hh < H; ++hh)
-            for (int part = 0; part < 2; ++part) {
-              const uint32_t d = tmem + (uint32_t)((hh * 2 + part) * n_pad);
-              int first_mma = 1;
-              for (int pass = 0; pass < G.passes; ++pass) {
-                const uint8_t* pa =
-                    s_a + (size_t)((kTcPassA[pass] * H + hh) * 2 + part) * kTcTileBytes;
-                const uint8_t* pb =
-                    reinterpret_cast<const uint8_t*>(s_b + kTcPassB[pass] * b_elems);
-                for (int kk = 0; kk < kTcK / 16; ++kk) {
-                  const uint64_t da = smem_desc_kmajor(pa + kk * 2 * lbo_a, lbo_a, 128);
-                  const uint64_t db = smem_desc_kmajor(pb + kk * 2 * lbo_b, lbo_b, 128);
-                  tc_mma_bf16(d, da, db, idesc, first_mma ? 0u : 1u);
-                  first_mma = 0;
-                }
-              }
-            }
-          tc_commit(bars + 2);
-        }
-        mma_pending = true;
-        ok = mbar_wait(bars + 2, ph_mma);
-        ph_mma ^= 1u;
-        if (__syncthreads_or(!ok)) { failed = true; continue; }
-        mma_pending = false;
-        tc_fence_after();
+        group_sync_or(g, false);
+        const char* const* mine = table + lam * P;
+        const uint32_t wq_bytes = (uint32_t)wq * (uint32_t)sizeof(float2);
+        float acc_re[P], acc_im[P];
+#pragma unroll
+        for (int i = 0; i < P; ++i) acc_re[i] = acc_im[i] = 0.f;
+        // The rows of all degrees in order. The channels of eight pairs are loaded
+        // one row ahead (two with 8 pairs per group): each of the two buffers is
+        // filled again as soon as it has been used, across degrees too, so that a
+        // warp keeps 8 to 16 loads in flight.
+        constexpr int kRows = 16 / P;  // rows per turn of the loop: two buffers
+        float2 ch[2][8];
+        auto fetch = [&](float2 (&to)[8], int row, int c) {
+          const uint32_t at = (uint32_t)(min(row, rows - 1) * G.row_bytes) + wq_bytes;
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            to[i] = __ldg(reinterpret_cast<const float2*>(mine[c * 8 + i] + at));
+        };
         if (reads) {
-          for (int r = 0; r < nr; ++r) {
-            float xr[kTcSub], xi[kTcSub];
-            tmem_ld8(lane_base + (uint32_t)((h * 2) * n_pad + r * kTcSub), xr);
-            tmem_ld8(lane_base + (uint32_t)((h * 2 + 1) * n_pad + r * kTcSub), xi);
-            if (m_ok) {
+          fetch(ch[0], 0, 0);
+          fetch(ch[1], P == 16 ? 0 : 1, P == 16 ? 1 : 0);
+        }
+        int l = 0, r = 0, nr = 1;
+        uint32_t base = 0;
+        for (int row0 = 0; row0 < rows && !failed; row0 += kRows) {
 #pragma unroll
-              for (int i = 0; i < kTcSub; ++i) {
-                const Ge2TcPair& P = s_pair[s * kTcSub + i];
-                if (P.pair < 0) continue;
-                const float2 ch =
-                    P.channels[lam * P.band_stride + (int64_t)(row0 + r) * P.omega_stride + wq];
-                acc_re[s][i] += ch.x * xr[i] - ch.y * xi[i];
-                acc_im[s][i] += ch.x * xi[i] + ch.y * xr[i];
+          for (int u = 0; u < kRows; ++u) {
+            if (row0 + u >= rows || failed) continue;  // the same for the whole warp
+            if (r == 0) {  // a degree's columns
+              const uint32_t step = before + (uint32_t)(l * t.groups + g);
+              base = lane_base + (step % kTcSlots) * 2u * kTcCols;
+              if (!warp_wait(&bars->t_full[g][taken & 1u], (taken >> 1) & 1u)) {
+                failed = true;
+                continue;
               }
+              tc_fence_after();
+            }
+            if (reads) {
+#pragma unroll
+              for (int c = 0; c < P / 8; ++c) {
+                if (c * 8 >= cnt) continue;
+                float2 (&x)[8] = ch[P == 16 ? c : u];
+#pragma unroll
+                for (int i0 = 0; i0 < 8; i0 += 4) {
+                  float xr[4], xi[4];
+                  tmem_ld4x2(base + (uint32_t)(r * P + c * 8 + i0),
+                             base + (uint32_t)(kTcCols + r * P + c * 8 + i0), xr, xi);
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) {
+                    acc_re[c * 8 + i0 + i] += x[i0 + i].x * xr[i] - x[i0 + i].y * xi[i];
+                    acc_im[c * 8 + i0 + i] += x[i0 + i].x * xi[i] + x[i0 + i].y * xr[i];
+                  }
+                }
+                fetch(x, row0 + u + kRows, c);
+              }
+            }
+            if (++r == nr) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars->t_empty[g][taken & 1u]);
+              ++taken;
+              ++l;
+              r = 0;
+              nr = 2 * min(l, T.max_m) + 1;
             }
           }
         }
-        tc_fence_before();
-        __syncthreads();  // TMEM and the B tile are free for the next sub-tile
-      }
-      if (G.a_buffers == 1 && tid == 0 && l + 1 < L1 && !failed) {
-        // one buffer: the next degree once this degree's MMAs are done
-        mbar_expect_tx(bars + 0, load_bytes);
-        bulk_g2s(s_a0, G.packed + ((size_t)j * L1 + l + 1) * block_bytes, load_bytes, bars + 0);
-      }
-    }
-    // the pairs' spectra: band scale and flight phase e^{i w r / v}
-    if (!failed && m_ok) {
+        // the pairs' sums; ge2_tc_reduce_kernel applies their scale and flight phase
+        if (!failed && m_ok) {
 #pragma unroll
-      for (int s = 0; s < kTcSubs; ++s)
-#pragma unroll
-        for (int i = 0; i < kTcSub; ++i) {
-          const Ge2TcPair& P = s_pair[s * kTcSub + i];
-          if (P.pair < 0) continue;
-          const float sc = G.A.g_scale[P.scale_at + lam * P.scale_stride];
-          float sv = 0.f, cv = 1.f;
-          if (T.flight) {
-            const double turns = omega * G.A.g_r[P.pair] * inv_speed * (1.0 / (2 * kPi));
-            sincospif(2.f * (float)(turns - rint(turns)), &sv, &cv);
-          }
-          G.partial[(int64_t)P.pair * M + m] =
-              make_float2(sc * (acc_re[s][i] * cv - acc_im[s][i] * sv),
-                          sc * (acc_re[s][i] * sv + acc_im[s][i] * cv));
+          for (int i = 0; i < P; ++i)
+            if (i < cnt)
+              G.partial[(int64_t)G.entries[t.first + g * P + i].pair * M + m] =
+                  make_float2(acc_re[i], acc_im[i]);
         }
+      }
+      before += (uint32_t)(L1 * t.groups);
     }
-    __syncthreads();  // the pair table is rewritten by the next tile
+  } else if (warp < kTcEpiWarps + kTcBuildWarps) {
+    // ---- builders: B[n = r * P + i][k = 4 p + q] = F[r][p] t^(3 - q), split in parts
+    const int b0 = (warp - kTcEpiWarps) * 32;
+    const int NP = T.n_pairs;
+    const uint32_t inv_np = 65536u / NP + 1u;  // x / NP = x inv_np >> 16 for x < 2^16 / NP
+    uint32_t seq = 0;
+    for (int item = blockIdx.x; item < n_items && !failed; item += gridDim.x) {
+      const Ge2TcTile t = ge2_tc_tile(G, item);
+      // lane k holds pairs k and 32 + k of the tile (at most kTcGroups x P = 48)
+      const Ge2TcEntry& e_lo = G.entries[t.first + min(lane, t.count - 1)];
+      const Ge2TcEntry& e_hi = G.entries[t.first + min(lane + 32, t.count - 1)];
+      const int id_lo = e_lo.pair, id_hi = e_hi.pair;
+      const float t_lo = e_lo.t, t_hi = e_hi.t;
+      for (int l = 0; l < L1 && !failed; ++l) {
+        const int nr = 2 * min(l, T.max_m) + 1, row0 = T.starts[l], per = nr * NP;
+        const uint32_t inv_per = 65536u / per + 1u;  // exact: P x per^2 < 2^16
+        for (int g = 0; g < t.groups; ++g, ++seq) {
+          const int total = min(P, t.count - g * P) * per;
+          const uint32_t stage = seq % kTcBStages;
+          if (!warp_wait(bars->b_empty + stage, ((seq / kTcBStages) & 1u) ^ 1u)) {
+            failed = true;
+            break;
+          }
+          uint8_t* out = s_b + stage * b_bytes;
+          const bool upper = g * P >= 32;
+          constexpr int kAhead = 5;  // elements whose F is on its way per thread
+          for (int e0 = b0; e0 < total; e0 += 32 * kTcBuildWarps * kAhead) {
+            float f[kAhead], t1[kAhead];
+            int at[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+              const int e = e0 + u * 32 * kTcBuildWarps + lane;
+              const bool ok = e < total;
+              const int i = ok ? (int)(((uint32_t)e * inv_per) >> 16) : 0;
+              const int rp = ok ? e - i * per : 0;
+              const int r = (int)(((uint32_t)rp * inv_np) >> 16), p = rp - r * NP;
+              const int src = (g * P + i) & 31;
+              const int id = __shfl_sync(0xffffffffu, upper ? id_hi : id_lo, src);
+              t1[u] = __shfl_sync(0xffffffffu, upper ? t_hi : t_lo, src);
+              at[u] = ok ? ((p >> 1) * kTcCols + r * P + i) * 16 + (p & 1) * 8 : -1;
+              f[u] = ok ? __ldg(G.A.g_F + ((int64_t)id * T.nch + row0) * NP + rp) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+              if (at[u] < 0) continue;
+              const float t2 = t1[u] * t1[u];
+              const float v[4] = {f[u] * (t2 * t1[u]), f[u] * t2, f[u] * t1[u], f[u]};
+              uint2 part[kTcParts];
+              split3_bf16x2(v[0], v[1], part[0].x, part[1].x, part[2].x);
+              split3_bf16x2(v[2], v[3], part[0].y, part[1].y, part[2].y);
+#pragma unroll
+              for (int k = 0; k < kTcParts; ++k)
+                if (k < parts) *reinterpret_cast<uint2*>(out + at[u] + k * kBElems * 2) = part[k];
+            }
+          }
+          fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bars->b_full + stage);
+        }
+      }
+    }
+  } else {
+    // ---- one warp loads the coefficients (one bulk copy per part) and issues the
+    // MMAs: the load of stage n + 2 goes out after the MMAs of stage n, once those
+    // of stage n - 1 have left its place. The whole warp walks the loops and one
+    // elected lane issues, so that addresses and descriptors are uniform values
+    // (tcgen05.mma takes them from uniform registers: issued from a branch of one
+    // lane, each MMA took ~50 cycles of register moves whatever its N).
+    const unsigned full = 0xffffffffu;
+    const bool leader = elect_one();
+    const uint32_t tmem_u = __shfl_sync(full, tmem, 0);
+    const size_t block_bytes = (size_t)kTcParts * H * 2u * kTcTileBytes;
+    int ld_item = blockIdx.x, ld_l = 0;  // the next stage to load
+    const uint8_t* ld_from = nullptr;
+    uint32_t loaded = 0;
+    auto load_next = [&]() {
+      if (ld_item >= n_items) return;
+      if (ld_l == 0) {
+        const Ge2TcTile t = ge2_tc_tile(G, ld_item);
+        ld_from = G.packed + (size_t)t.j * L1 * block_bytes + (size_t)t.h * 2 * kTcTileBytes;
+      }
+      const uint32_t as = loaded % kTcAStages;
+      if (!warp_wait(bars->a_empty + as, ((loaded / kTcAStages) & 1u) ^ 1u)) {
+        failed = true;
+        return;
+      }
+      if (leader) {
+        mbar_expect_tx(bars->a_full + as, a_bytes);
+        for (int k = 0; k < parts; ++k)
+          bulk_g2s(s_a + as * a_bytes + (size_t)k * 2 * kTcTileBytes,
+                   ld_from + (size_t)k * H * 2 * kTcTileBytes, 2 * kTcTileBytes,
+                   bars->a_full + as);
+      }
+      __syncwarp();
+      ++loaded;
+      ld_from += block_bytes;
+      if (++ld_l == L1) {
+        ld_l = 0;
+        ld_item += gridDim.x;
+      }
+    };
+    for (int k = 0; k < kTcAStages - 1; ++k) load_next();
+    const uint64_t desc_a = smem_desc_kmajor(s_a, kTcLboA, 128);
+    const uint64_t desc_b = smem_desc_kmajor(s_b, kTcLboB, 128);
+    uint32_t step = 0, a_seq = 0;
+    // Steps issued and drained per group, modulo 256, one byte per group, and each
+    // slot's last user and its step: packed in registers (arrays indexed at run
+    // time would sit in local memory, behind an L1 that the channels stream
+    // through).
+    uint32_t issued = 0, drained = 0, slot_user = 0, slot_step = 0, slot_used = 0;
+    auto byte_of = [](uint32_t v, int k) { return (v >> (8 * k)) & 0xffu; };
+    auto set_byte = [](uint32_t v, int k, uint32_t x) {
+      return (v & ~(0xffu << (8 * k))) | ((x & 0xffu) << (8 * k));
+    };
+    // the group's steps up to `upto` (exclusive) have been read
+    auto drain_group = [&](int g, uint32_t upto) {
+      uint32_t n = byte_of(drained, g);
+      while ((int8_t)(upto - n) > 0) {
+        if (!warp_wait(&bars->t_empty[g][n & 1u], (n >> 1) & 1u)) return false;
+        n = (n + 1) & 0xffu;
+      }
+      drained = set_byte(drained, g, n);
+      return true;
+    };
+    for (int item = blockIdx.x; item < n_items && !failed; item += gridDim.x) {
+      const int groups = __shfl_sync(full, ge2_tc_tile(G, item).groups, 0);
+      for (int l = 0; l < L1 && !failed; ++l, ++a_seq) {
+        const int nr = 2 * min(l, T.max_m) + 1, n_pad = (nr * P + 15) & ~15;
+        const uint32_t idesc = instr_desc_bf16_f32(128, n_pad);
+        const uint32_t as = a_seq % kTcAStages;
+        if (!warp_wait(bars->a_full + as, (a_seq / kTcAStages) & 1u)) { failed = true; break; }
+        const uint64_t da0 = desc_a + ((as * a_bytes) >> 4);
+        for (int g = 0; g < groups; ++g, ++step) {
+          const uint32_t bs = step % kTcBStages, slot = step % kTcSlots;
+          const uint32_t mine = byte_of(issued, g);
+          // the group's step before last and the slot's last step have been read
+          if (!(drain_group(g, mine - 1) &&
+                (!((slot_used >> slot) & 1u) ||
+                 drain_group((int)byte_of(slot_user, slot), byte_of(slot_step, slot) + 1)) &&
+                warp_wait(bars->b_full + bs, (step / kTcBStages) & 1u))) {
+            failed = true;
+            break;
+          }
+          slot_used |= 1u << slot;
+          slot_user = set_byte(slot_user, slot, (uint32_t)g);
+          slot_step = set_byte(slot_step, slot, mine);
+          tc_fence_after();
+          const uint64_t db0 = desc_b + ((bs * b_bytes) >> 4);
+          const uint32_t d = tmem_u + slot * 2u * kTcCols;
+          if (leader) {
+            if (G.passes > 1) ge2_tc_issue<6>(d, da0, db0, idesc);
+            else ge2_tc_issue<1>(d, da0, db0, idesc);
+            tc_commit(&bars->t_full[g][mine & 1u]);
+            tc_commit(bars->b_empty + bs);
+            if (g == groups - 1) tc_commit(bars->a_empty + as);
+          }
+          __syncwarp();
+          issued = set_byte(issued, g, mine + 1);
+        }
+        if (!failed) load_next();
+      }
+    }
+    // nothing in flight outlives the shared memory and the TMEM allocation:
+    // copies that were never waited for (a role gave up), then the MMAs
+    for (; a_seq < loaded; ++a_seq)
+      warp_wait(bars->a_full + a_seq % kTcAStages, (a_seq / kTcAStages) & 1u);
+    if (leader) tc_commit(&bars->drain);
+    __syncwarp();
+    warp_wait(&bars->drain, 0);
   }
-  if (failed && tid == 0) atomicOr(reinterpret_cast<unsigned*>(G.status), LH_STATUS_TIMEOUT);
-  // nothing in flight may outlive the TMEM allocation (bounded waits)
-  if (mma_pending) mbar_wait(bars + 2, ph_mma);
-  for (int b = 0; b < G.a_buffers; ++b)  // a prefetched degree that was never waited for
-    if (failed) mbar_wait(bars + b, ph_load[b]);
+  if (failed && lane == 0) atomicOr(reinterpret_cast<unsigned*>(G.status), LH_STATUS_TIMEOUT);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, (uint32_t)G.tmem_cols);
+  if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-// result[d][w] = e^{i w ref} * sum over points (in order) and bands of the pairs' spectra.
-__global__ void ge2_tc_reduce_kernel(const lh_ge2_table T, const Ge2Slot* slots, Ge2Arrays A,
-                                     const float2* partial) {
+// result[d][w] = e^{i w ref} * sum over points and bands of s e^{i w r / v} times the
+// pairs' sums (float32 each, added in float64). A CTA takes one OM and 32
+// frequencies; its kTcReduceParts warps take every kTcReduceParts-th point and
+// their sums are added in order, so that the result is the same alone and in a
+// batch. With one thread per (OM, frequency) over all points the chains of
+// loads took 190 us for 384 OMs x 160 points.
+constexpr int kTcReduceParts = 16;
+
+__global__ void __launch_bounds__(32 * kTcReduceParts)
+ge2_tc_reduce_kernel(const lh_ge2_table T, const Ge2Slot* slots, Ge2Arrays A,
+                     const float2* partial) {
+  __shared__ double2 s_sum[kTcReduceParts][32];
+  __shared__ double s_inv_speed[256];  // at most 256 (band, frequency) rows
+  for (int lam = threadIdx.x; lam < T.n_bands; lam += blockDim.x)
+    s_inv_speed[lam] = 1.0 / T.speed[lam];
+  __syncthreads();
   const Ge2Slot& S = slots[blockIdx.y];
   const int W = S.P.n_omega, M = T.n_bands * T.n_omega;
-  const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)S.P.n_om * W) return;
-  const int d = (int)(idx / W), w = (int)(idx % W);
+  const int blocks_w = (W + 31) / 32;
+  const int d = blockIdx.x / blocks_w;
+  if (d >= S.P.n_om) return;
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+  const int w = (blockIdx.x - d * blocks_w) * 32 + lane;
   double re = 0.0, im = 0.0;
-  for (int c = 0; c < S.P.n_points; ++c) {
-    const int64_t g = S.pair_offset + (int64_t)d * S.P.n_points + c;
-    if (A.g_j[g] < 0) continue;
-    for (int lam = 0; lam < T.n_bands; ++lam) {
-      const float2 v = partial[g * M + lam * T.n_omega + w];
-      re += v.x;
-      im += v.y;
+  if (w < W) {
+    const double omega = T.omega[w];
+    const int64_t pairs = (int64_t)S.P.n_om * S.P.n_points;
+    for (int c = part; c < S.P.n_points; c += kTcReduceParts) {
+      const int64_t idx = (int64_t)d * S.P.n_points + c, g = S.pair_offset + idx;
+      if (A.g_j[g] < 0) continue;
+      const double r = A.g_r[g];
+      for (int lam = 0; lam < T.n_bands; ++lam) {
+        const float2 v = partial[g * M + lam * T.n_omega + w];
+        const float sc = A.g_scale[S.pair_offset * T.n_bands + lam * pairs + idx];
+        float sv = 0.f, cv = 1.f;
+        if (T.flight) {
+          const double turns = omega * r * s_inv_speed[lam] * (1.0 / (2 * kPi));
+          sincospif(2.f * (float)(turns - rint(turns)), &sv, &cv);
+        }
+        re += (double)(sc * fmaf(v.x, cv, -(v.y * sv)));
+        im += (double)(sc * fmaf(v.y, cv, v.x * sv));
+      }
     }
+  }
+  s_sum[part][lane] = make_double2(re, im);
+  __syncthreads();
+  if (part != 0 || w >= W) return;
+  for (int k = 1; k < kTcReduceParts; ++k) {
+    re += s_sum[k][lane].x;
+    im += s_sum[k][lane].y;
   }
   const double ang = T.omega[w] * S.P.reference_ns;
   const double c = cos(ang), s = sin(ang);
+  const int64_t idx = (int64_t)d * W + w;
   S.P.result[2 * idx] = re * c - im * s;
   S.P.result[2 * idx + 1] = re * s + im * c;
 }
 
-size_t ge2_tc_smem_bytes(int halves, int n_pad_max, int parts, int a_buffers) {
-  return (size_t)a_buffers * parts * halves * 2 * kTcTileBytes +
-         (size_t)parts * n_pad_max * kTcK * 2 + sizeof(Ge2TcPair) * kTcPairs +
-         3 * sizeof(uint64_t) + 16;
+size_t ge2_tc_smem_bytes(int pairs, int n_bands, int parts) {
+  return (size_t)kTcAStages * parts * 2 * kTcTileBytes +
+         (size_t)kTcBStages * parts * kTcCols * kTcK * 2 +
+         sizeof(char*) * kTcGroups * pairs * n_bands + sizeof(Ge2TcBars) + 16;
 }
 
 size_t ge2_tc_pack_bytes(const lh_ge2_table& T) {
-  int halves, n_pad_max;
-  if (!ge2_tc_supported(T, halves, n_pad_max)) return 0;
+  int halves, group_pairs;
+  if (!ge2_tc_supported(T, halves, group_pairs)) return 0;
   return (size_t)T.n_intervals * (T.degree + 1) * ge2_tc_block_bytes(T, halves);
 }
 
 int ge2_tc_pack(const lh_ge2_table& T, void* packed, cudaStream_t s) {
-  int halves, n_pad_max;
-  if (!ge2_tc_supported(T, halves, n_pad_max)) return LH_EUNSUPPORTED;
+  int halves, group_pairs;
+  if (!ge2_tc_supported(T, halves, group_pairs)) return LH_EUNSUPPORTED;
   const int64_t total = (int64_t)T.n_intervals * (T.degree + 1) * halves * 2 * 128 * kTcK;
   ge2_tc_pack_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(
       T, halves, static_cast<__nv_bfloat16*>(packed));
@@ -896,34 +1176,43 @@ int ge2_tc_pack(const lh_ge2_table& T, void* packed, cudaStream_t s) {
 }
 
 // Workspace of the tensor-core batch: the batch layout of ge2_batch_workspace,
-// then the bucket arrays, the sorted pairs and the per-pair spectra.
+// then the bucket arrays, the pair entries and the per-pair spectra.
 size_t ge2_tc_workspace(const lh_ge2_table& T, const lh_ge2_problem* P, int32_t n) {
   size_t pairs = 0;
   for (int i = 0; i < n; ++i) pairs += (size_t)P[i].n_om * P[i].n_points;
   auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-  return ge2_batch_workspace(T, P, n) + 3 * up(sizeof(int32_t) * (T.n_intervals + 1)) +
-         2 * up(sizeof(int32_t) * pairs) + up(sizeof(float2) * pairs * T.n_bands * T.n_omega);
+  int halves, group_pairs;
+  if (!ge2_tc_supported(T, halves, group_pairs)) return 0;
+  return ge2_batch_workspace(T, P, n) + 2 * up(sizeof(int32_t) * (T.n_intervals + 1)) +
+         up(sizeof(int4) * (pairs / group_pairs + T.n_intervals + 1)) +
+         up(sizeof(Ge2TcEntry) * pairs) + up(sizeof(float2) * pairs * T.n_bands * T.n_omega);
 }
 
-int ge2_tc_batch_launch(const lh_ge2_table& T, const lh_ge2_problem* P, int32_t n, int passes,
-                        const void* packed, void* ws, void* host_slots, int32_t* status,
-                        cudaStream_t s) {
-  int halves, n_pad_max;
-  if (!ge2_tc_supported(T, halves, n_pad_max)) return LH_EUNSUPPORTED;
+// The problems whose channel rows have `stride` (n_omega_channels), with their
+// slots from `first_slot` on; the number of them comes back in `count`.
+static int ge2_tc_class_launch(const lh_ge2_table& T, const lh_ge2_problem* P, int32_t n,
+                               int32_t stride, int32_t first_slot, int32_t& count, int passes,
+                               const void* packed, void* ws, void* host_slots, int32_t* status,
+                               cudaStream_t s) {
+  int halves, group_pairs;
+  if (!ge2_tc_supported(T, halves, group_pairs)) return LH_EUNSUPPORTED;
   auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
-  Ge2Slot* hs = static_cast<Ge2Slot*>(host_slots);
+  Ge2Slot* hs = static_cast<Ge2Slot*>(host_slots) + first_slot;
   size_t pairs = 0;
-  int64_t max_pairs = 0, max_outs = 0;
+  int64_t max_pairs = 0;
+  int max_om = 0;
+  count = 0;
   for (int i = 0; i < n; ++i) {
-    if (P[i].n_omega != T.n_omega) return LH_EINVAL;  // full spectra only
-    hs[i].P = P[i];
-    hs[i].pair_offset = (int64_t)pairs;
-    hs[i].partial_offset = 0;
-    hs[i].chunks = 0;
+    if (P[i].n_omega_channels != stride) continue;
+    Ge2Slot& S = hs[count++];
+    S.P = P[i];
+    S.pair_offset = (int64_t)pairs;
+    S.partial_offset = 0;
+    S.chunks = 0;
     const int64_t pp = (int64_t)P[i].n_om * P[i].n_points;
     pairs += pp;
     max_pairs = std::max(max_pairs, pp);
-    max_outs = std::max(max_outs, (int64_t)P[i].n_om * P[i].n_omega);
+    max_om = std::max(max_om, P[i].n_om);
   }
   uint8_t* p = static_cast<uint8_t*>(ws);
   Ge2Slot* slots = reinterpret_cast<Ge2Slot*>(p); p += up(sizeof(Ge2Slot) * (size_t)n);
@@ -937,67 +1226,79 @@ int ge2_tc_batch_launch(const lh_ge2_table& T, const lh_ge2_problem* P, int32_t 
   // the CUDA-core path's chunk partials are not used here
   p = static_cast<uint8_t*>(ws) + ge2_batch_workspace(T, P, n);
   int32_t* counts = reinterpret_cast<int32_t*>(p); p += up(sizeof(int32_t) * (T.n_intervals + 1));
-  int32_t* bucket_start = reinterpret_cast<int32_t*>(p); p += up(sizeof(int32_t) * (T.n_intervals + 1));
-  int32_t* tile_start = reinterpret_cast<int32_t*>(p); p += up(sizeof(int32_t) * (T.n_intervals + 1));
-  int32_t* sorted = reinterpret_cast<int32_t*>(p); p += up(sizeof(int32_t) * pairs);
-  int32_t* sorted_slot = reinterpret_cast<int32_t*>(p); p += up(sizeof(int32_t) * pairs);
+  int32_t* n_tiles = reinterpret_cast<int32_t*>(p); p += up(sizeof(int32_t) * (T.n_intervals + 1));
+  int4* tiles = reinterpret_cast<int4*>(p);
+  p += up(sizeof(int4) * (pairs / group_pairs + T.n_intervals + 1));
+  Ge2TcEntry* entries = reinterpret_cast<Ge2TcEntry*>(p); p += up(sizeof(Ge2TcEntry) * pairs);
   float2* partial = reinterpret_cast<float2*>(p);
-  if (cudaMemcpyAsync(slots, hs, sizeof(Ge2Slot) * (size_t)n, cudaMemcpyHostToDevice, s) !=
+  slots += first_slot;
+  if (cudaMemcpyAsync(slots, hs, sizeof(Ge2Slot) * (size_t)count, cudaMemcpyHostToDevice, s) !=
       cudaSuccess)
     return LH_ECUDA;
-  if (max_outs == 0) return LH_OK;
+  if (max_om == 0) return LH_OK;
   if (max_pairs == 0) {  // no points anywhere: every result is zero
-    for (int i = 0; i < n; ++i)
-      cudaMemsetAsync(P[i].result, 0, sizeof(double) * 2 * (size_t)P[i].n_om * P[i].n_omega, s);
+    for (int i = 0; i < count; ++i)
+      cudaMemsetAsync(hs[i].P.result, 0, sizeof(double) * 2 * (size_t)hs[i].P.n_om * T.n_omega, s);
     return cudaGetLastError() == cudaSuccess ? LH_OK : LH_ECUDA;
   }
-  ge2_geometry_batch_kernel<<<dim3((unsigned)((max_pairs + 127) / 128), n), 128, 0, s>>>(T, slots,
+  ge2_geometry_batch_kernel<<<dim3((unsigned)((max_pairs + 127) / 128), count), 128, 0, s>>>(T, slots,
                                                                                       A);
   cudaMemsetAsync(counts, 0, sizeof(int32_t) * (T.n_intervals + 1), s);
   const unsigned bucket_blocks = (unsigned)std::min<int64_t>((max_pairs + 255) / 256, 148 * 4);
-  ge2_tc_bucket_kernel<<<dim3(bucket_blocks, n), 256, 0, s>>>(slots, A, counts, sorted,
-                                                              sorted_slot, 0);
-  ge2_tc_scan_kernel<<<1, 32, 0, s>>>(T.n_intervals, counts, bucket_start, tile_start,
-                                      kernel_units() ? kernel_units() + LH_KT_GE2_TC : nullptr);
-  ge2_tc_bucket_kernel<<<dim3(bucket_blocks, n), 256, 0, s>>>(slots, A, counts, sorted,
-                                                              sorted_slot, 1);
+  ge2_tc_bucket_kernel<<<dim3(bucket_blocks, count), 256, 0, s>>>(slots, A, T.nch, counts, nullptr);
+  ge2_tc_tiles_kernel<<<1, 256, sizeof(int32_t) * 2 * (T.n_intervals + 1), s>>>(
+      T.n_intervals, group_pairs, halves, counts, tiles, n_tiles,
+      kernel_units() ? kernel_units() + LH_KT_GE2_TC : nullptr);
+  ge2_tc_bucket_kernel<<<dim3(bucket_blocks, count), 256, 0, s>>>(slots, A, T.nch, counts, entries);
   Ge2TcArgs G;
-  G.slots = slots;
   G.A = A;
   G.packed = static_cast<const uint8_t*>(packed);
-  G.sorted = sorted;
-  G.sorted_slot = sorted_slot;
-  G.bucket_start = bucket_start;
-  G.tile_start = tile_start;
+  G.entries = entries;
+  G.tiles = tiles;
+  G.n_tiles = n_tiles;
+  G.row_bytes = stride * (int)sizeof(float2);
   G.partial = partial;
   G.status = status;
   G.passes = passes;
   G.halves = halves;
-  G.n_pad_max = n_pad_max;
-  // Two CTAs per SM (one overlapping the other's waits) when the accumulators
-  // fit 256 TMEM columns and one coefficient buffer each fits half the shared
-  // memory; otherwise one CTA per SM with 512 columns and a prefetch buffer.
-  const int parts = passes > 1 ? kTcParts : 1;
-  const bool two = 2 * halves * n_pad_max <= 256 &&
-                   ge2_tc_smem_bytes(halves, n_pad_max, parts, 1) <= 110 * 1024;
-  G.tmem_cols = two ? 256 : 512;
-  G.a_buffers = two ? 1 : 2;
-  const size_t smem = ge2_tc_smem_bytes(halves, n_pad_max, parts, G.a_buffers);
+  const size_t smem = ge2_tc_smem_bytes(group_pairs, T.n_bands, passes > 1 ? kTcParts : 1);
+  auto* kernel = group_pairs == 16 ? ge2_tc_kernel<16> : ge2_tc_kernel<8>;
   if (smem > 227 * 1024) return LH_EUNSUPPORTED;
-  if (cudaFuncSetAttribute(ge2_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
     return LH_ECUDA;
-  // persistent CTAs (one or two per SM); tiles beyond the grid are taken in turn
-  const int64_t tile_bound = (int64_t)(pairs + kTcPairs - 1) / kTcPairs + T.n_intervals;
-  const unsigned grid =
-      (unsigned)std::max<int64_t>(1, std::min<int64_t>(tile_bound, two ? 2 * 148 : 148));
+  // persistent CTAs, one per SM; work items beyond the grid are taken in turn
+  const int64_t item_bound = ((int64_t)(pairs + group_pairs - 1) / group_pairs + T.n_intervals) * halves;
+  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(item_bound, 148));
   {
     lh::TimedLaunch timed_launch(LH_KT_GE2_TC, s);
-    ge2_tc_kernel<<<grid, kTcThreads, smem, s>>>(T, G);
+    kernel<<<grid, kTcThreads, smem, s>>>(T, G);
   }
-  ge2_tc_reduce_kernel<<<dim3((unsigned)((max_outs + 255) / 256), n), 256, 0, s>>>(T, slots, A,
-                                                                                   partial);
+  ge2_tc_reduce_kernel<<<dim3((unsigned)(max_om * ((T.n_omega + 31) / 32)), count),
+                         32 * kTcReduceParts, 0, s>>>(T, slots, A, partial);
   return cudaGetLastError() == cudaSuccess ? LH_OK : LH_ECUDA;
+}
+
+// The epilogue takes one channel row stride per launch (the route's problems all
+// have the table's): problems of other strides follow in launches of their own
+// over the same workspace, each class with its own slots.
+int ge2_tc_batch_launch(const lh_ge2_table& T, const lh_ge2_problem* P, int32_t n, int passes,
+                        const void* packed, void* ws, void* host_slots, int32_t* status,
+                        cudaStream_t s) {
+  for (int i = 0; i < n; ++i)
+    if (P[i].n_omega != T.n_omega) return LH_EINVAL;  // full spectra only
+  int32_t done = 0;
+  for (int i = 0; i < n && done < n; ++i) {
+    bool seen = false;
+    for (int k = 0; k < i && !seen; ++k) seen = P[k].n_omega_channels == P[i].n_omega_channels;
+    if (seen) continue;
+    int32_t count = 0;
+    const int rc = ge2_tc_class_launch(T, P, n, P[i].n_omega_channels, done, count, passes, packed,
+                                       ws, host_slots, status, s);
+    if (rc != LH_OK) return rc;
+    done += count;
+  }
+  return LH_OK;
 }
 
 }  // namespace lh

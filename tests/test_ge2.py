@@ -187,3 +187,36 @@ def test_tensor_core_batched_problems_equal_alone():
         assert np.array_equal(got, alone)
     assert not np.any(together[-1])
     assert np.any(together[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_points", [1, 15, 16, 17, 48, 49, 140])
+def test_tensor_core_tile_edges(n_points):
+    """Work items at the edges of a group (16 pairs) and of a tile (48), with few
+    pairs per interval and with many, and problems whose channel rows have other
+    strides (more frequencies stored than read): against the float64 oracle."""
+    from lighthit_b200.ge2 import AxialSources, Ge2Table
+    g, t, frame = fixture()
+    table = Ge2Table(t, g["alpha"], source_degree=8, azimuthal_degree=2)
+    rng = np.random.default_rng(n_points)
+    pts = points(g, frame, "zero")[:n_points]
+    P = len(pts)
+    basis = (frame["centre"], frame["first"], frame["second"], frame["axis"])
+    oms = np.array([3, 20, 41])
+    items, expected = [], []
+    for stored in (65, 70, 65, 66):
+        ch = (rng.normal(size=(3, P, 39, stored))
+              + 1j * rng.normal(size=(3, P, 39, stored))).astype(np.complex64)
+        for some in (oms[:1], oms):
+            src = AxialSources(pts, ch, np.zeros(3), basis, 8, 2)
+            items.append((src, g["om_positions_m"][some], g["om_looks"][some],
+                          g["om_area_m2"][some], g["radial_window_m"]))
+            expected.append(oracle_apply(
+                t, dict(points_m=pts, channels=ch[..., :65], reference_ns=np.zeros(3),
+                        frame=frame, degree=8, azimuthal_degree=2), g["om_positions_m"][some],
+                g["om_looks"][some], g["alpha"], g["om_area_m2"][some], g["radial_window_m"],
+                fast=True))
+    out = table.apply_batch(items, mode="split-bf16")
+    assert int(table.status.item()) == 0
+    for got, ref in zip(out, expected):
+        assert np.abs(got.cpu().numpy().T - ref).max() <= GE2_TOL * np.abs(ref).max()
