@@ -33,122 +33,189 @@ constexpr int kGe2Out = 4;       // acceptance (detector) degree bound
 constexpr int kGe2M = 4;         // azimuthal degree bound
 constexpr int kGe2Chunk = 32;    // points per partial sum
 
-// One thread per (OM, point): radius, interval, band scales and F.
-LH_DEVICE void ge2_geometry_body(const lh_ge2_table& T, const lh_ge2_problem& P, int64_t idx,
-                                 int* g_j, float* g_t, double* g_r, float* g_scale, float* g_F) {
-  const int64_t total = (int64_t)P.n_om * P.n_points;
-  if (idx >= total) return;
-  const int d = (int)(idx / P.n_points), c = (int)(idx % P.n_points);
-  const double dx = P.receivers[3 * d] - P.points[3 * c];
-  const double dy = P.receivers[3 * d + 1] - P.points[3 * c + 1];
-  const double dz = P.receivers[3 * d + 2] - P.points[3 * c + 2];
-  const double radius = sqrt(dx * dx + dy * dy + dz * dz);
-  g_r[idx] = radius;
-  if (!(radius >= P.radial_low && radius <= P.radial_high)) {
-    g_j[idx] = -1;
-    return;
-  }
-  const int L = T.degree, A = T.acc_degree, M = T.max_m, W = 2 * A + 1, NP = T.n_pairs;
-  double cosine = dz / radius;
-  cosine = cosine > 1.0 ? 1.0 : (cosine < -1.0 ? -1.0 : cosine);
-  const double phi = atan2(dy, dx);
-  const double tr = sqrt(dx * dx + dy * dy);
-  const double sine = tr / radius;
-  const double cp = tr == 0.0 ? 1.0 : dx / tr;
-  const double sp = tr == 0.0 ? 0.0 : dy / tr;
-  double cosn[kGe2M + 1], sinn[kGe2M + 1];
-  for (int n = 0; n <= M; ++n) {
-    cosn[n] = cos(n * phi);
-    sinn[n] = sin(n * phi);
-  }
-  const double lx = P.looks[3 * d], ly = P.looks[3 * d + 1], lz = P.looks[3 * d + 2];
-  const double a1 = cosine * cp * lx + cosine * sp * ly - sine * lz;
-  const double a2 = -sp * lx + cp * ly;
-  const double a3 = sine * cp * lx + sine * sp * ly + cosine * lz;
-  double det[(kGe2Out + 1) * (kGe2Out + 1)];
-  real_harmonics(a1, a2, a3, A, det);
-  // pair weights D_p[a]: alpha_lam Y[lam, +mu] at a = A + mu, alpha Y[lam, -mu] at A - mu
-  // Wigner d^l_(mu nu): wig[l][nu + A][mu], mu = 0..M, by recurrence in l (:51-87)
-  double wig[kGe2Degree + 1][2 * kGe2Out + 1][kGe2M + 1];
-  for (int l = 0; l <= L; ++l)
-    for (int a = 0; a < W; ++a)
-      for (int m = 0; m <= M; ++m) wig[l][a][m] = 0.0;
-  const double hc = sqrt((1.0 + cosine) / 2.0), hs = sqrt((1.0 - cosine) / 2.0);
-  for (int nu = -A; nu <= A; ++nu) {
-    for (int mu = 0; mu <= M; ++mu) {
-      const int start = abs(nu) > mu ? abs(nu) : mu;
-      if (start > L) continue;
-      double prev = 0.0, cur = wigner_start(start, mu, nu, hc, hs, T.start_norm, T.jmax);
-      wig[start][nu + A][mu] = cur;
-      for (int l = start; l < L; ++l) {
-        double value;
-        if (l == 0) value = cosine * cur;
-        else {
-          double lower = (double)(l * l - mu * mu) * (double)(l * l - nu * nu);
-          lower = lower > 0.0 ? sqrt(lower) : 0.0;
-          const double upper = sqrt((double)((l + 1) * (l + 1) - mu * mu) *
-                                    (double)((l + 1) * (l + 1) - nu * nu));
-          value = ((2 * l + 1) * (l * (l + 1) * cosine - mu * nu) * cur - (l + 1) * lower * prev) /
-                  (l * upper);
-        }
-        prev = cur;
-        cur = value;
-        wig[l + 1][nu + A][mu] = cur;
-      }
-    }
-  }
-  // F_l[b][p] for every kept source channel (row = starts[l] + (b - M + keep))
-  float* F = g_F + idx * (int64_t)T.nch * NP;
+// Radius, interval, band scales and F of every (OM, point). A CTA takes a block of
+// consecutive pairs through three steps in shared memory: one thread per pair
+// forms the pair's angles, harmonics and scales; one thread per (pair, nu, mu)
+// runs that Wigner chain over the degrees; one thread per (pair, channel row)
+// forms the row's F. With one thread per pair the Wigner table (675 float64 at
+// degree 8) sat in local memory: 0.22 ms for 61k pairs and 0.105 ms for 8k, most
+// of it latency; now 0.139 and 0.041 ms.
+constexpr int kGe2GeoThreads = 128;
+constexpr size_t kGe2GeoSmem = 46 * 1024;
+
+// float64 values of shared memory: the recurrence factors, then per pair the
+// Wigner table, cosine, half-angle cosine and sine, cos/sin(n phi), and the
+// detector weight of each (lambda, +mu) and (lambda, -mu).
+__host__ __device__ inline int ge2_geo_wigner(const lh_ge2_table& T) {
+  return (T.degree + 1) * (2 * T.acc_degree + 1) * (T.max_m + 1);
+}
+__host__ __device__ inline int ge2_geo_pair_values(const lh_ge2_table& T) {
+  return ge2_geo_wigner(T) + 3 + 2 * (T.max_m + 1) + 2 * T.n_pairs;
+}
+// Pairs per CTA: as many as fit, at most 32.
+__host__ __device__ inline int ge2_geo_pairs(const lh_ge2_table& T) {
+  const int left = (int)(kGe2GeoSmem / sizeof(double)) - 2 * ge2_geo_wigner(T);
+  const int fit = left / ge2_geo_pair_values(T);
+  return fit < 32 ? fit : 32;
+}
+static size_t ge2_geo_smem(const lh_ge2_table& T) {
+  return sizeof(double) * (2 * (size_t)ge2_geo_wigner(T) +
+                           (size_t)ge2_geo_pairs(T) * ge2_geo_pair_values(T));
+}
+
+static unsigned ge2_geo_blocks(const lh_ge2_table& T, int64_t pairs) {
+  const int per = ge2_geo_pairs(T);
+  return (unsigned)((pairs + per - 1) / per);
+}
+
+// Entry (q, n) of the real rotation row block of degree l: detector order q and
+// source order n, from the Wigner table (_shower_basis.py:957-977).
+LH_DEVICE double ge2_rotation(const double* wig, int l, int A, int M, const double* cosn,
+                              const double* sinn, int q, int n) {
   const double root2 = sqrt(2.0);
-  for (int l = 0; l <= L; ++l) {
-    double erow[2 * kGe2Out + 1][2 * kGe2M + 1];
-    for (int a = 0; a < W; ++a)
-      for (int b = 0; b <= 2 * M; ++b) erow[a][b] = 0.0;
-    erow[A][M] = wig[l][A][0];
-    const int top_n = l < M ? l : M, top_p = l < A ? l : A;
-    for (int n = 1; n <= top_n; ++n) {
-      const double base = root2 * par(n) * wig[l][A][n];
-      erow[A][M + n] = base * cosn[n];
-      erow[A][M - n] = base * sinn[n];
+  const int W = 2 * A + 1, k = abs(n), pp = abs(q);
+  auto w = [&](int nu, int mu) { return wig[(l * W + nu + A) * (M + 1) + mu]; };
+  if (q == 0) {
+    if (n == 0) return w(0, 0);
+    const double base = root2 * par(k) * w(0, k);
+    return n > 0 ? base * cosn[k] : base * sinn[k];
+  }
+  if (n == 0) return q > 0 ? root2 * par(pp) * w(pp, 0) : 0.0;
+  const double cross = par(pp) * w(pp, k), straight = w(-pp, k);
+  if (q > 0) {
+    const double cc = par(k) * (cross + straight);
+    return n > 0 ? cc * cosn[k] : cc * sinn[k];
+  }
+  const double ss = par(k) * (cross - straight);
+  return n > 0 ? -ss * sinn[k] : ss * cosn[k];
+}
+
+LH_DEVICE void ge2_geometry_body(const lh_ge2_table& T, const lh_ge2_problem& P, int64_t block,
+                                 int* g_j, float* g_t, double* g_r, float* g_scale, float* g_F) {
+  extern __shared__ double s_geo[];
+  __shared__ int s_inside[32];
+  const int64_t total = (int64_t)P.n_om * P.n_points;
+  const int per_block = ge2_geo_pairs(T);
+  const int64_t first = block * per_block;
+  if (first >= total) return;
+  const int count = (int)min((int64_t)per_block, total - first);
+  const int L = T.degree, A = T.acc_degree, M = T.max_m, W = 2 * A + 1, NP = T.n_pairs;
+  const int chains = W * (M + 1), n_wig = ge2_geo_wigner(T), values = ge2_geo_pair_values(T);
+  double* s_lower = s_geo;          // [l][chain]: (l + 1) sqrt((l^2 - mu^2)(l^2 - nu^2))
+  double* s_upper = s_geo + n_wig;  // [l][chain]: l sqrt(((l+1)^2 - mu^2)((l+1)^2 - nu^2))
+  double* s_pair = s_geo + 2 * n_wig;
+  for (int e = threadIdx.x; e < L * chains; e += blockDim.x) {
+    const int l = e / chains, chain = e - l * chains, nu = chain / (M + 1) - A,
+              mu = chain % (M + 1);
+    double lower = (double)(l * l - mu * mu) * (double)(l * l - nu * nu);
+    lower = lower > 0.0 ? sqrt(lower) : 0.0;
+    const double upper = sqrt((double)((l + 1) * (l + 1) - mu * mu) *
+                              (double)((l + 1) * (l + 1) - nu * nu));
+    s_lower[e] = (l + 1) * lower;
+    s_upper[e] = l * upper;
+  }
+  for (int k = threadIdx.x; k < count; k += blockDim.x) {
+    const int64_t idx = first + k;
+    const int d = (int)(idx / P.n_points), c = (int)(idx % P.n_points);
+    const double dx = P.receivers[3 * d] - P.points[3 * c];
+    const double dy = P.receivers[3 * d + 1] - P.points[3 * c + 1];
+    const double dz = P.receivers[3 * d + 2] - P.points[3 * c + 2];
+    const double radius = sqrt(dx * dx + dy * dy + dz * dz);
+    g_r[idx] = radius;
+    const bool inside = radius >= P.radial_low && radius <= P.radial_high;
+    s_inside[k] = inside;
+    if (!inside) {
+      g_j[idx] = -1;
+      continue;
     }
-    for (int pp = 1; pp <= top_p; ++pp) {
-      erow[A + pp][M] = root2 * par(pp) * wig[l][A + pp][0];
-      for (int n = 1; n <= top_n; ++n) {
-        const double cross = par(pp) * wig[l][A + pp][n];
-        const double straight = wig[l][A - pp][n];
-        const double cc = par(n) * (cross + straight), ss = par(n) * (cross - straight);
-        erow[A + pp][M + n] = cc * cosn[n];
-        erow[A + pp][M - n] = cc * sinn[n];
-        erow[A - pp][M + n] = -ss * sinn[n];
-        erow[A - pp][M - n] = ss * cosn[n];
-      }
+    double* pair = s_pair + k * values + n_wig;
+    double* cosn = pair + 3;
+    double* sinn = cosn + M + 1;
+    double* weight = sinn + M + 1;
+    double cosine = dz / radius;
+    cosine = cosine > 1.0 ? 1.0 : (cosine < -1.0 ? -1.0 : cosine);
+    const double phi = atan2(dy, dx);
+    const double tr = sqrt(dx * dx + dy * dy);
+    const double sine = tr / radius;
+    const double cp = tr == 0.0 ? 1.0 : dx / tr;
+    const double sp = tr == 0.0 ? 0.0 : dy / tr;
+    pair[0] = cosine;
+    pair[1] = sqrt((1.0 + cosine) / 2.0);
+    pair[2] = sqrt((1.0 - cosine) / 2.0);
+    for (int n = 0; n <= M; ++n) {
+      cosn[n] = cos(n * phi);
+      sinn[n] = sin(n * phi);
     }
-    const int keep = top_n;
-    for (int b = M - keep; b <= M + keep; ++b) {
-      const int row = T.starts[l] + keep + (b - M);
-      for (int p = 0; p < NP; ++p) {
-        const int lam = T.pair_lambda[p], mup = T.pair_mu[p];
-        double f = 0.0;
-        if (mup <= top_p) {
-          const int cidx = lam * lam + lam;
-          const double pos = T.alpha[lam] * det[cidx + mup];
-          const double neg = mup ? T.alpha[lam] * det[cidx - mup] : 0.0;
-          if (neg != 0.0) f += erow[A - mup][b] * neg;
-          if (pos != 0.0) f += erow[A + mup][b] * pos;
-        }
-        F[row * NP + p] = (float)f;
-      }
+    const double lx = P.looks[3 * d], ly = P.looks[3 * d + 1], lz = P.looks[3 * d + 2];
+    const double a1 = cosine * cp * lx + cosine * sp * ly - sine * lz;
+    const double a2 = -sp * lx + cp * ly;
+    const double a3 = sine * cp * lx + sine * sp * ly + cosine * lz;
+    double det[(kGe2Out + 1) * (kGe2Out + 1)];
+    real_harmonics(a1, a2, a3, A, det);
+    // pair weights: alpha_lam Y[lam, +mu], alpha_lam Y[lam, -mu]
+    for (int p = 0; p < NP; ++p) {
+      const int lam = T.pair_lambda[p], mup = T.pair_mu[p], centre = lam * lam + lam;
+      weight[2 * p] = T.alpha[lam] * det[centre + mup];
+      weight[2 * p + 1] = mup ? T.alpha[lam] * det[centre - mup] : 0.0;
+    }
+    const double logr = log(radius);
+    int j = bin_right(T.log_r, T.n_intervals + 1, logr);
+    j = j < 0 ? 0 : (j > T.n_intervals - 1 ? T.n_intervals - 1 : j);
+    g_j[idx] = j;
+    g_t[idx] = (float)(logr - T.log_r[j]);
+    for (int lam = 0; lam < T.n_bands; ++lam)
+      g_scale[(int64_t)lam * total + idx] =
+          (float)(P.out_scale[(int64_t)lam * P.n_om + d] * exp(-T.absorption[lam] * radius) /
+                  (4 * kPi * radius * radius));
+  }
+  __syncthreads();
+  // Wigner d^l_(mu nu), mu = 0..M, by recurrence in l (:51-87)
+  for (int e = threadIdx.x; e < count * chains; e += blockDim.x) {
+    const int k = e / chains, chain = e - k * chains, nu = chain / (M + 1) - A,
+              mu = chain % (M + 1);
+    const int start = abs(nu) > mu ? abs(nu) : mu;
+    if (!s_inside[k] || start > L) continue;
+    double* wig = s_pair + k * values;
+    const double cosine = wig[n_wig], hc = wig[n_wig + 1], hs = wig[n_wig + 2];
+    double prev = 0.0, cur = wigner_start(start, mu, nu, hc, hs, T.start_norm, T.jmax);
+    wig[start * chains + chain] = cur;
+    for (int l = start; l < L; ++l) {
+      double value;
+      if (l == 0) value = cosine * cur;
+      else
+        value = ((2 * l + 1) * (l * (l + 1) * cosine - mu * nu) * cur -
+                 s_lower[l * chains + chain] * prev) / s_upper[l * chains + chain];
+      prev = cur;
+      cur = value;
+      wig[(l + 1) * chains + chain] = cur;
     }
   }
-  const double logr = log(radius);
-  int j = bin_right(T.log_r, T.n_intervals + 1, logr);
-  j = j < 0 ? 0 : (j > T.n_intervals - 1 ? T.n_intervals - 1 : j);
-  g_j[idx] = j;
-  g_t[idx] = (float)(logr - T.log_r[j]);
-  for (int lam = 0; lam < T.n_bands; ++lam)
-    g_scale[(int64_t)lam * total + idx] =
-        (float)(P.out_scale[(int64_t)lam * P.n_om + d] * exp(-T.absorption[lam] * radius) /
-                (4 * kPi * radius * radius));
+  __syncthreads();
+  // F_l[b][p] for every kept source channel (row = starts[l] + keep + n)
+  const int rows = T.starts[L] + 2 * min(L, M) + 1;
+  for (int e = threadIdx.x; e < count * rows; e += blockDim.x) {
+    const int k = e / rows, row = e - k * rows;
+    if (!s_inside[k]) continue;
+    int l = 0;
+    while (l < L && T.starts[l + 1] <= row) ++l;
+    const int keep = l < M ? l : M, top_p = l < A ? l : A;
+    const int n = row - T.starts[l] - keep;
+    const double* wig = s_pair + k * values;
+    const double* cosn = wig + n_wig + 3;
+    const double* sinn = cosn + M + 1;
+    const double* weight = sinn + M + 1;
+    float* F = g_F + ((first + k) * (int64_t)T.nch + row) * NP;
+    for (int p = 0; p < NP; ++p) {
+      const int mup = T.pair_mu[p];
+      double f = 0.0;
+      if (mup <= top_p && n <= keep) {
+        const double pos = weight[2 * p], neg = weight[2 * p + 1];
+        if (neg != 0.0) f += ge2_rotation(wig, l, A, M, cosn, sinn, -mup, n) * neg;
+        if (pos != 0.0) f += ge2_rotation(wig, l, A, M, cosn, sinn, mup, n) * pos;
+      }
+      F[p] = (float)f;
+    }
+  }
 }
 
 // Grid (OM, point chunk); thread = (band, frequency). Partial sums per chunk.
@@ -305,7 +372,7 @@ LH_DEVICE void ge2_reduce_body(const lh_ge2_table& T, const lh_ge2_problem& P, i
 // One problem: grids over its own sizes.
 __global__ void ge2_geometry_kernel(lh_ge2_table T, lh_ge2_problem P, int* g_j, float* g_t,
                                     double* g_r, float* g_scale, float* g_F) {
-  ge2_geometry_body(T, P, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, g_j, g_t, g_r, g_scale,
+  ge2_geometry_body(T, P, blockIdx.x, g_j, g_t, g_r, g_scale,
                     g_F);
 }
 
@@ -342,7 +409,7 @@ struct Ge2Arrays {
 __global__ void ge2_geometry_batch_kernel(lh_ge2_table T, const Ge2Slot* slots, Ge2Arrays A) {
   const Ge2Slot& S = slots[blockIdx.y];
   const int64_t o = S.pair_offset;
-  ge2_geometry_body(T, S.P, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, A.g_j + o, A.g_t + o,
+  ge2_geometry_body(T, S.P, blockIdx.x, A.g_j + o, A.g_t + o,
                     A.g_r + o, A.g_scale + o * T.n_bands, A.g_F + o * T.nch * T.n_pairs);
 }
 
@@ -391,7 +458,7 @@ int ge2_launch(const lh_ge2_table& T, const lh_ge2_problem& P, void* ws, cudaStr
   float* g_scale = reinterpret_cast<float*>(p); p += up(pairs * T.n_bands * 4);
   float* g_F = reinterpret_cast<float*>(p); p += up(pairs * T.nch * T.n_pairs * 4);
   double2* partial = reinterpret_cast<double2*>(p);
-  ge2_geometry_kernel<<<(unsigned)((pairs + 127) / 128), 128, 0, s>>>(T, P, g_j, g_t, g_r, g_scale, g_F);
+  ge2_geometry_kernel<<<ge2_geo_blocks(T, (int64_t)pairs), kGe2GeoThreads, ge2_geo_smem(T), s>>>(T, P, g_j, g_t, g_r, g_scale, g_F);
   const int chunks = ge2_chunks(P);
   const size_t smem = ge2_apply_smem(T, T.n_bands * P.n_omega);
   if (smem > 48 * 1024)
@@ -453,8 +520,8 @@ int ge2_batch_launch(const lh_ge2_table& T, const lh_ge2_problem* P, int32_t n, 
     return LH_ECUDA;
   if (max_outs == 0) return LH_OK;
   if (max_pairs > 0) {  // problems without points reduce nothing: their results are zero
-    ge2_geometry_batch_kernel<<<dim3((unsigned)((max_pairs + 127) / 128), n), 128, 0, s>>>(
-        T, slots, A);
+    ge2_geometry_batch_kernel<<<dim3(ge2_geo_blocks(T, max_pairs), n), kGe2GeoThreads,
+                                ge2_geo_smem(T), s>>>(T, slots, A);
     size_t smem = 0;
     for (int i = 0; i < n; ++i) smem = std::max(smem, ge2_apply_smem(T, T.n_bands * P[i].n_omega));
     if (smem > 48 * 1024)
@@ -1241,8 +1308,8 @@ static int ge2_tc_class_launch(const lh_ge2_table& T, const lh_ge2_problem* P, i
       cudaMemsetAsync(hs[i].P.result, 0, sizeof(double) * 2 * (size_t)hs[i].P.n_om * T.n_omega, s);
     return cudaGetLastError() == cudaSuccess ? LH_OK : LH_ECUDA;
   }
-  ge2_geometry_batch_kernel<<<dim3((unsigned)((max_pairs + 127) / 128), count), 128, 0, s>>>(T, slots,
-                                                                                      A);
+  ge2_geometry_batch_kernel<<<dim3(ge2_geo_blocks(T, max_pairs), count), kGe2GeoThreads,
+                              ge2_geo_smem(T), s>>>(T, slots, A);
   cudaMemsetAsync(counts, 0, sizeof(int32_t) * (T.n_intervals + 1), s);
   const unsigned bucket_blocks = (unsigned)std::min<int64_t>((max_pairs + 255) / 256, 148 * 4);
   ge2_tc_bucket_kernel<<<dim3(bucket_blocks, count), 256, 0, s>>>(slots, A, T.nch, counts, nullptr);
