@@ -136,32 +136,53 @@ LH_DEVICE O1Subseg o1_subseg(const lh_order1_elements& E, int64_t i, int64_t ia,
   return s;
 }
 
-constexpr int kO1CoopGroups = 8;  // at most this many groups per warp: summed by the whole warp
+// At most this many groups per warp are summed by the whole warp.
+constexpr int kO1CoopGroups = 16;
 
 // Warp-level sums by key: every lane writes its n values to its row of the
 // warp's staging area (`stage`, 32 rows of n doubles in shared memory), and
 // each group of lanes with equal keys (`group`, a __match_any_sync mask; its
 // lowest lane the `leader`, holding the group's `row`) adds its members' rows
-// in lane order with one atomic per value. With few groups the whole warp
-// takes one group at a time (lane k sums value k); with many, each leader
-// sums its own group's values one after another. Both sum in the same order.
+// in lane order with one atomic per value. Where the groups are few the warp
+// takes several at a time (three of 18 values, two of 23: a lane sums two
+// values of one group); with many, each leader sums its own group's values one
+// after another. Both sum in the same order.
 LH_DEVICE void o1_warp_group_add(double* stage, int n, unsigned group, bool leader, double* row) {
   __syncwarp();
   const unsigned full = 0xffffffffu;
   unsigned leaders = __ballot_sync(full, leader && row != nullptr);
   if (__popc(leaders) <= kO1CoopGroups) {
     const int lane = threadIdx.x & 31;
+    const int per = (n + 1) >> 1, at_once = min(32 / per, 3);  // n <= 32: at least two
+    const int place = lane / per, k = lane - place * per;
     while (leaders) {
-      const int src = __ffs(leaders) - 1;
+      int src = __ffs(leaders) - 1;
       leaders &= leaders - 1;
-      const unsigned members = __shfl_sync(full, group, src);
+      bool mine = place == 0;
+#pragma unroll
+      for (int i = 1; i < 3; ++i)
+        if (i < at_once && leaders) {  // the same for the whole warp
+          const int next = __ffs(leaders) - 1;
+          leaders &= leaders - 1;
+          if (place == i) {
+            src = next;
+            mine = true;
+          }
+        }
+      unsigned members = __shfl_sync(full, group, src);
       double* target = reinterpret_cast<double*>(
           __shfl_sync(full, reinterpret_cast<unsigned long long>(row), src));
-      for (int k = lane; k < n; k += 32) {
-        double sum = 0.0;
-        for (unsigned g = members; g; g &= g - 1) sum += stage[(__ffs(g) - 1) * n + k];
-        atomicAdd(target + k, sum);
+      if (!mine) continue;
+      const bool second = k + per < n;
+      const double* from = stage + k;
+      double sum0 = 0.0, sum1 = 0.0;
+      for (; members; members &= members - 1) {
+        const double* value = from + (__ffs(members) - 1) * n;
+        sum0 += value[0];
+        if (second) sum1 += value[per];
       }
+      atomicAdd(target + k, sum0);
+      if (second) atomicAdd(target + k + per, sum1);
     }
   } else if (leader && row) {
     for (int k = 0; k < n; ++k) {
@@ -534,7 +555,8 @@ LH_DEVICE void o1_write_pencil(const double* a, lh_order1_pencil_table& Pn, int 
 // rest of its warp waits. Each lane of `need` receives s0 = 1 / sqrt(scale),
 // scale = 2 (var_u + var_v) + u^2 + v^2 (its sums stay 0 when scale <= 0),
 // the sum of the node masses and of mass x the radial second moment. Call
-// with the whole warp.
+// with the whole warp; the second moment only with kRadial.
+template <bool kRadial>
 LH_DEVICE void o1_node_sums(unsigned need, double u, double v, double var_u, double var_v,
                             const double* tangent, const double* wsec2, int n, double& s0_out,
                             double& mass_out, double& radial_out) {
@@ -548,18 +570,22 @@ LH_DEVICE void o1_node_sums(unsigned need, double u, double v, double var_u, dou
     const double bvu = __shfl_sync(full, var_u, src), bvv = __shfl_sync(full, var_v, src);
     const double scale = 2.0 * (bvu + bvv) + bu * bu + bv * bv;
     if (scale <= 0.0) continue;  // the same for the whole warp
-    const double s0 = 1.0 / sqrt(scale);
+    const double s0 = rsqrt(scale);
+    const double uu = bu * bu, vv = bv * bv;
     double mass = 0.0, radial = 0.0;
     for (int k = lane; k < n; k += 32) {
-      const double t = s0 * tangent[k];
-      const double a = 1.0 + 2.0 * t * t * bvu, b = 1.0 + 2.0 * t * t * bvv;
-      const double m = wsec2[k] * exp(-t * t * (bu * bu / a + bv * bv / b)) / sqrt(a * b);
+      // a = 1 + 2 t^2 var_u, b likewise; their inverses from one reciprocal root
+      const double t = s0 * tangent[k], t2 = t * t;
+      const double a = fma(2.0 * t2, bvu, 1.0), b = fma(2.0 * t2, bvv, 1.0);
+      const double root = rsqrt(a * b), inv = root * root;  // 1 / sqrt(a b), 1 / (a b)
+      const double ia = b * inv, ib = a * inv;
+      const double m = wsec2[k] * exp(-t2 * (uu * ia + vv * ib)) * root;
       mass += m;
-      radial += m * (bvu / a + bvv / b + bu * bu / (a * a) + bv * bv / (b * b));
+      if (kRadial) radial += m * (ia * (bvu + uu * ia) + ib * (bvv + vv * ib));
     }
     for (int off = 16; off; off >>= 1) {
       mass += __shfl_xor_sync(full, mass, off);
-      radial += __shfl_xor_sync(full, radial, off);
+      if (kRadial) radial += __shfl_xor_sync(full, radial, off);
     }
     if (lane == src) {
       s0_out = s0;
@@ -607,16 +633,35 @@ LH_DEVICE bool o1_refined(const lh_order1_config& C, const lh_order1_pencil_tabl
                           double rx, double ry, double rz) {
   const double dx = rx - Pn.position[3 * x], dy = ry - Pn.position[3 * x + 1],
                dz = rz - Pn.position[3 * x + 2];
-  const double r = sqrt(dx * dx + dy * dy + dz * dz);
-  const double hx = dx / r, hy = dy / r, hz = dz / r;
+  const double inv_r = rsqrt(dx * dx + dy * dy + dz * dz);
+  const double hx = dx * inv_r, hy = dy * inv_r, hz = dz * inv_r;
   const double sx = Pn.direction[3 * x], sy = Pn.direction[3 * x + 1], sz = Pn.direction[3 * x + 2];
   const double cosine = hx * sx + hy * sy + hz * sz;
   const double qx = hx - cosine * sx, qy = hy - cosine * sy, qz = hz - cosine * sz;
-  const double theta = atan2(sqrt(qx * qx + qy * qy + qz * qz), cosine);
   const double* cov = Pn.pos_cov + 6 * x;
-  const double extent2 = Pn.var_major[x] + (cov[0] + cov[1] + cov[2]) / (r * r);
+  const double extent2 = Pn.var_major[x] + (cov[0] + cov[1] + cov[2]) * (inv_r * inv_r);
   const double sf = C.smoothing_factor;
+  // theta >= sin(theta): most pencils are decided without the angle
+  const double s2 = qx * qx + qy * qy + qz * qz;
+  if (!(s2 < sf * sf * extent2 * (1.0 + 1e-12))) return false;
+  const double theta = atan2(sqrt(s2), cosine);
   return theta < 0.5 * kPi && theta * theta < sf * sf * extent2;
+}
+
+// floor(log(x) * scale + shift) of a positive normal x: the hardware's float32
+// logarithm decides it wherever its value is further than 2e-3 from a whole number
+// (its error is below 1.8e-3 for |scale| <= 64 and |value| < 1024: three ulp of a
+// logarithm below 70), the float64 logarithm elsewhere, so the result is the
+// float64 one.
+LH_DEVICE int o1_log_floor(double x, double scale, double shift) {
+  const float xf = (float)x;
+  if (xf > 1e-30f && xf < 1e30f && fabs(scale) <= 64.0) {
+    const float lf = __logf(xf);
+    const float v = fmaf(lf, (float)scale, (float)shift);
+    const float f = floorf(v), part = v - f;
+    if (part > 2e-3f && part < 1.0f - 2e-3f && fabsf(v) < 1024.0f) return (int)f;
+  }
+  return (int)floor(fma(log(x), scale, shift));
 }
 
 constexpr int kO1GroupOms = 8;       // work OMs per warp chunk of the group stage
@@ -652,7 +697,16 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
   }
   __syncthreads();
   const int n_values = 2 * C.n_mono + 6;
-  const double log_theta_ratio = log(1.0 + C.theta_ratio);
+  // the monomials of a quadratic acceptance in their usual order: their powers in
+  // registers instead of arrays indexed at run time
+  const bool quadratic =
+      C.n_mono == 6 && S.ipow[0] == 0 && S.jpow[0] == 0 && S.ipow[1] == 0 && S.jpow[1] == 1 &&
+      S.ipow[2] == 1 && S.jpow[2] == 0 && S.ipow[3] == 0 && S.jpow[3] == 2 && S.ipow[4] == 1 &&
+      S.jpow[4] == 1 && S.ipow[5] == 2 && S.jpow[5] == 0;
+  const double theta_scale = 1.0 / log(1.0 + C.theta_ratio);
+  const double theta_shift = -log(C.theta_lo) * theta_scale;
+  const double log_r_scale = 0.5 / C.log_r_step;  // of log(r^2)
+  const double tau_scale = 1.0 / C.tau_step, inv_speed = 1.0 / C.speed_ref;
   const int theta_bins = C.theta_bins;
   const int64_t cap = C.group_capacity;
   // the pencil count is read on the device when given (no host round trip)
@@ -701,16 +755,20 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
     const double nx = C.om_look[3 * d], ny = C.om_look[3 * d + 1], nz = C.om_look[3 * d + 2];
     // _prepare_receiver_geometry (_prompt_numba.py:1590-1612)
     const double dx = rx - pen[0], dy = ry - pen[32], dz = rz - pen[64];
-    const double r = sqrt(dx * dx + dy * dy + dz * dz);
-    const double hx = dx / r, hy = dy / r, hz = dz / r;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double inv_r = rsqrt(r2), r = r2 * inv_r;
+    const double hx = dx * inv_r, hy = dy * inv_r, hz = dz * inv_r;
     // the screen's charge batches ignore emission time (_prompt_screen.py:220-229)
     const double t_emit = kScreen ? 0.0 : pen[96] - origins[d];
-    const double tau = kScreen ? 0.0 : t_emit + r / C.speed_ref;
-    const double log_r = log(r);
-    const long long key0 = (long long)floor(log_r / C.log_r_step) + (1ll << 20);
-    const long long key1 =
-        min(max((long long)floor(tau / C.tau_step) + (1ll << 20), 0ll), (1ll << 21) - 1);
-    const long long base = kScreen ? key0 * 2 * theta_bins : ((key1 << 21) + key0) * 2 * theta_bins;
+    const double tau = kScreen ? 0.0 : fma(r, inv_speed, t_emit);
+    const long long key0 = (long long)o1_log_floor(r2, log_r_scale, 0.0) + (1ll << 20);
+    long long base = key0 * 2 * theta_bins;
+    if (!kScreen) {
+      const int tau_bin = __double2int_rd(tau * tau_scale);  // saturates
+      const long long key1 =
+          (long long)(min(max(tau_bin, -(1 << 20)), (1 << 20) - 1) + (1 << 20));
+      base = ((key1 << 21) + key0) * 2 * theta_bins;
+    }
     if (kScreen && live) {  // a parent unless the OM looks into it, else its children
       // rows of a table whose stage A overflowed are not written (the caller
       // redoes it): an index outside the table is never followed
@@ -726,8 +784,10 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
     const double c1 = sx * nx + sy * ny + sz * nz;
     const double cosine = hx * sx + hy * sy + hz * sz;
     const double qx = hx - cosine * sx, qy = hy - cosine * sy, qz = hz - cosine * sz;
-    const double sine = sqrt(qx * qx + qy * qy + qz * qz);
-    const double c3 = sine > 1e-300 ? (qx * nx + qy * ny + qz * nz) / sine : 0.0;
+    const double s2 = qx * qx + qy * qy + qz * qz;
+    const bool off_axis = s2 > 0.0;
+    const double inv_sine = off_axis ? rsqrt(s2) : 0.0, sine = s2 * inv_sine;
+    const double c3 = (qx * nx + qy * ny + qz * nz) * inv_sine;
     double theta = atan2(sine, cosine);
     const bool backward = theta > 0.5 * kPi;
     double weight = 0.0, weight2 = 0.0, theta2 = theta;
@@ -747,11 +807,12 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
     double u_ = 0.0, v_ = 0.0, r_extent = 0.0;
     double arg_u = 0.0, arg_v = 0.0, arg_var_u = 0.0, arg_var_v = 0.0;  // of the node sums
     if (backward) {
-      weight = 1.0 / r;
+      weight = inv_r;
     } else {
-      const double bound = pen[320] + pen[352] + trace / (r * r);
-      if (sine > 1e-300 && bound < 1e-4 * sine * sine) {
-        weight = (1.0 / sine) / r;
+      const double inv_r2 = inv_r * inv_r;
+      const double bound = pen[320] + pen[352] + trace * inv_r2;
+      if (off_axis && bound < 1e-4 * s2) {
+        weight = inv_sine * inv_r;
       } else {
         // _pencil_shape_factor_from_ray (_prompt_numba.py:1389-1436)
         const double caa = ax * (cov[0] * ax + cov[3] * ay + cov[4] * az) +
@@ -763,7 +824,6 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
         const double cab = ax * (cov[0] * bx + cov[3] * by + cov[4] * bz) +
                            ay * (cov[3] * bx + cov[1] * by + cov[5] * bz) +
                            az * (cov[4] * bx + cov[5] * by + cov[2] * bz);
-        const double inv_r2 = 1.0 / (r * r);
         m11 = pen[320] + caa * inv_r2;
         m22 = pen[352] + cbb * inv_r2;
         m12 = cab * inv_r2;
@@ -789,7 +849,7 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
           const double r_mu2 = fmax(half_tr - disc, 1e-16 * r_mu1 + 1e-300);
           r_extent = sqrt(fmax(r_mu1, 0.0));
           if (r_extent > 0.0 && theta < sf * r_extent) {
-            const double st = sine > 0.0 ? theta / sine : 1.0;
+            const double st = off_axis ? theta * inv_sine : 1.0;
             const double uu = u_ * st, vv = v_ * st;
             double sa, ca;
             sincos(0.5 * atan2(2.0 * m12, m11 - m22), &sa, &ca);
@@ -807,7 +867,7 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
     double s0n, mass, radial;
     const unsigned need_rule = __ballot_sync(full, mode == 1);
     if (need_rule) {
-      o1_node_sums(need_rule, arg_u, arg_v, arg_var_u, arg_var_v, S.tangent, S.wsec2, C.n_gauss,
+      o1_node_sums<true>(need_rule, arg_u, arg_v, arg_var_u, arg_var_v, S.tangent, S.wsec2, C.n_gauss,
                    s0n, mass, radial);
       if (mode == 1) {
         double w0r, t0r, w1r, t1r;
@@ -815,8 +875,8 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
                                w1r, t1r);
         if (t0r > 0.0 && t1r < 0.5 * kPi && w0r > 0.0 && w1r >= 0.0) {
           averaged = theta < r_extent;
-          weight = (w0r * t0r / sin(t0r)) / r;
-          weight2 = (w1r * t1r / sin(t1r)) / r;
+          weight = (w0r * t0r / sin(t0r)) * inv_r;
+          weight2 = (w1r * t1r / sin(t1r)) * inv_r;
           theta = t0r;
           theta2 = t1r;
           mode = 0;
@@ -835,36 +895,28 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
     }
     const unsigned need_mean = __ballot_sync(full, mode == 2);
     if (need_mean) {
-      o1_node_sums(need_mean, arg_u, arg_v, arg_var_u, arg_var_v, S.tangent, S.wsec2, C.n_gauss,
+      o1_node_sums<false>(need_mean, arg_u, arg_v, arg_var_u, arg_var_v, S.tangent, S.wsec2, C.n_gauss,
                    s0n, mass, radial);
       if (mode == 2) {
         const double mean = o1_gauss_inverse_mean(arg_u, arg_v, arg_var_u, arg_var_v, s0n, mass);
-        const double factor = mean * (sine > 1e-300 ? theta / sine : 1.0);
+        const double factor = mean * (off_axis ? theta * inv_sine : 1.0);
         averaged = theta < extent;
         theta = factor > 1.0 ? asin(fmin(1.0, 1.0 / factor)) : theta;
-        weight = factor / r;
+        weight = factor * inv_r;
       }
     }
     if (mode == 3) {
-      if (sine <= 1e-300) live = false;
+      if (!off_axis) live = false;
       const double d2 = u_ * u_ + v_ * v_;
-      double factor = 1.0 / sine;
+      double factor = inv_sine;
       if (d2 > 0.0) {
         const double qf = m11 * u_ * u_ + 2.0 * m12 * u_ * v_ + m22 * v_ * v_;
-        factor *= 1.0 + 0.5 * (3.0 * qf / d2 - (m11 + m22)) / d2;
+        const double inv_d2 = 1.0 / d2;
+        factor *= 1.0 + 0.5 * (3.0 * qf * inv_d2 - (m11 + m22)) * inv_d2;
       }
-      weight = factor / r;
+      weight = factor * inv_r;
     }
-    // _fill_moments_averaged_pair (_prompt_numba.py:1260-1277): the angular powers
-    double cpw[5], spw[5];
-    cpw[0] = 1.0;
-    spw[0] = 1.0;
     const double perp2 = fmax(1.0 - c1 * c1, 0.0);
-    for (int q = 1; q <= C.max_power; ++q) {
-      cpw[q] = cpw[q - 1] * c1;
-      if (averaged) spw[q] = (q & 1) ? 0.0 : spw[q - 2] * perp2 * (q - 1.0) / q;
-      else spw[q] = spw[q - 1] * c3;
-    }
     const int nm = C.n_mono;
     // one group entry per radial node: the screen's two-node rule adds a second
     // (_prompt_screen.py:281-336); every lane of the warp takes both rounds
@@ -874,14 +926,13 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
       const double wn = node == 0 ? weight : weight2;
       const double th = node == 0 ? theta : theta2;
       // theta index (scalar_theta_index, _prompt_numba.py:1628-1631)
-      int i_theta;
-      if (!(th >= C.theta_lo)) i_theta = 0;
-      else i_theta = min(1 + (int)(log(th / C.theta_lo) / log_theta_ratio), theta_bins - 1);
+      int i_theta = 0;
+      if (th >= C.theta_lo)
+        i_theta = min(1 + max(o1_log_floor(th, theta_scale, theta_shift), 0), theta_bins - 1);
       const long long key = base + (backward ? theta_bins : 0) + i_theta;
-      // lanes with the same (OM, group key) sum their moments in registers; the
+      // lanes with the same group key (the OM is the warp's) sum their moments; the
       // group's lowest lane inserts the key and adds the sums
-      const unsigned group = __match_any_sync(0xffffffffu, live_n ? key : -1ll) &
-                             __match_any_sync(0xffffffffu, live_n ? w : -1);
+      const unsigned group = __match_any_sync(0xffffffffu, live_n ? key : -1ll);
       const bool leader = live_n && lane == __ffs(group) - 1;
       double* row = nullptr;
       if (leader) {
@@ -895,14 +946,35 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
         }
       }
       const double field0 = wn * pen[576], field2 = wn * pen[608];
-      double omega = 0.0;
+      // the angular powers (_fill_moments_averaged_pair, _prompt_numba.py:1260-1277)
+      double omega;
       double* mine = stage + lane * n_values;
-      for (int m = 0; m < nm; ++m) {
-        const double basis = cpw[S.ipow[m]] * spw[S.jpow[m]];
-        const double v0 = field0 * basis;
-        if (m == 0) omega = fabs(v0);
-        mine[m] = v0;
-        mine[nm + m] = field2 * basis;
+      if (quadratic) {
+        const double p1 = averaged ? 0.0 : c3, p2 = averaged ? 0.5 * perp2 : c3 * c3;
+        const double basis[6] = {1.0, p1, c1, p2, c1 * p1, c1 * c1};
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+          mine[m] = field0 * basis[m];
+          mine[6 + m] = field2 * basis[m];
+        }
+        omega = fabs(field0);
+      } else {
+        double cpw[5], spw[5];
+        cpw[0] = 1.0;
+        spw[0] = 1.0;
+        for (int q = 1; q <= C.max_power; ++q) {
+          cpw[q] = cpw[q - 1] * c1;
+          if (averaged) spw[q] = (q & 1) ? 0.0 : spw[q - 2] * perp2 * (q - 1.0) / q;
+          else spw[q] = spw[q - 1] * c3;
+        }
+        omega = 0.0;
+        for (int m = 0; m < nm; ++m) {
+          const double basis = cpw[S.ipow[m]] * spw[S.jpow[m]];
+          const double v0 = field0 * basis;
+          if (m == 0) omega = fabs(v0);
+          mine[m] = v0;
+          mine[nm + m] = field2 * basis;
+        }
       }
       mine[2 * nm] = omega;
       mine[2 * nm + 1] = omega * th;

@@ -176,3 +176,33 @@ def test_long_path_grids_match_the_oracle(step):
         merge=(float(g["merge_theta_min"]), float(g["merge_theta_ratio"]),
                float(g["merge_tau_ns"]), float(g["merge_log_r"])))
     check(q.cpu().numpy(), b.cpu().numpy(), q_ref, b_ref)
+
+
+@pytest.mark.parametrize("alpha, log_r", [((6.0, 1.9), 0.02), ((6.0, 1.9, 0.2, 0.05), 0.02),
+                                          ((6.0, 1.9, 0.2), 0.004), ((6.0, 1.9, 0.2), 0.3)])
+def test_acceptance_degrees_and_group_steps_match_the_oracle(alpha, log_r):
+    """Acceptances of degree 1, 2 and 3 (degree 2 keeps its monomials in registers,
+    the others take the general loop) and radius steps whose group index the
+    float32 logarithm estimate may and may not decide: stage B on the
+    reference's pencils against the oracle's grouped order 1."""
+    from dataclasses import replace
+    from lighthit_b200.order1 import Order1Tables, PencilTable, acceptance_monomials, grouped
+    from oracle import order1 as O1
+    g = fixture()
+    mono = acceptance_monomials(alpha)
+    s = replace(tables_of(g).settings, merge_log_r=log_r)
+    bands = {k: g[k] for k in ("mus", "mut", "speed", "s0w", "s2w")}
+    tables = Order1Tables(bands, float(g["g"]), mono, g["positions_m"], g["looks"],
+                          g["areas_m2"], g["edges_ns"], settings=s)
+    pencils = {k: g[f"sub_pencil_{k}"] for k in PENCIL_KEYS}
+    table, n = PencilTable.from_host(pencils, tables.device)
+    work = np.array([0, 11, 30, 47])
+    q, b = grouped(tables, table, work, g["origins_ns"], n_pencils=n)
+    q_ref, b_ref, _, _ = O1.grouped(
+        pencils, g["positions_m"], g["looks"], g["areas_m2"], g["origins_ns"], work, mono,
+        float(g["g"]), bands, g["edges_ns"], path_step=s.path_step,
+        path_step_tail=s.path_step_tail, tail_exponent=s.tail_exponent,
+        direct_bins=s.direct_bins, max_path_nodes=s.max_path_nodes,
+        smoothing_factor=s.smoothing_factor,
+        merge=(s.merge_theta_min, s.merge_theta_ratio, s.merge_tau_ns, log_r))
+    check(q.cpu().numpy(), b.cpu().numpy(), q_ref, b_ref)
