@@ -667,6 +667,13 @@ LH_DEVICE int o1_log_floor(double x, double scale, double shift) {
 constexpr int kO1GroupOms = 8;       // work OMs per warp chunk of the group stage
 constexpr int kO1PencilFields = 20;  // float64 fields of a pencil read by the group stage
 
+// The monomials of a quadratic acceptance in their usual order.
+LH_DEVICE bool o1_quadratic(const lh_order1_config& C, const int* ipow, const int* jpow) {
+  return C.n_mono == 6 && ipow[0] == 0 && jpow[0] == 0 && ipow[1] == 0 && jpow[1] == 1 &&
+         ipow[2] == 1 && jpow[2] == 0 && ipow[3] == 0 && jpow[3] == 2 && ipow[4] == 1 &&
+         jpow[4] == 1 && ipow[5] == 2 && jpow[5] == 0;
+}
+
 struct O1GroupShared {
   double tangent[kO1MaxGauss], wsec2[kO1MaxGauss];
   double coef[kO1MaxMono];
@@ -699,10 +706,7 @@ o1_group_kernel(const lh_order1_config C, const lh_order1_pencil_table Pn,
   const int n_values = 2 * C.n_mono + 6;
   // the monomials of a quadratic acceptance in their usual order: their powers in
   // registers instead of arrays indexed at run time
-  const bool quadratic =
-      C.n_mono == 6 && S.ipow[0] == 0 && S.jpow[0] == 0 && S.ipow[1] == 0 && S.jpow[1] == 1 &&
-      S.ipow[2] == 1 && S.jpow[2] == 0 && S.ipow[3] == 0 && S.jpow[3] == 2 && S.ipow[4] == 1 &&
-      S.jpow[4] == 1 && S.ipow[5] == 2 && S.jpow[5] == 0;
+  const bool quadratic = o1_quadratic(C, S.ipow, S.jpow);
   const double theta_scale = 1.0 / log(1.0 + C.theta_ratio);
   const double theta_shift = -log(C.theta_lo) * theta_scale;
   const double log_r_scale = 0.5 / C.log_r_step;  // of log(r^2)
@@ -1068,33 +1072,33 @@ o1_batches_kernel(const lh_order1_config C, int32_t n_work, const long long* gke
   (void)status;
 }
 
-// _ifuncs (_prompt_numba.py:139-154): I_k(z) = int_0^1 x^k e^{z x} dx, k = 0, 1, 2
+// _ifuncs (_prompt_numba.py:139-154): I_k(z) = int_0^1 x^k e^{z x} dx, k = 0, 1, 2,
+// with ez = e^z. Below |z| = 1 the series of I_2 (sum z^n / (n! (n + 3)); 19 terms
+// reach 1e-18), then I_1 and I_0 by parts, I_{k-1} = (e^z - z I_k) / k.
 LH_DEVICE void o1_ifuncs(double z, double ez, double& i0, double& i1, double& i2) {
   if (fabs(z) < 1.0) {
-    // Taylor coefficients 1 / (n! (n + j + 1)), Horner from n = 23
-    double f = 1.0;  // 1/n!
-    double c0[24], c1[24], c2[24];
-    for (int n = 0; n < 24; ++n) {
+    constexpr int kTerms = 19;
+    double f = 1.0, c[kTerms];
+#pragma unroll
+    for (int n = 0; n < kTerms; ++n) {
       if (n > 0) f /= n;
-      c0[n] = f / (n + 1.0);
-      c1[n] = f / (n + 2.0);
-      c2[n] = f / (n + 3.0);
+      c[n] = f / (n + 3.0);
     }
-    i0 = c0[23]; i1 = c1[23]; i2 = c2[23];
-    for (int n = 22; n >= 0; --n) {
-      i0 = i0 * z + c0[n];
-      i1 = i1 * z + c1[n];
-      i2 = i2 * z + c2[n];
-    }
+    i2 = c[kTerms - 1];
+#pragma unroll
+    for (int n = kTerms - 2; n >= 0; --n) i2 = fma(i2, z, c[n]);
+    i1 = 0.5 * fma(-z, i2, ez);
+    i0 = fma(-z, i1, ez);
     return;
   }
-  i0 = (ez - 1.0) / z;
-  i1 = (ez * (z - 1.0) + 1.0) / (z * z);
-  i2 = (ez * (z * z - 2.0 * z + 2.0) - 2.0) / (z * z * z);
+  const double inv = 1.0 / z;
+  i0 = (ez - 1.0) * inv;
+  i1 = (ez - i0) * inv;
+  i2 = (ez - 2.0 * i1) * inv;
 }
 
 // _quad_integral (_prompt_numba.py:158-163)
-LH_DEVICE double o1_quad(double e_start, double alpha, double beta, double gamma, double width,
+__device__ __noinline__ double o1_quad(double e_start, double alpha, double beta, double gamma, double width,
                          double kappa, double e_end) {
   const double z = kappa * width;
   const double ez = e_start > 0.0 ? e_end / e_start : exp(z);
@@ -1117,7 +1121,7 @@ LH_DEVICE int o1_find_bin(const double* edges, int nb, double t) {
 
 // _deposit_panel (_prompt_numba.py:186-254) into the OM's accumulators
 // pre[3] and acc[nb][4] of one band.
-LH_DEVICE void o1_deposit_panel(double t_a, double t_b, double e_a, double e_b, double alpha,
+__device__ __noinline__ void o1_deposit_panel(double t_a, double t_b, double e_a, double e_b, double alpha,
                                 double beta, double gamma, double kappa, const double* edges,
                                 const double* eedge, int nb, double* pre, double* acc,
                                 int direct_bins) {
@@ -1171,68 +1175,440 @@ LH_DEVICE void o1_deposit_panel(double t_a, double t_b, double e_a, double e_b, 
 }
 
 struct O1BandDeposit {
-  double v, kappa, spread, t_base, e_emit, w0, w2, h_front, total;
+  double v, kappa, spread, t_base, e_emit, w0, w2, h_front;
   int last, pairs, panels;
   bool outside;
 };
 
-// NODES: the path-grid nodes a CTA holds in shared memory (kO1SmallNodes for
-// the common short grids, kO1MaxNodes for the rest).
-constexpr int kO1SmallNodes = 512;
+// What the batch's path grid and deposit need: mean radius and emission time,
+// front width, grid scale, its two ends and node counts.
+struct O1BatchGrid {
+  double r_b, t_b, front_extra, sigma, u_win, u_end;
+  int n_in, n_out, n;  // n = n_in + n_out + 1 nodes, 0: nothing to deposit
+  bool backward;
+};
 
-template <int NODES>
+// The batch's grid from its groups' sums (_batch_sigma, _batch_grid:
+// _prompt_numba.py:258-292).
+LH_DEVICE O1BatchGrid o1_batch_grid(const lh_order1_config& C, bool backward, double omega_sum,
+                                    double r_sum, double t_sum, double tau_sum, double tau2_sum,
+                                    double theta_small, double mut_min, double speed_max,
+                                    int32_t* status) {
+  O1BatchGrid G{};
+  G.backward = backward;
+  if (!(omega_sum > 0.0)) return G;
+  const int nb = C.n_edges - 1;
+  const double inv = 1.0 / omega_sum;
+  const double r_b = r_sum * inv, t_b = t_sum * inv, tau_mean = tau_sum * inv;
+  const double tau_var = fmax(tau2_sum * inv - tau_mean * tau_mean, 0.0);
+  const double g = C.g;
+  const double y_g = g != 0.0 ? (1.0 - fabs(g)) / (1.0 + fabs(g)) : 1.0;
+  theta_small = fmax(theta_small, 1e-9);
+  double sin_t, cos_t;
+  sincos(theta_small, &sin_t, &cos_t);
+  double sigma;
+  if (backward)
+    sigma = fmax(0.5 * r_b * sin_t * y_g, 0.25 * r_b * (1.0 - cos_t));
+  else
+    sigma = fmax(0.5 * r_b * sin_t * fmax(y_g, 0.5 * tan(0.5 * theta_small)), 1e-9 * r_b);
+  const double ext_end = C.tail_exponent / mut_min;
+  // the screen's grids run to the tail without a window edge
+  // (_prompt_screen.py:413: edge_end = inf)
+  double ext_win = C.screen ? ext_end : speed_max * (C.edges[nb] - t_b) - r_b;
+  ext_win = fmin(fmax(ext_win, 0.0), ext_end);
+  double u_end = 0.0, u_win = 0.0;
+#pragma unroll 1
+  for (int i = 0; i < 2; ++i) {  // one copy of asinh
+    u_end = u_win;
+    u_win = asinh((i ? ext_win : ext_end) / sigma);
+  }
+  if (!(u_win >= 0.0) || !(u_end >= u_win) || !(u_end < 1e6)) {
+    atomicOr(reinterpret_cast<unsigned*>(status), LH_STATUS_OVERFLOW);
+    return G;
+  }
+  long long n_in = u_win > 0.0 ? (long long)ceil(u_win / C.path_step) : 0;
+  long long n_out = u_end > u_win ? (long long)ceil((u_end - u_win) / C.path_step_tail) : 0;
+  const int capacity = C.max_path_nodes;
+  if (n_in + n_out + 1 > capacity) {
+    const double scale = (capacity - 1.0) / (double)(n_in + n_out);
+    n_in = (long long)(n_in * scale);
+    n_out = capacity - 1 - n_in;
+  }
+  G.r_b = r_b; G.t_b = t_b; G.front_extra = sqrt(12.0 * tau_var);
+  G.sigma = sigma; G.u_win = u_win; G.u_end = u_end;
+  G.n_in = (int)n_in; G.n_out = (int)n_out;
+  G.n = (int)(n_in + n_out + 1);
+  return G;
+}
+
+LH_DEVICE double o1_batch_node(const O1BatchGrid& G, int k) {
+  if (k == 0) return G.r_b;
+  const double u = k <= G.n_in ? G.u_win * k / G.n_in
+                               : G.u_win + (G.u_end - G.u_win) * (k - G.n_in) / G.n_out;
+  return G.r_b + G.sigma * sinh(u);
+}
+
+// Profile at path s of the groups [q0, q1): _batch_add_moments
+// (_prompt_numba.py:394-447), generic monomials. `mom` holds rows of nv values.
+LH_DEVICE void o1_batch_profile(const lh_order1_config& C, const O1BatchGrid& G, double s,
+                                const double* mom, int nv, const double* sin_q,
+                                const double* cos_q, const double* coef, const int* ipow,
+                                const int* jpow, bool quadratic, int q0, int q1, double& out0,
+                                double& out2) {
+  const int nm = C.n_mono;
+  const double g = C.g, g1 = 1.0 + g * g, gg = 2.0 * g, norm = (1.0 - g * g) / (4.0 * kPi);
+  double a0s = 0.0, a2s = 0.0;
+  for (int q = q0; q < q1; ++q) {
+    const double* row = mom + q * nv;
+    if (row[2 * nm] <= 0.0) continue;
+    const double sin_t = sin_q[q], cos_t = cos_q[q];
+    const double rs = G.r_b * sin_t;
+    double c, sn, path_jacobian;
+    if (G.backward) {
+      const double shift = s - G.r_b * cos_t;
+      const double inv = 1.0 / (rs * rs + shift * shift);
+      c = (rs * rs - shift * shift) * inv;
+      sn = 2.0 * rs * shift * inv;
+      path_jacobian = 2.0 * G.r_b * inv;
+    } else {
+      const double inv_rs = 1.0 / rs;
+      const double y = (s - G.r_b) * inv_rs + sin_t / (1.0 + cos_t);
+      const double inv = 1.0 / (1.0 + y * y);
+      c = (1.0 - y * y) * inv;
+      sn = 2.0 * y * inv;
+      path_jacobian = 2.0 * inv_rs * inv;
+    }
+    double a0 = 0.0, a2 = 0.0;
+    if (quadratic) {
+      const double basis[6] = {coef[0], coef[1] * sn, coef[2] * c, coef[3] * (sn * sn),
+                               coef[4] * (c * sn), coef[5] * (c * c)};
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        a0 += basis[m] * row[m];
+        a2 += basis[m] * row[6 + m];
+      }
+    } else {
+      double cpw[5], spw[5];
+      cpw[0] = 1.0;
+      spw[0] = 1.0;
+      for (int pw = 1; pw <= C.max_power; ++pw) {
+        cpw[pw] = cpw[pw - 1] * c;
+        spw[pw] = spw[pw - 1] * sn;
+      }
+      for (int m = 0; m < nm; ++m) {
+        const double basis = coef[m] * cpw[ipow[m]] * spw[jpow[m]];
+        a0 += basis * row[m];
+        a2 += basis * row[nm + m];
+      }
+    }
+    const double root = rsqrt(g1 - gg * c);
+    const double value = path_jacobian * norm * (root * root * root);
+    a0s += a0 * value;
+    a2s += a2 * value;
+  }
+  out0 = a0s;
+  out2 = a2s;
+}
+
+// A band's deposit constants (_batch_deposit, _prompt_numba.py:451-551).
+LH_DEVICE void o1_band_setup(const lh_order1_config& C, const O1BatchGrid& G, int lam,
+                             const double* s, const double* g0, const double* g2,
+                             O1BandDeposit& B) {
+  const int nb = C.n_edges - 1;
+  B.panels = 0;
+  B.pairs = 0;
+  if (C.mus[lam] == 0.0) return;
+  const double v = C.speed[lam];
+  int last = G.n - 1;
+  const double limit = G.r_b + C.tail_exponent / C.mut[lam];
+  while (last > 2 && s[last - 1] > limit) last -= 1;
+  if (last < 2) return;
+  B.v = v;
+  B.kappa = -C.mut[lam] * v;
+  B.last = last;
+  B.spread = fmin(G.front_extra, (s[last] - G.r_b) / v);
+  const double front_time = G.t_b + G.r_b / v;
+  const double end_time = G.t_b + s[last] / v;
+  B.outside = front_time - 0.5 * B.spread >= C.edges[nb] ||
+              end_time + 0.5 * B.spread <= C.edges[0];
+  B.t_base = B.outside ? 0.0 : G.t_b;
+  B.e_emit = exp(B.kappa * B.t_base);
+  const double h_scale = C.mus[lam] * v / B.e_emit;
+  B.w0 = C.s0w[lam] * h_scale;
+  B.w2 = C.s2w[lam] * h_scale;
+  B.h_front = B.w0 * g0[0] + B.w2 * g2[0];
+  // panels start at even nodes with step 2; an odd `last` ends with one step
+  B.pairs = last / 2;
+  B.panels = B.pairs + (last & 1);
+}
+
+// Panel pi of band lam: its integral (returned) and its deposit into the bins.
+LH_DEVICE double o1_panel(const lh_order1_config& C, const O1BandDeposit& B, int lam, int pi,
+                          const double* s, const double* g0, const double* g2, double* pre) {
+  const int nb = C.n_edges - 1;
+  const double inv_v = 1.0 / B.v, mut = C.mut[lam];
+  auto node_t = [&](int j) { return B.t_base + s[j] * inv_v; };
+  auto node_h = [&](int j) { return (B.w0 * g0[j] + B.w2 * g2[j]) - B.h_front; };
+  // the parabola through nodes j, j + 1, j + 2: a panel spans both steps, the
+  // single last step of an odd grid only the second
+  const bool tail = pi >= B.pairs;
+  const int j = tail ? B.last - 2 : 2 * pi;
+  const double t0 = node_t(j), t1 = node_t(j + 1), t_b2 = node_t(j + 2);
+  const double h0 = node_h(j), h1 = node_h(j + 1), h2 = node_h(j + 2);
+  const double u_m = t1 - t0;
+  const double d1 = (h1 - h0) / u_m;
+  const double gamma = ((h2 - h1) / (t_b2 - t1) - d1) / (t_b2 - t0);
+  const double t_a = tail ? t1 : t0, alpha = tail ? h1 : h0;
+  const double beta = tail ? d1 - gamma * u_m + 2.0 * gamma * u_m : d1 - gamma * u_m;
+  const double e_a = B.e_emit * exp(-mut * s[tail ? j + 1 : j]);
+  const double e_b = B.e_emit * exp(-mut * s[j + 2]);
+  if (pre)
+    o1_deposit_panel(t_a, t_b2, e_a, e_b, alpha, beta, gamma, B.kappa, C.edges,
+                     C.eedge + (int64_t)lam * C.n_edges, nb, pre, pre + 3, C.direct_bins);
+  return o1_quad(e_a, alpha, beta, gamma, t_b2 - t_a, B.kappa, e_b);
+}
+
+// The front step of band lam as a mass-normalised ramp of width `spread`; adds
+// the band's charge (`total`: its panels') and deposits the ramp.
+LH_DEVICE void o1_front(const lh_order1_config& C, const O1BandDeposit& B, int lam,
+                        const double* s, double total, double* pre, double* chg) {
+  const int nb = C.n_edges - 1;
+  const double* eedge = C.eedge + (int64_t)lam * C.n_edges;
+  const double e_first = B.e_emit * exp(-C.mut[lam] * s[0]);
+  const double e_last = B.e_emit * exp(-C.mut[lam] * s[B.last]);
+  const double t_f = B.t_base + s[0] / B.v, t_end = B.t_base + s[B.last] / B.v;
+  const double spread = B.spread, kappa = B.kappa;
+  const double exact = o1_quad(e_first, B.h_front, 0.0, 0.0, t_end - t_f, kappa, e_last);
+  atomicAdd(chg, total + exact);
+  if (!pre) return;
+  // the step's part behind the ramp: from t_2 at `height` to the end
+  double t_2 = t_f, e_2 = e_first, height = B.h_front;
+  if (spread > 0.0) {
+    const double t_1 = t_f - 0.5 * spread;
+    t_2 = t_f + 0.5 * spread;
+    const double e_1 = exp(kappa * t_1);
+    e_2 = exp(kappa * t_2);
+    const double ramp = o1_quad(e_1, 0.0, 1.0 / spread, 0.0, spread, kappa, e_2);
+    const double flat = t_end > t_2 ? o1_quad(e_2, 1.0, 0.0, 0.0, t_end - t_2, kappa, e_last) : 0.0;
+    height = ramp + flat != 0.0 ? exact / (ramp + flat) : 0.0;
+    o1_deposit_panel(t_1, t_2, e_1, e_2, 0.0, height / spread, 0.0, kappa, C.edges, eedge,
+                     nb, pre, pre + 3, C.direct_bins);
+  }
+  if (t_end > t_2)
+    o1_deposit_panel(t_2, t_end, e_2, e_last, height, 0.0, 0.0, kappa, C.edges, eedge, nb,
+                     pre, pre + 3, C.direct_bins);
+}
+
+LH_DEVICE void o1_band_extremes(const lh_order1_config& C, double& mut_min, double& speed_max) {
+  mut_min = C.mut[0];
+  speed_max = C.speed[0];
+  for (int l = 1; l < C.n_bands; ++l) {
+    mut_min = fmin(mut_min, C.mut[l]);
+    speed_max = fmax(speed_max, C.speed[l]);
+  }
+}
+
+// _grouped_pencils_order1_block's batch loop (_prompt_numba.py:1934-1993) with
+// _batch_grid, _batch_add_moments and _batch_deposit (_prompt_numba.py:258-551),
+// one warp per batch. A batch is small (typically 7 groups, 33 path nodes and 51
+// (band, panel) items), so its steps are chains of short loops: with a CTA of four
+// warps per batch they waited on one another (barrier 13 of 25 stall cycles per
+// issue, 0.61 ms for 8400 batches); a warp needs no barrier and 20 of them per SM
+// work on batches of their own (0.22 ms, and 0.035 ms for the deferred ones; 3, 4
+// or 6 CTAs per SM are 1-3 % slower). What is left is the latency of one batch's
+// float64 chain, ~40 us, and its instruction fetch. Batches with more than
+// kO1WarpNodes nodes or kO1WarpGroups groups go to `deferred`.
+constexpr int kO1WarpNodes = 128;
+constexpr int kO1WarpGroups = 32;
+constexpr int kO1WarpSums = 256;  // (node, part) sums of the profile
+constexpr int kO1BatchWarps = 4;  // per CTA
+
+struct O1WarpBatch {
+  double s[kO1WarpNodes];
+  double g0[kO1WarpSums], g2[kO1WarpSums];
+  double sin_q[kO1WarpGroups], cos_q[kO1WarpGroups];
+  O1BandDeposit band[kO1MaxBands];
+};
+
+static size_t o1_warp_batch_bytes(const lh_order1_config& C) {
+  return kO1BatchWarps *
+         (sizeof(O1WarpBatch) + sizeof(double) * kO1WarpGroups * (size_t)(2 * C.n_mono + 6));
+}
+
+LH_DEVICE double o1_warp_sum(double v) {
+  for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+__global__ void __launch_bounds__(32 * kO1BatchWarps, 5)
+o1_batch_warp_kernel(const lh_order1_config C, const long long* gkeys, const double* grows,
+                     const int32_t* sorted_slots, const int32_t* batch_list,
+                     const int32_t* batch_total, int32_t* deferred, int32_t* n_deferred,
+                     double* accum, int32_t* status) {
+  extern __shared__ __align__(16) unsigned char o1w_smem[];
+  __shared__ double s_coef[kO1MaxMono];
+  __shared__ int s_ipow[kO1MaxMono], s_jpow[kO1MaxMono];
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nm = C.n_mono, nv = 2 * nm + 6, nb = C.n_edges - 1, NL = C.n_bands;
+  O1WarpBatch& S = reinterpret_cast<O1WarpBatch*>(o1w_smem)[warp];
+  double* mom = reinterpret_cast<double*>(o1w_smem + kO1BatchWarps * sizeof(O1WarpBatch)) +
+                warp * kO1WarpGroups * nv;
+  for (int k = threadIdx.x; k < nm; k += blockDim.x) {
+    s_coef[k] = C.coef[k];
+    s_ipow[k] = C.ipow[k];
+    s_jpow[k] = C.jpow[k];
+  }
+  __syncthreads();
+  const bool quadratic = o1_quadratic(C, s_ipow, s_jpow);
+  double mut_min, speed_max;
+  o1_band_extremes(C, mut_min, speed_max);
+  const int64_t cap = C.group_capacity;
+  const int64_t per_om = (int64_t)NL * (3 + 4 * nb + 1);
+  const int total = *batch_total;
+  const int warps = gridDim.x * kO1BatchWarps;
+  for (int b = blockIdx.x * kO1BatchWarps + warp; b < total; b += warps) {
+    const int w = batch_list[3 * b], start = batch_list[3 * b + 1],
+              count = batch_list[3 * b + 2] - start;
+    if (count > kO1WarpGroups) {
+      if (lane == 0) deferred[atomicAdd(n_deferred, 1)] = b;
+      continue;
+    }
+    const double* rows = grows + (int64_t)w * cap * kO1MaxValues;
+    const int slot = lane < count ? sorted_slots[(int64_t)w * cap + start + lane] : 0;
+    for (int q0 = 0; q0 < count; q0 += 8) {  // eight rows on their way at a time
+      double value[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int from = __shfl_sync(full, slot, min(q0 + j, count - 1));
+        value[j] = lane < nv ? rows[(int64_t)from * kO1MaxValues + lane] : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (q0 + j < count && lane < nv) mom[(q0 + j) * nv + lane] = value[j];
+    }
+    const bool backward =
+        ((gkeys[(int64_t)w * cap + __shfl_sync(full, slot, 0)] / C.theta_bins) & 1) == 1;
+    __syncwarp();
+    // the groups' sums and mean angles, one lane per group
+    const double* row = mom + lane * nv + 2 * nm;
+    const double omega = lane < count ? row[0] : 0.0;
+    const bool some = omega > 0.0;
+    const double angle = some ? row[1] / omega : kPi;
+    double small = angle;
+    for (int off = 16; off; off >>= 1) small = fmin(small, __shfl_xor_sync(full, small, off));
+    const double omega_sum = o1_warp_sum(some ? omega : 0.0);
+    const double r_sum = o1_warp_sum(some ? row[2] : 0.0);
+    const double t_sum = o1_warp_sum(some ? row[3] : 0.0);
+    const double tau_sum = o1_warp_sum(some ? row[4] : 0.0);
+    const double tau2_sum = o1_warp_sum(some ? row[5] : 0.0);
+    double sin_t = 0.0, cos_t = 0.0;
+    if (some) sincos(fmax(angle, 1e-9), &sin_t, &cos_t);
+    S.sin_q[lane] = sin_t;
+    S.cos_q[lane] = cos_t;
+    const O1BatchGrid G = o1_batch_grid(C, backward, omega_sum, r_sum, t_sum, tau_sum, tau2_sum,
+                                        small, mut_min, speed_max, status);
+    const int n = G.n;
+    if (n > kO1WarpNodes) {
+      if (lane == 0) deferred[atomicAdd(n_deferred, 1)] = b;
+      __syncwarp();
+      continue;
+    }
+    if (n == 0) {
+      __syncwarp();
+      continue;
+    }
+    for (int k = lane; k < n; k += 32) S.s[k] = o1_batch_node(G, k);
+    __syncwarp();
+    // the profile: the groups in `parts` ranges, as many as keep the warp's rounds
+    // over (node, part) shortest (33 nodes with one part idle 31 lanes in two)
+    int parts = 1, best = ((n + 31) >> 5) * count;
+    for (int p = 2; p <= 4 && p <= count && n * p <= kO1WarpSums; ++p) {
+      const int cost = ((n * p + 31) >> 5) * ((count + p - 1) / p);
+      if (cost < best) {
+        best = cost;
+        parts = p;
+      }
+    }
+    for (int it = lane; it < n * parts; it += 32) {
+      const int part = it / n, k = it - part * n;
+      o1_batch_profile(C, G, S.s[k], mom, nv, S.sin_q, S.cos_q, s_coef, s_ipow, s_jpow, quadratic,
+                       part * count / parts, (part + 1) * count / parts, S.g0[it], S.g2[it]);
+    }
+    __syncwarp();
+    if (parts > 1) {
+      for (int k = lane; k < n; k += 32)
+        for (int p = 1; p < parts; ++p) {
+          S.g0[k] += S.g0[p * n + k];
+          S.g2[k] += S.g2[p * n + k];
+        }
+      __syncwarp();
+    }
+    if (lane < NL) o1_band_setup(C, G, lane, S.s, S.g0, S.g2, S.band[lane]);
+    __syncwarp();
+    double* accw = accum + (int64_t)w * per_om;
+    int n_panels = 0;
+    for (int lam = 0; lam < NL; ++lam) n_panels += S.band[lam].panels;
+    double band_total = 0.0;  // lane lam: the charge of band lam's panels
+    for (int first = 0; first < n_panels; first += 32) {
+      int lam = 0, pi = first + lane;
+      while (lam < NL && pi >= S.band[lam].panels) pi -= S.band[lam].panels, ++lam;
+      double value = 0.0;
+      if (lam < NL)
+        value = o1_panel(C, S.band[lam], lam, pi, S.s, S.g0, S.g2,
+                         C.compute_bins && !S.band[lam].outside
+                             ? accw + (int64_t)lam * (3 + 4 * nb + 1) : nullptr);
+      for (int l = 0; l < NL; ++l) {
+        const double sum = o1_warp_sum(lam == l ? value : 0.0);
+        if (lane == l) band_total += sum;
+      }
+    }
+    if (lane < NL && S.band[lane].panels > 0) {
+      double* pre = accw + (int64_t)lane * (3 + 4 * nb + 1);
+      o1_front(C, S.band[lane], lane, S.s, band_total,
+               C.compute_bins && !S.band[lane].outside ? pre : nullptr, pre + 3 + 4 * nb);
+    }
+    __syncwarp();
+  }
+}
+
+// The deferred batches: one CTA per batch, up to kO1MaxNodes nodes and 128 groups.
 struct O1BatchShared {
-  double s[NODES];
-  double g0[NODES];
-  double g2[NODES];
+  double s[kO1MaxNodes];
+  double g0[kO1MaxNodes];
+  double g2[kO1MaxNodes];
   double mom[kO1MaxValues * 128];  // moments of the batch's theta groups (<= 128)
   double sin_q[128], cos_q[128];   // per group: sin, cos of its mean angle (0, 0: empty)
   double coef[kO1MaxMono];
+  double total[kO1MaxBands];
   int ipow[kO1MaxMono], jpow[kO1MaxMono];
-  double red[kO1BatchThreads / 32];
-  double stats[8];
   O1BandDeposit band[kO1MaxBands];
-  int n, last;
+  O1BatchGrid grid;
 };
 
-// Persistent CTAs over the batch list: _grouped_pencils_order1_block's batch
-// loop (_prompt_numba.py:1934-1993) with _batch_grid, _batch_add_moments and
-// _batch_deposit (_prompt_numba.py:258-551).
-// The small-grid instance (NODES < kO1MaxNodes, 42 KB of shared memory, five
-// CTAs per SM) takes the whole list and hands each batch whose path grid needs
-// more than NODES nodes to `deferred`; the full-size instance (two CTAs per
-// SM) then takes only those.
-template <int NODES>
 __global__ void __launch_bounds__(kO1BatchThreads)
-o1_batch_kernel(const lh_order1_config C, const int32_t* work, const long long* gkeys,
-                const double* grows, const int32_t* sorted_slots, const int32_t* batch_list,
-                const int32_t* batch_total, int32_t* deferred, int32_t* n_deferred,
-                double* accum, int32_t* status) {
-  constexpr bool kSmall = NODES < kO1MaxNodes;
+o1_batch_kernel(const lh_order1_config C, const long long* gkeys, const double* grows,
+                const int32_t* sorted_slots, const int32_t* batch_list, const int32_t* deferred,
+                const int32_t* n_deferred, double* accum, int32_t* status) {
   extern __shared__ __align__(16) unsigned char o1_smem[];
-  O1BatchShared<NODES>& S = *reinterpret_cast<O1BatchShared<NODES>*>(o1_smem);
+  O1BatchShared& S = *reinterpret_cast<O1BatchShared*>(o1_smem);
   const int tid = threadIdx.x;
-  const int nm = C.n_mono;
-  const int nv = 2 * nm + 6;
-  const int nb = C.n_edges - 1;
-  const int NL = C.n_bands;
+  const int nm = C.n_mono, nv = 2 * nm + 6, nb = C.n_edges - 1, NL = C.n_bands;
   const int64_t cap = C.group_capacity;
+  const int total = *n_deferred;
+  if ((int)blockIdx.x >= total) return;
   for (int k = tid; k < nm; k += blockDim.x) {
     S.coef[k] = C.coef[k];
     S.ipow[k] = C.ipow[k];
     S.jpow[k] = C.jpow[k];
   }
-  double mut_min = C.mut[0], speed_max = C.speed[0];
-  for (int l = 1; l < NL; ++l) {
-    mut_min = fmin(mut_min, C.mut[l]);
-    speed_max = fmax(speed_max, C.speed[l]);
-  }
-  const double g = C.g;
-  const double y_g = g != 0.0 ? (1.0 - fabs(g)) / (1.0 + fabs(g)) : 1.0;
-  const int total = kSmall ? *batch_total : *n_deferred;
+  __syncthreads();
+  const bool quadratic = o1_quadratic(C, S.ipow, S.jpow);
+  double mut_min, speed_max;
+  o1_band_extremes(C, mut_min, speed_max);
   const int64_t per_om = (int64_t)NL * (3 + 4 * nb + 1);
   for (int i = blockIdx.x; i < total; i += gridDim.x) {
-    const int b = kSmall ? i : deferred[i];
+    const int b = deferred[i];
     __syncthreads();
     const int w = batch_list[3 * b], start = batch_list[3 * b + 1], stop = batch_list[3 * b + 2];
     const int count = stop - start;
@@ -1244,15 +1620,15 @@ o1_batch_kernel(const lh_order1_config C, const int32_t* work, const long long* 
     }
     for (int k = tid; k < count * nv; k += blockDim.x) {
       const int q = k / nv, c = k - q * nv;
-      S.mom[q * kO1MaxValues + c] = rows[(int64_t)slots[q] * kO1MaxValues + c];
+      S.mom[k] = rows[(int64_t)slots[q] * kO1MaxValues + c];
     }
-    const long long key0 = gkeys[(int64_t)w * cap + slots[0]];
-    const bool backward = ((key0 / C.theta_bins) & 1) == 1;
+    const bool backward = ((gkeys[(int64_t)w * cap + slots[0]] / C.theta_bins) & 1) == 1;
+    if (tid < NL) S.total[tid] = 0.0;
     __syncthreads();
     if (tid == 0) {
       double omega_sum = 0, r_sum = 0, t_sum = 0, tau_sum = 0, tau2_sum = 0, theta_small = kPi;
       for (int q = 0; q < count; ++q) {
-        const double* row = S.mom + q * kO1MaxValues;
+        const double* row = S.mom + q * nv;
         const double omega = row[2 * nm];
         if (omega > 0.0) {
           omega_sum += omega;
@@ -1263,272 +1639,58 @@ o1_batch_kernel(const lh_order1_config C, const int32_t* work, const long long* 
           theta_small = fmin(theta_small, row[2 * nm + 1] / omega);
         }
       }
-      S.n = 0;
-      if (omega_sum > 0.0) {
-        const double r_b = r_sum / omega_sum;
-        const double t_b = t_sum / omega_sum;
-        const double tau_mean = tau_sum / omega_sum;
-        const double tau_var = fmax(tau2_sum / omega_sum - tau_mean * tau_mean, 0.0);
-        theta_small = fmax(theta_small, 1e-9);
-        double sigma;
-        if (backward) {
-          sigma = fmax(0.5 * r_b * sin(theta_small) * y_g, 0.25 * r_b * (1.0 - cos(theta_small)));
-        } else {
-          // _batch_sigma (_prompt_numba.py:290-292)
-          sigma = fmax(0.5 * r_b * sin(theta_small) * fmax(y_g, 0.5 * tan(0.5 * theta_small)),
-                       1e-9 * r_b);
-        }
-        // _batch_grid (_prompt_numba.py:258-286): node counts
-        const double ext_end = C.tail_exponent / mut_min;
-        // the screen's grids run to the tail without a window edge
-        // (_prompt_screen.py:413: edge_end = inf)
-        double ext_win = C.screen ? ext_end : speed_max * (C.edges[nb] - t_b) - r_b;
-        ext_win = fmin(fmax(ext_win, 0.0), ext_end);
-        const double u_end = asinh(ext_end / sigma), u_win = asinh(ext_win / sigma);
-        if (!(u_win >= 0.0) || !(u_end >= u_win) || !(u_end < 1e6)) {
-          atomicOr(reinterpret_cast<unsigned*>(status), LH_STATUS_OVERFLOW);
-          S.n = 0;
-          goto stats_done;
-        }
-        long long n_in = u_win > 0.0 ? (long long)ceil(u_win / C.path_step) : 0;
-        long long n_out = u_end > u_win ? (long long)ceil((u_end - u_win) / C.path_step_tail) : 0;
-        const int capacity = C.max_path_nodes;
-        if (n_in + n_out + 1 > capacity) {
-          const double scale = (capacity - 1.0) / (double)(n_in + n_out);
-          n_in = (long long)(n_in * scale);
-          n_out = capacity - 1 - n_in;
-        }
-        S.n = (int)(n_in + n_out + 1);
-        if (S.n > NODES) {  // a long path grid: the full-size instance takes this batch
-          deferred[atomicAdd(n_deferred, 1)] = b;
-          S.n = 0;
-          goto stats_done;
-        }
-        S.stats[0] = r_b; S.stats[1] = t_b; S.stats[2] = sqrt(12.0 * tau_var);
-        S.stats[3] = sigma; S.stats[4] = u_win; S.stats[5] = u_end;
-        S.stats[6] = (double)n_in; S.stats[7] = (double)n_out;
-      }
+      S.grid = o1_batch_grid(C, backward, omega_sum, r_sum, t_sum, tau_sum, tau2_sum, theta_small,
+                             mut_min, speed_max, status);
     }
-  stats_done:
-    __syncthreads();
-    const int n = S.n;
-    if (n == 0) continue;
-    const double r_b = S.stats[0], t_b = S.stats[1], front_extra = S.stats[2];
-    const double sigma = S.stats[3], u_win = S.stats[4], u_end = S.stats[5];
-    const int n_in = (int)S.stats[6], n_out = (int)S.stats[7];
-    // the groups' mean angles, once per batch (the profile loop below reads them
-    // for every path node)
     for (int q = tid; q < count; q += blockDim.x) {
-      const double* row = S.mom + q * kO1MaxValues;
+      const double* row = S.mom + q * nv;
       const double omega = row[2 * nm];
       double sin_t = 0.0, cos_t = 0.0;
       if (omega > 0.0) sincos(fmax(row[2 * nm + 1] / omega, 1e-9), &sin_t, &cos_t);
       S.sin_q[q] = sin_t;
       S.cos_q[q] = cos_t;
     }
+    __syncthreads();
+    const int n = S.grid.n;
+    if (n == 0) continue;
     for (int k = tid; k < n; k += blockDim.x) {
-      double s;
-      if (k == 0) s = r_b;
-      else if (k <= n_in) s = r_b + sigma * sinh(u_win * k / n_in);
-      else s = r_b + sigma * sinh(u_win + (u_end - u_win) * (k - n_in) / n_out);
+      const double s = o1_batch_node(S.grid, k);
       S.s[k] = s;
+      o1_batch_profile(C, S.grid, s, S.mom, nv, S.sin_q, S.cos_q, S.coef, S.ipow, S.jpow,
+                       quadratic, 0, count, S.g0[k], S.g2[k]);
     }
     __syncthreads();
-    // profile: _batch_add_moments (_prompt_numba.py:394-447), generic monomials
-    // With few path nodes (typically ~33) the groups are split into `parts`
-    // contiguous ranges so that every thread works: each (node, part) sum goes
-    // to the unused upper part of g0/g2 and the parts are added in order.
-    const double g1 = 1.0 + g * g, gg = 2.0 * g, norm = (1.0 - g * g) / (4.0 * kPi);
-    constexpr int kSplitNodes = NODES / 4;
-    const int parts = n <= kSplitNodes ? max(1, min(3, (int)blockDim.x / n)) : 1;
-    for (int it = tid; it < n * parts; it += blockDim.x) {
-      const int k = it % n, part = it / n;
-      const int q0 = part * count / parts, q1 = (part + 1) * count / parts;
-      double a0s = 0.0, a2s = 0.0;
-      for (int q = q0; q < q1; ++q) {
-        const double* row = S.mom + q * kO1MaxValues;
-        const double omega = row[2 * nm];
-        if (omega <= 0.0) continue;
-        const double sin_t = S.sin_q[q], cos_t = S.cos_q[q];
-        const double rs = r_b * sin_t;
-        double c, s, path_jacobian;
-        if (backward) {
-          const double shift = S.s[k] - r_b * cos_t;
-          const double den = rs * rs + shift * shift;
-          c = (rs * rs - shift * shift) / den;
-          s = 2.0 * rs * shift / den;
-          path_jacobian = 2.0 * r_b / den;
-        } else {
-          const double y = (S.s[k] - r_b) / rs + sin_t / (1.0 + cos_t);
-          const double inv = 1.0 / (1.0 + y * y);
-          c = (1.0 - y * y) * inv;
-          s = 2.0 * y * inv;
-          path_jacobian = 2.0 / (r_b * sin_t) * inv;
-        }
-        double cpw[5], spw[5];
-        cpw[0] = 1.0;
-        spw[0] = 1.0;
-        for (int pw = 1; pw <= C.max_power; ++pw) {
-          cpw[pw] = cpw[pw - 1] * c;
-          spw[pw] = spw[pw - 1] * s;
-        }
-        double a0 = 0.0, a2 = 0.0;
-        for (int m = 0; m < nm; ++m) {
-          const double basis = S.coef[m] * cpw[S.ipow[m]] * spw[S.jpow[m]];
-          a0 += basis * row[m];
-          a2 += basis * row[nm + m];
-        }
-        const double den = g1 - gg * c;
-        const double value = path_jacobian * norm / (den * sqrt(den));
-        a0s += a0 * value;
-        a2s += a2 * value;
-      }
-      if (parts == 1) {
-        S.g0[k] = a0s;
-        S.g2[k] = a2s;
-      } else {
-        S.g0[kSplitNodes * (part + 1) + k] = a0s;
-        S.g2[kSplitNodes * (part + 1) + k] = a2s;
-      }
-    }
-    if (parts > 1) {
-      __syncthreads();
-      for (int k = tid; k < n; k += blockDim.x) {
-        double a0s = 0.0, a2s = 0.0;
-        for (int part = 0; part < parts; ++part) {
-          a0s += S.g0[kSplitNodes * (part + 1) + k];
-          a2s += S.g2[kSplitNodes * (part + 1) + k];
-        }
-        S.g0[k] = a0s;
-        S.g2[k] = a2s;
-      }
-    }
+    if (tid < NL) o1_band_setup(C, S.grid, tid, S.s, S.g0, S.g2, S.band[tid]);
     __syncthreads();
-    // _batch_deposit (_prompt_numba.py:451-551) for every band at once: the
-    // band constants in shared memory, node times and profile values evaluated
-    // from the path grid on the fly, (band, panel) items over the whole CTA,
-    // then each band's front ramp by its own thread
-    const int d = work[w];
     double* accw = accum + (int64_t)w * per_om;
-    const bool bins = C.compute_bins != 0;
-    if (tid < NL) {
-      const int lam = tid;
-      O1BandDeposit& B = S.band[lam];
-      B.panels = 0;
-      B.total = 0.0;
-      if (C.mus[lam] != 0.0) {
-        const double v = C.speed[lam];
-        int last = n - 1;
-        const double limit = r_b + C.tail_exponent / C.mut[lam];
-        while (last > 2 && S.s[last - 1] > limit) last -= 1;
-        if (last >= 2) {
-          B.v = v;
-          B.kappa = -C.mut[lam] * v;
-          B.last = last;
-          B.spread = fmin(front_extra, (S.s[last] - r_b) / v);
-          const double front_time = t_b + r_b / v;
-          const double end_time = t_b + S.s[last] / v;
-          B.outside = front_time - 0.5 * B.spread >= C.edges[nb] ||
-                      end_time + 0.5 * B.spread <= C.edges[0];
-          B.t_base = B.outside ? 0.0 : t_b;
-          B.e_emit = exp(B.kappa * B.t_base);
-          const double h_scale = C.mus[lam] * v / B.e_emit;
-          B.w0 = C.s0w[lam] * h_scale;
-          B.w2 = C.s2w[lam] * h_scale;
-          B.h_front = B.w0 * S.g0[0] + B.w2 * S.g2[0];
-          // panels start at even nodes with step 2; an odd `last` ends with one step
-          B.pairs = last / 2;
-          B.panels = B.pairs + (last & 1);
-        }
-      }
-    }
-    __syncthreads();
-    int n_items = 0;
-    for (int lam = 0; lam < NL; ++lam) n_items += S.band[lam].panels;
-    for (int item = tid; item < n_items; item += blockDim.x) {
+    int n_panels = 0;
+    for (int lam = 0; lam < NL; ++lam) n_panels += S.band[lam].panels;
+    for (int item = tid; item < n_panels; item += blockDim.x) {
       int lam = 0, pi = item;
       while (pi >= S.band[lam].panels) pi -= S.band[lam].panels, ++lam;
-      const O1BandDeposit& B = S.band[lam];
-      const double v = B.v, mut = C.mut[lam];
-      auto node_t = [&](int j) { return B.t_base + S.s[j] / v; };
-      auto node_h = [&](int j) { return (B.w0 * S.g0[j] + B.w2 * S.g2[j]) - B.h_front; };
-      double t_a, t_b2, alpha, beta, gamma, e_a, e_b;
-      if (pi < B.pairs) {
-        const int j = 2 * pi;
-        t_a = node_t(j);
-        const double t_m = node_t(j + 1);
-        t_b2 = node_t(j + 2);
-        const double h0 = node_h(j), h1 = node_h(j + 1), h2 = node_h(j + 2);
-        const double u_m = t_m - t_a, u_b = t_b2 - t_a;
-        const double d1 = (h1 - h0) / u_m;
-        const double d2 = ((h2 - h1) / (t_b2 - t_m) - d1) / u_b;
-        alpha = h0;
-        beta = d1 - d2 * u_m;
-        gamma = d2;
-        e_a = B.e_emit * exp(-mut * S.s[j]);
-        e_b = B.e_emit * exp(-mut * S.s[j + 2]);
-      } else {
-        const int j = B.last - 1;
-        const double t_p = node_t(j - 1);
-        t_a = node_t(j);
-        t_b2 = node_t(j + 1);
-        const double hp = node_h(j - 1), h0 = node_h(j), h1 = node_h(j + 1);
-        const double u_m = t_a - t_p, u_b = t_b2 - t_p;
-        const double d1 = (h0 - hp) / u_m;
-        const double d2 = ((h1 - h0) / (t_b2 - t_a) - d1) / u_b;
-        alpha = h0;
-        beta = d1 - d2 * u_m + 2.0 * d2 * u_m;
-        gamma = d2;
-        e_a = B.e_emit * exp(-mut * S.s[j]);
-        e_b = B.e_emit * exp(-mut * S.s[j + 1]);
-      }
-      atomicAdd(&S.band[lam].total, o1_quad(e_a, alpha, beta, gamma, t_b2 - t_a, B.kappa, e_b));
-      if (bins && !B.outside) {
-        double* pre = accw + (int64_t)lam * (3 + 4 * nb + 1);
-        o1_deposit_panel(t_a, t_b2, e_a, e_b, alpha, beta, gamma, B.kappa, C.edges,
-                         C.eedge + (int64_t)lam * C.n_edges, nb, pre, pre + 3, C.direct_bins);
-      }
+      const double value = o1_panel(C, S.band[lam], lam, pi, S.s, S.g0, S.g2,
+                                    C.compute_bins && !S.band[lam].outside
+                                        ? accw + (int64_t)lam * (3 + 4 * nb + 1) : nullptr);
+      atomicAdd(&S.total[lam], value);
     }
     __syncthreads();
     if (tid < NL && S.band[tid].panels > 0) {
-      const int lam = tid;
-      const O1BandDeposit& B = S.band[lam];
-      const double* eedge = C.eedge + (int64_t)lam * C.n_edges;
-      double* pre = accw + (int64_t)lam * (3 + 4 * nb + 1);
-      double* acc = pre + 3;
-      double* chg = acc + 4 * nb;
-      double sum = B.total;
-      // front step as a mass-normalised ramp of width `spread`
-      const double e_first = B.e_emit * exp(-C.mut[lam] * S.s[0]);
-      const double e_last = B.e_emit * exp(-C.mut[lam] * S.s[B.last]);
-      const double t_f = B.t_base + S.s[0] / B.v, t_end = B.t_base + S.s[B.last] / B.v;
-      const double h_front = B.h_front, spread = B.spread, kappa = B.kappa;
-      const double exact = o1_quad(e_first, h_front, 0.0, 0.0, t_end - t_f, kappa, e_last);
-      sum += exact;
-      if (bins && spread > 0.0 && !B.outside) {
-        const double t_1 = t_f - 0.5 * spread, t_2 = t_f + 0.5 * spread;
-        const double e_1 = exp(kappa * t_1), e_2 = exp(kappa * t_2);
-        const double ramp = o1_quad(e_1, 0.0, 1.0 / spread, 0.0, spread, kappa, e_2);
-        const double flat = t_end > t_2 ? o1_quad(e_2, 1.0, 0.0, 0.0, t_end - t_2, kappa, e_last) : 0.0;
-        const double height = ramp + flat != 0.0 ? exact / (ramp + flat) : 0.0;
-        o1_deposit_panel(t_1, t_2, e_1, e_2, 0.0, height / spread, 0.0, kappa, C.edges, eedge,
-                         nb, pre, acc, C.direct_bins);
-        if (t_end > t_2)
-          o1_deposit_panel(t_2, t_end, e_2, e_last, height, 0.0, 0.0, kappa, C.edges, eedge, nb,
-                           pre, acc, C.direct_bins);
-      } else if (bins && t_end > t_f && !B.outside) {
-        o1_deposit_panel(t_f, t_end, e_first, e_last, h_front, 0.0, 0.0, kappa, C.edges, eedge,
-                         nb, pre, acc, C.direct_bins);
-      }
-      atomicAdd(chg, sum);
+      double* pre = accw + (int64_t)tid * (3 + 4 * nb + 1);
+      o1_front(C, S.band[tid], tid, S.s, S.total[tid],
+               C.compute_bins && !S.band[tid].outside ? pre : nullptr, pre + 3 + 4 * nb);
     }
-    (void)d;
   }
 }
 
-// _finalize (_prompt_numba.py:610-632): one CTA per work OM.
-__global__ void o1_finalize_kernel(const lh_order1_config C, const int32_t* work, int32_t n_work,
-                                   const double* accum, double* charge, double* bins) {
+// _finalize (_prompt_numba.py:610-632): one CTA per work OM, one warp per band.
+// The running coefficients of the bins are prefix sums over 32 bins at a time
+// (one thread per band walked the 160 bins in 61 us, each bin's loads behind the
+// last's).
+constexpr int kO1FinalWarps = 4;
+
+__global__ void __launch_bounds__(32 * kO1FinalWarps)
+o1_finalize_kernel(const lh_order1_config C, const int32_t* work, int32_t n_work,
+                   const double* accum, double* charge, double* bins) {
   const int w = blockIdx.x;
   const int d = work[w];
   const int nb = C.n_edges - 1;
@@ -1542,26 +1704,41 @@ __global__ void o1_finalize_kernel(const lh_order1_config C, const int32_t* work
     charge[d] = area * total;
   }
   if (!C.compute_bins || !bins) return;
-  // one thread per band runs the prefix; the bands are summed in order
   extern __shared__ __align__(16) unsigned char o1f_smem[];
   double* band_bins = reinterpret_cast<double*>(o1f_smem);
-  for (int lam = threadIdx.x; lam < NL; lam += blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (int lam = threadIdx.x >> 5; lam < NL; lam += kO1FinalWarps) {
     const double* pre = accw + (int64_t)lam * (3 + 4 * nb + 1);
     const double* acc = pre + 3;
     const double* eedge = C.eedge + (int64_t)lam * C.n_edges;
     const double* itab = C.itab + (int64_t)lam * nb * 3;
-    double a = pre[0], b = pre[1], c = pre[2];
-    for (int k = 0; k < nb; ++k) {
-      const double e_k = C.edges[k];
-      const double width = C.edges[k + 1] - e_k;
-      const double a_loc = a + e_k * (b + c * e_k);
-      const double b_loc = b + 2.0 * c * e_k;
-      const double value = eedge[k] * width *
-                           (a_loc * itab[3 * k] + width * (b_loc * itab[3 * k + 1] + width * c * itab[3 * k + 2]));
-      band_bins[(int64_t)lam * nb + k] = area * (value + acc[4 * k + 3]);
-      a += acc[4 * k];
-      b += acc[4 * k + 1];
-      c += acc[4 * k + 2];
+    double carry[3] = {pre[0], pre[1], pre[2]};
+    for (int first = 0; first < nb; first += 32) {
+      const int k = first + lane;
+      double own[3], run[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        own[j] = k < nb ? acc[4 * k + j] : 0.0;
+        run[j] = own[j];
+        for (int off = 1; off < 32; off <<= 1) {
+          const double up = __shfl_up_sync(0xffffffffu, run[j], off);
+          if (lane >= off) run[j] += up;
+        }
+      }
+      if (k < nb) {
+        // exclusive: what the bins before deposited
+        const double a = carry[0] + (run[0] - own[0]), b = carry[1] + (run[1] - own[1]),
+                     c = carry[2] + (run[2] - own[2]);
+        const double e_k = C.edges[k];
+        const double width = C.edges[k + 1] - e_k;
+        const double a_loc = a + e_k * (b + c * e_k);
+        const double b_loc = b + 2.0 * c * e_k;
+        const double value = eedge[k] * width *
+                             (a_loc * itab[3 * k] + width * (b_loc * itab[3 * k + 1] + width * c * itab[3 * k + 2]));
+        band_bins[(int64_t)lam * nb + k] = area * (value + acc[4 * k + 3]);
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j) carry[j] += __shfl_sync(0xffffffffu, run[j], 31);
     }
   }
   __syncthreads();
@@ -1589,7 +1766,7 @@ struct O1Workspace {
   int32_t* sorted;
   int32_t* batch_list;
   int32_t* batch_total;  // [4]: batches, then batches deferred to the full-size grid
-  int32_t* deferred;     // batches whose path grid exceeds kO1SmallNodes
+  int32_t* deferred;     // batches too large for one warp
   double* accum;
   unsigned long long* sort_keys;  // tables above kO1SmemSort only
   int32_t* sort_slots;
@@ -1799,29 +1976,27 @@ extern "C" int lh_order1_grouped(const lh_order1_config* C, const lh_order1_penc
   lh::o1_batches_kernel<<<n_work, 1024, sort_smem, s>>>(*C, n_work, W.gkeys, W.sorted, W.batch_list,
                                                         W.batch_total, W.sort_keys, W.sort_slots,
                                                         status);
-  const size_t small_smem = sizeof(lh::O1BatchShared<lh::kO1SmallNodes>);
-  const size_t full_smem = sizeof(lh::O1BatchShared<lh::kO1MaxNodes>);
-  if (cudaFuncSetAttribute(lh::o1_batch_kernel<lh::kO1SmallNodes>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)small_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(lh::o1_batch_kernel<lh::kO1MaxNodes>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const size_t warp_smem = lh::o1_warp_batch_bytes(*C);
+  const size_t full_smem = sizeof(lh::O1BatchShared);
+  if (cudaFuncSetAttribute(lh::o1_batch_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)warp_smem) != cudaSuccess ||
+      cudaFuncSetAttribute(lh::o1_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)full_smem) != cudaSuccess)
     return LH_ECUDA;
   {
     lh::TimedLaunch timed_launch(LH_KT_O1_BATCH, s);
-    lh::o1_batch_kernel<lh::kO1SmallNodes><<<148 * 5, lh::kO1BatchThreads, small_smem, s>>>(
-        *C, work, W.gkeys, W.grows, W.sorted, W.batch_list, W.batch_total, W.deferred,
+    lh::o1_batch_warp_kernel<<<148 * 5, 32 * lh::kO1BatchWarps, warp_smem, s>>>(
+        *C, W.gkeys, W.grows, W.sorted, W.batch_list, W.batch_total, W.deferred,
         W.batch_total + 1, W.accum, status);
-    lh::o1_batch_kernel<lh::kO1MaxNodes><<<148 * 2, lh::kO1BatchThreads, full_smem, s>>>(
-        *C, work, W.gkeys, W.grows, W.sorted, W.batch_list, W.batch_total, W.deferred,
-        W.batch_total + 1, W.accum, status);
+    lh::o1_batch_kernel<<<148 * 2, lh::kO1BatchThreads, full_smem, s>>>(
+        *C, W.gkeys, W.grows, W.sorted, W.batch_list, W.deferred, W.batch_total + 1, W.accum,
+        status);
   }
   const size_t fin_smem = sizeof(double) * C->n_bands * nb;
   if (fin_smem > 200 * 1024) return LH_EUNSUPPORTED;
   if (cudaFuncSetAttribute(lh::o1_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)fin_smem) != cudaSuccess)
     return LH_ECUDA;
-  lh::o1_finalize_kernel<<<n_work, 128, fin_smem, s>>>(*C, work, n_work, W.accum, charge, bins);
+  lh::o1_finalize_kernel<<<n_work, 32 * lh::kO1FinalWarps, fin_smem, s>>>(*C, work, n_work, W.accum, charge, bins);
   return cudaGetLastError() == cudaSuccess ? LH_OK : LH_ECUDA;
 }

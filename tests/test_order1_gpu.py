@@ -206,3 +206,33 @@ def test_acceptance_degrees_and_group_steps_match_the_oracle(alpha, log_r):
         smoothing_factor=s.smoothing_factor,
         merge=(s.merge_theta_min, s.merge_theta_ratio, s.merge_tau_ns, log_r))
     check(q.cpu().numpy(), b.cpu().numpy(), q_ref, b_ref)
+
+
+@pytest.mark.parametrize("step, tau, log_r", [(0.1, 0.5, 0.02), (0.03, 0.5, 0.02),
+                                              (0.024, 2.0, 0.1), (0.1, 1e3, 2.0)])
+def test_batches_around_one_warps_share_match_the_oracle(step, tau, log_r):
+    """Batches of up to 128 path nodes and 32 groups are one warp's; longer grids
+    (steps of 0.03 and 0.024 give about 110 and 140 nodes) and batches of more
+    angle groups (wide time and radius cells) a CTA's: stage B on the
+    reference's pencils against the oracle's grouped order 1."""
+    from dataclasses import replace
+    from lighthit_b200.order1 import Order1Tables, PencilTable, grouped
+    from oracle import order1 as O1
+    g = fixture()
+    s = replace(tables_of(g).settings, path_step=step, path_step_tail=2.5 * step,
+                merge_tau_ns=tau, merge_log_r=log_r, merge_theta_ratio=0.07)
+    bands = {k: g[k] for k in ("mus", "mut", "speed", "s0w", "s2w")}
+    mono = (g["coef"], g["ipow"], g["jpow"], int(g["degree"]))
+    tables = Order1Tables(bands, float(g["g"]), mono, g["positions_m"], g["looks"],
+                          g["areas_m2"], g["edges_ns"], settings=s)
+    pencils = {k: g[f"sub_pencil_{k}"] for k in PENCIL_KEYS}
+    table, n = PencilTable.from_host(pencils, tables.device)
+    work = np.array([0, 11, 30, 47])
+    q, b = grouped(tables, table, work, g["origins_ns"], n_pencils=n)
+    q_ref, b_ref, _, _ = O1.grouped(
+        pencils, g["positions_m"], g["looks"], g["areas_m2"], g["origins_ns"], work, mono,
+        float(g["g"]), bands, g["edges_ns"], path_step=step, path_step_tail=2.5 * step,
+        tail_exponent=s.tail_exponent, direct_bins=s.direct_bins,
+        max_path_nodes=s.max_path_nodes, smoothing_factor=s.smoothing_factor,
+        merge=(s.merge_theta_min, 0.07, tau, log_r))
+    check(q.cpu().numpy(), b.cpu().numpy(), q_ref, b_ref)
