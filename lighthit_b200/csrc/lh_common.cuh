@@ -109,6 +109,18 @@ LH_DEVICE void bulk_g2s(void* smem_dst, const void* gmem_src, uint32_t bytes, ui
       : "memory");
 }
 
+// Copies of 8 bytes global -> shared by the calling thread, in groups: commit ends a
+// group, wait<N> waits for all but the last N groups of this thread.
+LH_DEVICE void copy_async8(void* smem_dst, const void* gmem_src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(smem_dst)), "l"(gmem_src)
+               : "memory");
+}
+LH_DEVICE void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+LH_DEVICE void copy_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+
 // ---------------------------------------------------------------- tcgen05
 // Shared-memory matrix descriptor, K-major, no swizzle: 8-row x 16-byte core
 // matrices; ``lbo`` = byte distance between core matrices along K, ``sbo`` =

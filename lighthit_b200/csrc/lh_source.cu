@@ -18,11 +18,20 @@
 // and the slice's points carry V (thin slice, one point at the field-0
 // centroid) or the stencil combination of its five moments (wide slice).
 //
-// B200 layout: nodes are counting-sorted by base lattice key (zb, tb); one
-// CTA per occupied base key forms the 8 link x 5 moment x channel products of
-// its nodes in shared memory (float64) and adds them to the dense
-// (slice, tick) deposit once; one CTA per (slice, band) runs the time-lattice
-// transform with a rotating phasor and writes the points' channels.
+// B200 layout: one thread per node forms the node's link weights, band factors,
+// harmonics and Legendre values once and counts it under its base lattice key
+// (zb, tb); the occupied keys are listed as they are first met. Ticks are stored
+// for each slice's own range only, one row of [band][moment][channel] per (slice,
+// tick). One CTA per occupied key adds its nodes' products, eight links in
+// registers per (moment, channel) thread, to the rows; one CTA per (slice, band,
+// block of frequencies) runs the time-lattice transform with rotating phasors and
+// writes the points' channels.
+// Measured on 6637 elements (2700 keys, 39 channels, 65 frequencies), before and
+// after: key scan 45 us (one CTA over every lattice key) -> 3 us; clearing 42 us
+// (203 MB of lattice, mostly never read) -> 8 us; keys 121 us (one thread per node
+// forming its harmonics inside the key's CTA) -> 25 us; layout 51 us (one
+// thread) -> 3 us; transform 143 us (one frequency per thread, no copies ahead) ->
+// 97 us, bound by the float64 chain of two CTAs per SM. The node pass takes 24 us.
 #include <algorithm>
 
 #include "lh_common.cuh"
@@ -32,15 +41,27 @@ namespace lh {
 
 constexpr int kSrcMaxBands = 8;
 constexpr int kSrcMaxNch = 153;       // degree 16, azimuthal degree 4
-constexpr int kSrcChunk = 16;         // nodes staged per pass
-constexpr int kSrcThreads = 256;
+constexpr int kSrcChunk = 32;         // most nodes staged per pass
+constexpr size_t kSrcStageBytes = 40 * 1024;  // of a pass's nodes
 
-struct SrcNode {
-  double zr, tr, x, y;
-  int64_t key;
-  int el;
-  int pad;
+// Float64 values of a node: harmonics [nch], Legendre values [band][degree + 1],
+// link weights [8], axial weights [4], factors [band][5].
+struct SrcRow {
+  int legendre, link, axial, factor, size;
 };
+__host__ __device__ inline SrcRow src_row(const lh_source_problem& P) {
+  SrcRow r;
+  r.legendre = P.nch;
+  r.link = r.legendre + P.n_bands * (P.degree + 1);
+  r.axial = r.link + 8;
+  r.factor = r.axial + 4;
+  r.size = r.factor + P.n_bands * 5;
+  return r;
+}
+__host__ __device__ inline int src_chunk(const lh_source_problem& P) {
+  const int fit = (int)(kSrcStageBytes / sizeof(double)) / src_row(P).size;
+  return fit < kSrcChunk ? fit : kSrcChunk;
+}
 
 // Cubic Lagrange weights of shifts -1, 0, 1, 2 at offset r (_shower_basis.py:112-118)
 LH_DEVICE void src_axial_weights(double r, double* w) {
@@ -93,13 +114,29 @@ LH_DEVICE void src_harmonics(double x, double y, double z, const lh_source_probl
   }
 }
 
-// One thread per (element, node): lattice coordinates, counts per base key,
-// slice occupancy and each slice's tick range.
-__global__ void src_nodes_kernel(const lh_source_problem P, SrcNode* nodes, int32_t* counts,
-                                 int32_t* slice_lo, int32_t* slice_hi, int32_t* status) {
+struct SrcWorkspace {
+  int64_t* key;        // [node], -1 outside the lattice
+  double* rows;        // [node][SrcRow]
+  int32_t *counts, *offsets, *cursor;  // [lattice key]
+  int32_t* order;      // nodes by key
+  int64_t* groups;     // occupied keys, in no order
+  int32_t* n_groups;   // [4]: occupied keys, nodes listed, occupied slices
+  int32_t *slice_lo, *slice_hi;        // tick range, hi < 0: empty
+  int64_t* slice_row;  // [n_slices + 1] first deposit row of each slice
+  int32_t *slice_point, *slice_wide;
+  double *deposit, *zero;
+  size_t bytes;
+};
+
+// One thread per (element, node): lattice coordinates, the node's row of values,
+// counts and first meeting of its base key, each slice's tick range.
+__global__ void __launch_bounds__(64)
+src_nodes_kernel(const lh_source_problem P, const SrcWorkspace W, int32_t* status) {
   const int64_t total = (int64_t)P.n_el * P.element_order;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const unsigned full = 0xffffffffu;
+  long long key = -1;
+  if (k < total) {
     const int e = (int)(k / P.element_order);
     const int n = (int)(k - (int64_t)e * P.element_order);
     const double f = P.node_fraction[n];
@@ -116,364 +153,366 @@ __global__ void src_nodes_kernel(const lh_source_problem P, SrcNode* nodes, int3
     const double zbf = floor(zl);
     const double tl = (t - P.reference_ns) / P.time_step_ns;
     const double tbf = floor(tl);
-    SrcNode N;
-    N.zr = zl - zbf;
-    N.tr = tl - tbf;
-    N.x = x;
-    N.y = y;
-    N.el = e;
-    N.pad = n;  // Gauss node of the chord
     const long long zb = (long long)zbf, tb = (long long)tbf;
     if (zb < 1 || zb + 2 >= P.n_slices || tb < 0 || tb + 1 >= P.kmax) {
       atomicOr(reinterpret_cast<unsigned*>(status), LH_STATUS_OVERFLOW);
-      N.key = -1;
-      nodes[k] = N;
-      continue;
-    }
-    N.key = zb * P.kmax + tb;
-    nodes[k] = N;
-    atomicAdd(counts + N.key, 1);
-    for (int j = -1; j <= 2; ++j) {
-      atomicMin(slice_lo + zb + j, (int)tb);
-      atomicMax(slice_hi + zb + j, (int)tb + 1);
-    }
-  }
-}
-
-// Single CTA: exclusive scan of the base-key counts and the list of occupied keys.
-__global__ void __launch_bounds__(1024)
-src_scan_kernel(int64_t n_keys, const int32_t* counts, int32_t* offsets, int32_t* cursor,
-                int64_t* groups, int32_t* n_groups) {
-  __shared__ int32_t warp_sum[32];
-  __shared__ int32_t carry, carry_groups;
-  if (threadIdx.x == 0) {
-    carry = 0;
-    carry_groups = 0;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int64_t base = 0; base < n_keys; base += blockDim.x) {
-    const int64_t i = base + threadIdx.x;
-    const int32_t c = i < n_keys ? counts[i] : 0;
-    // inclusive scans of the counts and of the occupied flags
-    int32_t v = c, g = c > 0 ? 1 : 0;
-    for (int off = 1; off < 32; off <<= 1) {
-      const int32_t a = __shfl_up_sync(0xffffffffu, v, off);
-      const int32_t b = __shfl_up_sync(0xffffffffu, g, off);
-      if (lane >= off) {
-        v += a;
-        g += b;
+    } else {
+      key = zb * P.kmax + tb;
+      for (int j = -1; j <= 2; ++j) {
+        atomicMin(W.slice_lo + zb + j, (int)tb);
+        atomicMax(W.slice_hi + zb + j, (int)tb + 1);
       }
-    }
-    __shared__ int32_t warp_g[32];
-    if (lane == 31) {
-      warp_sum[warp] = v;
-      warp_g[warp] = g;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      int32_t s = lane < (int)(blockDim.x >> 5) ? warp_sum[lane] : 0;
-      int32_t h = lane < (int)(blockDim.x >> 5) ? warp_g[lane] : 0;
-      for (int off = 1; off < 32; off <<= 1) {
-        const int32_t a = __shfl_up_sync(0xffffffffu, s, off);
-        const int32_t b = __shfl_up_sync(0xffffffffu, h, off);
-        if (lane >= off) {
-          s += a;
-          h += b;
-        }
+      const SrcRow R = src_row(P);
+      double* row = W.rows + k * R.size;
+      const double ux = P.direction[3 * e], uy = P.direction[3 * e + 1], uz = P.direction[3 * e + 2];
+      // the direction in (first, second, axis)
+      src_harmonics(ux * P.first[0] + uy * P.first[1] + uz * P.first[2],
+                    ux * P.second[0] + uy * P.second[1] + uz * P.second[2],
+                    ux * P.axis[0] + uy * P.axis[1] + uz * P.axis[2], P, row);
+      double wz[4];
+      const double zr = zl - zbf, tr = tl - tbf;
+      src_axial_weights(zr, wz);
+      const double wt[2] = {1 - tr, tr};
+      for (int j = 0; j < 4; ++j) {
+        row[R.axial + j] = wz[j];
+        for (int d = 0; d < 2; ++d) row[R.link + 2 * j + d] = wz[j] * wt[d];
       }
-      warp_sum[lane] = s;
-      warp_g[lane] = h;
-    }
-    __syncthreads();
-    const int32_t before = (warp ? warp_sum[warp - 1] : 0) + v - c + carry;
-    const int32_t before_g = (warp ? warp_g[warp - 1] : 0) + g - (c > 0 ? 1 : 0) + carry_groups;
-    if (i < n_keys) {
-      offsets[i] = before;
-      cursor[i] = before;
-      if (c > 0) groups[before_g] = i;
-    }
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) {
-      carry = before + c;
-      carry_groups = before_g + (c > 0 ? 1 : 0);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *n_groups = carry_groups;
-}
-
-__global__ void src_scatter_kernel(const lh_source_problem P, const SrcNode* nodes, int32_t* cursor,
-                                   int32_t* order) {
-  const int64_t total = (int64_t)P.n_el * P.element_order;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t key = nodes[k].key;
-    if (key < 0) continue;
-    order[atomicAdd(cursor + key, 1)] = (int32_t)k;
-  }
-}
-
-struct SrcGroupShared {
-  double harm[kSrcChunk][kSrcMaxNch];
-  double pl[kSrcChunk][kSrcMaxBands][17];
-  double link[kSrcChunk][8];
-  double axial[kSrcChunk][4];
-  double factor[kSrcChunk][kSrcMaxBands][5];
-};
-
-// One CTA per occupied base key: sum its nodes' products over
-// (band, link, moment, channel) and add them to the deposit.
-__global__ void __launch_bounds__(kSrcThreads)
-src_group_kernel(const lh_source_problem P, const SrcNode* nodes, const int32_t* offsets,
-                 const int32_t* counts, const int32_t* order, const int64_t* groups,
-                 const int32_t* n_groups, double* deposit, double* zero) {
-  extern __shared__ __align__(16) unsigned char src_smem[];
-  SrcGroupShared& S = *reinterpret_cast<SrcGroupShared*>(src_smem);
-  double* acc = reinterpret_cast<double*>(src_smem + sizeof(SrcGroupShared));
-  const int NB = P.n_bands, nch = P.nch;
-  const int entries = NB * 8 * 5 * nch;        // (band, link, moment, channel)
-  const int zentries = NB * 4 * 5;             // (band, axial shift, moment)
-  const int total_groups = *n_groups;
-  for (int gi = blockIdx.x; gi < total_groups; gi += gridDim.x) {
-    const int64_t key = groups[gi];
-    const int begin = offsets[key], count = counts[key];
-    for (int i = threadIdx.x; i < entries + zentries; i += blockDim.x) acc[i] = 0.0;
-    for (int c0 = 0; c0 < count; c0 += kSrcChunk) {
-      const int nn = min(kSrcChunk, count - c0);
-      __syncthreads();
-      if (threadIdx.x < nn) {
-        const int q = threadIdx.x;
-        const SrcNode N = nodes[order[begin + c0 + q]];
-        const int e = N.el;
-        const double ux = P.direction[3 * e], uy = P.direction[3 * e + 1], uz = P.direction[3 * e + 2];
-        // rotate into (first, second, axis)
-        const double rx = ux * P.first[0] + uy * P.first[1] + uz * P.first[2];
-        const double ry = ux * P.second[0] + uy * P.second[1] + uz * P.second[2];
-        const double rz = ux * P.axis[0] + uy * P.axis[1] + uz * P.axis[2];
-        src_harmonics(rx, ry, rz, P, S.harm[q]);
-        double wz[4];
-        src_axial_weights(N.zr, wz);
-        const double wt[2] = {1 - N.tr, N.tr};
-        for (int j = 0; j < 4; ++j) {
-          S.axial[q][j] = wz[j];
-          for (int d = 0; d < 2; ++d) S.link[q][2 * j + d] = wz[j] * wt[d];
-        }
-        for (int b = 0; b < NB; ++b) {
-          // signed band field C0/lambda^2 + C2/(lambda n)^2 times the chord node weight
-          const double f = (P.c0[e] * P.band_s0[b] + P.c2[e] * P.band_s2[b]) * P.node_weight[N.pad];
-          S.factor[q][b][0] = f;
-          S.factor[q][b][1] = f * N.x;
-          S.factor[q][b][2] = f * N.y;
-          S.factor[q][b][3] = f * N.x * N.x;
-          S.factor[q][b][4] = f * N.y * N.y;
-          const double mu = 1.0 / (P.beta[e] * P.band_phase[b]);
-          double prev = 1.0, cur = mu;
-          for (int ell = 0; ell <= P.degree; ++ell) {
-            double p;
-            if (ell == 0) p = 1.0;
-            else if (ell == 1) p = cur;
-            else {
-              p = ((2 * ell - 1) * mu * cur - (ell - 1) * prev) / ell;
-              prev = cur;
-              cur = p;
-            }
-            S.pl[q][b][ell] = p;
+      for (int b = 0; b < P.n_bands; ++b) {
+        // signed band field C0/lambda^2 + C2/(lambda n)^2 times the chord node weight
+        const double g = (P.c0[e] * P.band_s0[b] + P.c2[e] * P.band_s2[b]) * P.node_weight[n];
+        double* factor = row + R.factor + 5 * b;
+        factor[0] = g;
+        factor[1] = g * x;
+        factor[2] = g * y;
+        factor[3] = g * x * x;
+        factor[4] = g * y * y;
+        const double mu = 1.0 / (P.beta[e] * P.band_phase[b]);
+        double* legendre = row + R.legendre + b * (P.degree + 1);
+        double prev = 1.0, cur = mu;
+        for (int ell = 0; ell <= P.degree; ++ell) {
+          double p;
+          if (ell == 0) p = 1.0;
+          else if (ell == 1) p = cur;
+          else {
+            p = ((2 * ell - 1) * mu * cur - (ell - 1) * prev) / ell;
+            prev = cur;
+            cur = p;
           }
+          legendre[ell] = p;
         }
       }
-      __syncthreads();
-      for (int i = threadIdx.x; i < entries; i += blockDim.x) {
-        const int c = i % nch;
-        int rest = i / nch;
-        const int k = rest % 5;
-        rest /= 5;
-        const int link = rest % 8;
-        const int b = rest / 8;
-        const int ell = P.channel_degree[c];
-        double sum = 0.0;
-        for (int q = 0; q < nn; ++q)
-          sum += S.link[q][link] * S.factor[q][b][k] * (S.harm[q][c] * S.pl[q][b][ell]);
-        acc[i] += sum;
-      }
-      for (int i = threadIdx.x; i < zentries; i += blockDim.x) {
-        const int k = i % 5;
-        const int j = (i / 5) % 4;
-        const int b = i / 20;
-        double sum = 0.0;
-        for (int q = 0; q < nn; ++q) sum += S.axial[q][j] * S.factor[q][b][k];
-        acc[entries + i] += sum;
-      }
     }
-    __syncthreads();
-    const long long zb = key / P.kmax, tb = key - zb * P.kmax;
-    for (int i = threadIdx.x; i < entries; i += blockDim.x) {
-      const double v = acc[i];
-      if (v == 0.0) continue;
-      const int c = i % nch;
-      int rest = i / nch;
-      const int k = rest % 5;
-      rest /= 5;
-      const int link = rest % 8;
-      const int b = rest / 8;
-      const long long row = (zb + (link >> 1) - 1) * P.kmax + tb + (link & 1);
-      atomicAdd(deposit + ((row * NB + b) * 5 + k) * nch + c, v);
-    }
-    for (int i = threadIdx.x; i < zentries; i += blockDim.x) {
-      const int k = i % 5;
-      const int j = (i / 5) % 4;
-      const int b = i / 20;
-      atomicAdd(zero + ((zb + j - 1) * NB + b) * 5 + k, acc[entries + i]);
-    }
-    __syncthreads();
+    W.key[k] = key;
+  }
+  const bool fresh = key >= 0 && atomicAdd(W.counts + key, 1) == 0;
+  const unsigned news = __ballot_sync(full, fresh);
+  if (news) {
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    if (lane == __ffs(news) - 1) at = atomicAdd(W.n_groups, __popc(news));
+    at = __shfl_sync(full, at, __ffs(news) - 1);
+    if (fresh) W.groups[at + __popc(news & ((1u << lane) - 1u))] = key;
   }
 }
 
-// Single thread: point layout of every band (_shower_basis.py:375-420, 466-475):
-// occupied slices in order, then the +x, -x, +y, -y stencil points of the wide
-// slices; thin slices sit at their field-0 centroid, wide ones on the axis.
-__global__ void src_layout_kernel(const lh_source_problem P, const int32_t* slice_lo,
-                                  const int32_t* slice_hi, const double* zero, int32_t* slice_point,
-                                  int32_t* slice_wide, double* centroid, int32_t* n_occ_out,
+// CTA 0: the first deposit row of each slice. The others: each occupied key's
+// place in the node list (in no order).
+__global__ void __launch_bounds__(256)
+src_rows_kernel(const lh_source_problem P, const SrcWorkspace W) {
+  if (blockIdx.x > 0) {
+    const int total = W.n_groups[0];
+    for (int g = (blockIdx.x - 1) * blockDim.x + threadIdx.x; g < total;
+         g += (gridDim.x - 1) * blockDim.x) {
+      const int64_t key = W.groups[g];
+      const int at = atomicAdd(W.n_groups + 1, W.counts[key]);
+      W.offsets[key] = at;
+      W.cursor[key] = at;
+    }
+    return;
+  }
+  __shared__ long long warp_sum[8];
+  __shared__ int occupied;
+  if (threadIdx.x == 0) occupied = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long carry = 0;
+  int mine = 0;
+  for (int64_t first = 0; first < P.n_slices; first += blockDim.x) {
+    const int64_t s = first + threadIdx.x;
+    const int hi = s < P.n_slices ? W.slice_hi[s] : -1;
+    const long long n = hi >= 0 ? hi - W.slice_lo[s] + 1 : 0;
+    mine += hi >= 0;
+    long long v = n;
+    for (int off = 1; off < 32; off <<= 1) {
+      const long long up = __shfl_up_sync(0xffffffffu, v, off);
+      if (lane >= off) v += up;
+    }
+    __syncthreads();
+    if (lane == 31) warp_sum[warp] = v;
+    __syncthreads();
+    long long before = carry;
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) before += warp_sum[w];
+      carry += warp_sum[w];
+    }
+    if (s < P.n_slices) W.slice_row[s] = before + v - n;
+  }
+  atomicAdd(&occupied, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    W.slice_row[P.n_slices] = carry;
+    W.n_groups[2] = occupied;
+  }
+}
+
+// Lists the nodes by key and clears the deposit rows in use.
+__global__ void src_scatter_kernel(const lh_source_problem P, const SrcWorkspace W) {
+  const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t total = (int64_t)P.n_el * P.element_order;
+  for (int64_t k = first; k < total; k += stride) {
+    const int64_t key = W.key[k];
+    if (key >= 0) W.order[atomicAdd(W.cursor + key, 1)] = (int32_t)k;
+  }
+  const int64_t values = W.slice_row[P.n_slices] * P.n_bands * 5 * P.nch;
+  double2* pairs = reinterpret_cast<double2*>(W.deposit);
+  for (int64_t k = first; k < (values + 1) / 2; k += stride) pairs[k] = make_double2(0.0, 0.0);
+}
+
+// One CTA per occupied base key, one thread per (moment, channel): the nodes'
+// products of a band summed over the eight links in registers, then added to the
+// links' rows.
+__global__ void src_group_kernel(const lh_source_problem P, const SrcWorkspace W) {
+  extern __shared__ __align__(16) double s_node[];  // [node of the pass][SrcRow]
+  const SrcRow R = src_row(P);
+  const int NB = P.n_bands, nch = P.nch, chunk = src_chunk(P);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int k = threadIdx.x / nch, c = threadIdx.x - k * nch;
+  const bool mine = k < 5;
+  const int ell = mine ? P.channel_degree[c] : 0;
+  const int total_groups = W.n_groups[0];
+  for (int gi = blockIdx.x; gi < total_groups; gi += gridDim.x) {
+    const int64_t key = W.groups[gi];
+    const int begin = W.offsets[key], count = W.counts[key];
+    const long long zb = key / P.kmax, tb = key - zb * P.kmax;
+    auto stage = [&](int from, int nn) {
+      __syncthreads();
+      for (int q = warp; q < nn; q += warps) {
+        const double* row = W.rows + (int64_t)W.order[begin + from + q] * R.size;
+        for (int i = lane; i < R.size; i += 32) s_node[q * R.size + i] = row[i];
+      }
+      __syncthreads();
+    };
+    const bool once = count <= chunk;
+    for (int b = 0; b < NB; ++b) {
+      double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, sum = 0.0;
+      // the field moments of the slices: thread (axial shift, moment)
+      const bool zeroth = threadIdx.x < 20;
+      const int shift = threadIdx.x / 5, moment = threadIdx.x - 5 * shift;
+      for (int from = 0; from < count; from += chunk) {
+        const int nn = min(chunk, count - from);
+        if (!once || b == 0) stage(from, nn);
+        if (mine)
+          for (int q = 0; q < nn; ++q) {
+            const double* row = s_node + q * R.size;
+            const double v = row[R.factor + 5 * b + k] *
+                             (row[c] * row[R.legendre + b * (P.degree + 1) + ell]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] += row[R.link + j] * v;
+          }
+        if (zeroth)
+          for (int q = 0; q < nn; ++q)
+            sum += s_node[q * R.size + R.axial + shift] *
+                   s_node[q * R.size + R.factor + 5 * b + moment];
+      }
+      if (mine) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (acc[j] == 0.0) continue;
+          const long long slice = zb + (j >> 1) - 1;
+          const int64_t at = W.slice_row[slice] + tb + (j & 1) - W.slice_lo[slice];
+          atomicAdd(W.deposit + ((at * NB + b) * 5 + k) * nch + c, acc[j]);
+        }
+      }
+      if (zeroth) atomicAdd(W.zero + ((zb + shift - 1) * NB + b) * 5 + moment, sum);
+    }
+  }
+}
+
+// One warp per band: point layout (_shower_basis.py:375-420, 466-475): occupied
+// slices in order, then the +x, -x, +y, -y stencil points of the wide slices; thin
+// slices sit at their field-0 centroid, wide ones on the axis.
+__global__ void src_layout_kernel(const lh_source_problem P, const SrcWorkspace W,
                                   lh_source_output O) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int NB = P.n_bands;
+  const int NB = P.n_bands, b = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu, lower = (1u << lane) - 1u;
   const int64_t S = P.n_slices;
-  int n_occ = 0;
-  for (int64_t s = 0; s < S; ++s) n_occ += slice_hi[s] >= 0 ? 1 : 0;
-  *n_occ_out = n_occ;
-  for (int b = 0; b < NB; ++b) {
-    int occ = 0, wide_count = 0;
-    for (int64_t s = 0; s < S; ++s) {
-      slice_point[b * S + s] = -1;
-      slice_wide[b * S + s] = -1;
-      if (slice_hi[s] < 0) continue;
-      const double* zm = zero + (s * NB + b) * 5;
+  const double h = P.stencil_m;
+  int occ = 0, wide_count = 0;
+  for (int64_t first = 0; first < S; first += 32) {
+    const int64_t s = first + lane;
+    const bool used = s < S && W.slice_hi[s] >= 0;
+    bool wide = false;
+    double cx = 0.0, cy = 0.0;
+    if (used) {
+      const double* zm = W.zero + (s * NB + b) * 5;
       const double mass = zm[0];
       const double safe = mass != 0.0 ? mass : 1.0;
       // absolute values by comparison: nvcc 12.9 at -O3 dropped fabs() of this
       // select (fabs(safe) came back negative for a negative mass)
       const double num = zm[3] + zm[4];
       const double spread = sqrt((num < 0.0 ? -num : num) / (safe < 0.0 ? -safe : safe));
-      const bool wide = spread > P.stencil_threshold_m;
-      const double cx = wide ? 0.0 : zm[1] / safe, cy = wide ? 0.0 : zm[2] / safe;
-      centroid[(b * S + s) * 2] = cx;
-      centroid[(b * S + s) * 2 + 1] = cy;
-      slice_point[b * S + s] = occ;
-      const double z = P.z_origin + (double)s * P.cell_m;
-      double* pt = O.points + ((int64_t)b * O.capacity + occ) * 3;
-      pt[0] = z;
-      pt[1] = cx;
-      pt[2] = cy;
-      if (wide) slice_wide[b * S + s] = wide_count++;
-      ++occ;
+      wide = spread > P.stencil_threshold_m;
+      cx = wide ? 0.0 : zm[1] / safe;
+      cy = wide ? 0.0 : zm[2] / safe;
     }
-    // stencil points: offsets (h,0), (-h,0), (0,h), (0,-h) in wide-slice order
-    const double h = P.stencil_m;
-    const double ox[4] = {h, -h, 0.0, 0.0}, oy[4] = {0.0, 0.0, h, -h};
-    for (int64_t s = 0; s < S; ++s) {
-      const int w = slice_wide[b * S + s];
-      if (w < 0) continue;
-      const double z = P.z_origin + (double)s * P.cell_m;
-      for (int o = 0; o < 4; ++o) {
-        double* pt = O.points + ((int64_t)b * O.capacity + occ + o * wide_count + w) * 3;
-        pt[0] = z;
-        pt[1] = ox[o];
-        pt[2] = oy[o];
+    const unsigned used_mask = __ballot_sync(full, used), wide_mask = __ballot_sync(full, wide);
+    if (s < S) {
+      const int point = occ + __popc(used_mask & lower);
+      W.slice_point[b * S + s] = used ? point : -1;
+      W.slice_wide[b * S + s] = wide ? wide_count + __popc(wide_mask & lower) : -1;
+      if (used) {
+        double* pt = O.points + ((int64_t)b * O.capacity + point) * 3;
+        pt[0] = P.z_origin + (double)s * P.cell_m;
+        pt[1] = cx;
+        pt[2] = cy;
       }
     }
-    O.n_points[b] = occ + 4 * wide_count;
+    occ += __popc(used_mask);
+    wide_count += __popc(wide_mask);
+  }
+  __syncwarp();
+  // stencil points: offsets (h,0), (-h,0), (0,h), (0,-h) in wide-slice order
+  for (int64_t s = lane; s < S; s += 32) {
+    const int w = W.slice_wide[b * S + s];
+    if (w < 0) continue;
+    for (int o = 0; o < 4; ++o) {
+      double* pt = O.points + ((int64_t)b * O.capacity + occ + o * wide_count + w) * 3;
+      pt[0] = P.z_origin + (double)s * P.cell_m;
+      pt[1] = o == 0 ? h : (o == 1 ? -h : 0.0);
+      pt[2] = o == 2 ? h : (o == 3 ? -h : 0.0);
+    }
+  }
+  if (lane == 0) O.n_points[b] = occ + 4 * wide_count;
+}
+
+// One CTA per (slice, band, block of 2 `pairs` frequencies): time-lattice
+// transform and the slice's points (_shower_basis.py:577-611). One thread per
+// (channel, two frequencies) walks the slice's ticks with two rotating phasors, so
+// that a value read from shared memory is used four times; the CTA stages the
+// deposit rows of kSrcTransformBytes worth of ticks at a time (coalesced,
+// independent loads).
+constexpr int kSrcPairs = 8;
+constexpr int kSrcTransformBytes = 48 * 1024;
+
+// The sums of kMoments moments over the slice's ticks; `deposit` is the band's first
+// row, `stride` float64 values from tick to tick.
+template <int kMoments>
+LH_DEVICE void src_transform_ticks(const double* deposit, int64_t stride, int ticks, int nch,
+                                   double* s_dep, bool mine, int c, double (&pc)[2],
+                                   double (&ps)[2], const double (&dc)[2], const double (&ds)[2],
+                                   double (&re)[2][5], double (&im)[2][5]) {
+  // two buffers: the next ticks' rows are on their way while these are used
+  const int row = kMoments * nch;  // staged doubles per tick
+  const int room = (int)(kSrcTransformBytes / sizeof(double)) / 2;
+  const int chunk = max(1, min(64, room / row));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  auto fetch = [&](int t0, double* to) {
+    const int n_t = min(chunk, ticks - t0);
+    for (int tt = warp; tt < n_t; tt += warps) {
+      const double* from = deposit + (t0 + tt) * stride;
+      for (int r = lane; r < row; r += 32) copy_async8(to + tt * row + r, from + r);
+    }
+    copy_async_commit();
+  };
+  fetch(0, s_dep);
+  for (int t0 = 0, buf = 0; t0 < ticks; t0 += chunk, buf ^= 1) {
+    const int n_t = min(chunk, ticks - t0);
+    if (t0 + chunk < ticks) {
+      fetch(t0 + chunk, s_dep + (buf ^ 1) * room);
+      copy_async_wait<1>();
+    } else {
+      copy_async_wait<0>();
+    }
+    __syncthreads();
+    const double* rowp = s_dep + buf * room + c;
+    for (int tt = 0; tt < (mine ? n_t : 0); ++tt, rowp += row) {
+#pragma unroll
+      for (int k = 0; k < kMoments; ++k) {
+        const double v = rowp[k * nch];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          re[u][k] += v * pc[u];
+          im[u][k] += v * ps[u];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const double npc = pc[u] * dc[u] - ps[u] * ds[u], nps = ps[u] * dc[u] + pc[u] * ds[u];
+        pc[u] = npc;
+        ps[u] = nps;
+      }
+    }
+    __syncthreads();  // the buffer is filled again
   }
 }
 
-// One CTA per (slice, band, block of `w_block` frequencies): time-lattice
-// transform and the slice's points (_shower_basis.py:577-611). One thread per
-// (channel, frequency) walks the slice's ticks with a rotating phasor; the
-// CTA stages the deposit rows of kSrcStageBytes worth of ticks at a time in
-// shared memory (coalesced, independent loads) before the threads read them.
-constexpr int kSrcOmegaBlock = 8;
-constexpr int kSrcStageBytes = 48 * 1024;
-
-__global__ void src_transform_kernel(const lh_source_problem P, const int32_t* slice_lo,
-                                     const int32_t* slice_hi, const double* deposit,
-                                     const int32_t* slice_point, const int32_t* slice_wide,
-                                     const int32_t* n_occ, lh_source_output O, int w_block) {
+__global__ void __launch_bounds__(512)
+src_transform_kernel(const lh_source_problem P, const SrcWorkspace Wk, lh_source_output O,
+                     int pairs) {
   extern __shared__ double s_dep[];  // [tick][moment][channel]
   const int64_t s = blockIdx.x;
   const int b = blockIdx.y;
   const int NB = P.n_bands, nch = P.nch, W = P.n_omega;
-  if (slice_hi[s] < 0) return;
-  const int lo = slice_lo[s], hi = slice_hi[s];
-  const int64_t S = P.n_slices;
-  const int point = slice_point[b * S + s];
-  const int wide = slice_wide[b * S + s];
-  const int occ = *n_occ;
+  if (Wk.slice_hi[s] < 0) return;
+  const int lo = Wk.slice_lo[s], hi = Wk.slice_hi[s];
+  const int64_t S = P.n_slices, row0 = Wk.slice_row[s];
+  const int point = Wk.slice_point[b * S + s];
+  const int wide = Wk.slice_wide[b * S + s];
+  const int occ = Wk.n_groups[2];
   const int wide_count = (O.n_points[b] - occ) / 4;
   const double h = P.stencil_m, h2 = h * h;
   const double scale = P.band_scale[b];
-  const int w_begin = blockIdx.z * w_block;
-  const int w_count = min(w_block, W - w_begin);
-  const int nk = wide >= 0 ? 5 : 1;
-  const int row = nk * nch;  // staged doubles per tick
-  const int chunk = max(1, min(64, (int)(kSrcStageBytes / sizeof(double)) / row));
   const int i = threadIdx.x;
-  const bool mine = i < nch * w_count;
-  const int c = mine ? i % nch : 0, w = w_begin + (mine ? i / nch : 0);
-  const double om = P.omega[w];
-  double ps = 0, pc = 1, ds = 0, dc = 1;
-  if (mine) {
-    sincos(om * lo * P.time_step_ns, &ps, &pc);
-    sincos(om * P.time_step_ns, &ds, &dc);
+  const int c = i % nch, w0 = blockIdx.z * 2 * pairs + i / nch;
+  const bool mine = i < nch * pairs && w0 < W;
+  double ps[2], pc[2], ds[2], dc[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const double om = mine ? P.omega[min(w0 + u * pairs, W - 1)] : 0.0;
+    sincos(om * lo * P.time_step_ns, &ps[u], &pc[u]);
+    sincos(om * P.time_step_ns, &ds[u], &dc[u]);
   }
-  double re[5] = {0, 0, 0, 0, 0}, im[5] = {0, 0, 0, 0, 0};
-  for (int t0 = lo; t0 <= hi; t0 += chunk) {
-    const int n_t = min(chunk, hi - t0 + 1);
-    __syncthreads();
-    for (int e = threadIdx.x; e < n_t * row; e += blockDim.x) {
-      const int tt = e / row, r = e - tt * row;
-      s_dep[e] = deposit[(((s * P.kmax + t0 + tt) * NB + b) * 5) * nch + r];
-    }
-    __syncthreads();
-    if (!mine) continue;
-    for (int tt = 0; tt < n_t; ++tt) {
-      const double* rowp = s_dep + tt * row + c;
-      for (int k = 0; k < nk; ++k) {
-        const double v = rowp[k * nch];
-        re[k] += v * pc;
-        im[k] += v * ps;
-      }
-      const double npc = pc * dc - ps * ds, nps = ps * dc + pc * ds;
-      pc = npc;
-      ps = nps;
-    }
-  }
-  if (mine) {
-    float2* out = reinterpret_cast<float2*>(O.channels);
-    auto put = [&](int p, double r, double m) {
+  double re[2][5] = {}, im[2][5] = {};
+  const double* deposit = Wk.deposit + (row0 * NB + b) * 5 * (int64_t)nch;
+  const int64_t stride = (int64_t)NB * 5 * nch;
+  if (wide >= 0)
+    src_transform_ticks<5>(deposit, stride, hi - lo + 1, nch, s_dep, mine, c, pc, ps, dc, ds, re, im);
+  else
+    src_transform_ticks<1>(deposit, stride, hi - lo + 1, nch, s_dep, mine, c, pc, ps, dc, ds, re, im);
+  if (!mine) return;
+  float2* out = reinterpret_cast<float2*>(O.channels);
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int w = w0 + u * pairs;
+    if (w >= W) continue;
+    const double* r = re[u];
+    const double* m = im[u];
+    auto put = [&](int p, double vr, double vi) {
       out[(((int64_t)b * O.capacity + p) * nch + c) * W + w] =
-          make_float2((float)(scale * r), (float)(scale * m));
+          make_float2((float)(scale * vr), (float)(scale * vi));
     };
     if (wide < 0) {
-      put(point, re[0], im[0]);
+      put(point, r[0], m[0]);
     } else {
       // m0, mx, my, mxx, myy -> centre, +x, -x, +y, -y
-      put(point, re[0] - (re[3] + re[4]) / h2, im[0] - (im[3] + im[4]) / h2);
-      put(occ + 0 * wide_count + wide, 0.5 * (re[3] / h2 + re[1] / h), 0.5 * (im[3] / h2 + im[1] / h));
-      put(occ + 1 * wide_count + wide, 0.5 * (re[3] / h2 - re[1] / h), 0.5 * (im[3] / h2 - im[1] / h));
-      put(occ + 2 * wide_count + wide, 0.5 * (re[4] / h2 + re[2] / h), 0.5 * (im[4] / h2 + im[2] / h));
-      put(occ + 3 * wide_count + wide, 0.5 * (re[4] / h2 - re[2] / h), 0.5 * (im[4] / h2 - im[2] / h));
+      put(point, r[0] - (r[3] + r[4]) / h2, m[0] - (m[3] + m[4]) / h2);
+      put(occ + 0 * wide_count + wide, 0.5 * (r[3] / h2 + r[1] / h), 0.5 * (m[3] / h2 + m[1] / h));
+      put(occ + 1 * wide_count + wide, 0.5 * (r[3] / h2 - r[1] / h), 0.5 * (m[3] / h2 - m[1] / h));
+      put(occ + 2 * wide_count + wide, 0.5 * (r[4] / h2 + r[2] / h), 0.5 * (m[4] / h2 + m[2] / h));
+      put(occ + 3 * wide_count + wide, 0.5 * (r[4] / h2 - r[2] / h), 0.5 * (m[4] / h2 - m[2] / h));
     }
   }
 }
-
-struct SrcWorkspace {
-  SrcNode* nodes;
-  int32_t *counts, *offsets, *cursor, *order, *n_groups, *slice_lo, *slice_hi, *slice_point,
-      *slice_wide, *n_occ;
-  int64_t* groups;
-  double *deposit, *zero, *centroid;
-  size_t bytes;
-};
 
 static size_t src_align(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -488,21 +527,22 @@ static SrcWorkspace src_layout(const lh_source_problem& P, unsigned char* base) 
   const int64_t n_nodes = (int64_t)P.n_el * P.element_order;
   const int64_t n_keys = P.n_slices * P.kmax;
   const int NB = P.n_bands;
-  W.nodes = reinterpret_cast<SrcNode*>(take(sizeof(SrcNode) * n_nodes));
+  // cleared together: counts, n_groups, zero
   W.counts = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * n_keys));
+  W.n_groups = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * 4));
+  W.zero = reinterpret_cast<double*>(take(sizeof(double) * P.n_slices * NB * 5));
+  W.slice_lo = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * P.n_slices));
+  W.slice_hi = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * P.n_slices));
+  W.key = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * n_nodes));
+  W.rows = reinterpret_cast<double*>(take(sizeof(double) * src_row(P).size * n_nodes));
   W.offsets = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * n_keys));
   W.cursor = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * n_keys));
   W.order = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * n_nodes));
-  W.groups = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * n_keys));
-  W.n_groups = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * 4));
-  W.n_occ = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * 4));
-  W.slice_lo = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * P.n_slices));
-  W.slice_hi = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * P.n_slices));
+  W.groups = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * std::min(n_keys, n_nodes)));
+  W.slice_row = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * (P.n_slices + 1)));
   W.slice_point = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * P.n_slices * NB));
   W.slice_wide = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * P.n_slices * NB));
   W.deposit = reinterpret_cast<double*>(take(sizeof(double) * n_keys * NB * 5 * P.nch));
-  W.zero = reinterpret_cast<double*>(take(sizeof(double) * P.n_slices * NB * 5));
-  W.centroid = reinterpret_cast<double*>(take(sizeof(double) * P.n_slices * NB * 2));
   W.bytes = off;
   return W;
 }
@@ -540,39 +580,30 @@ extern "C" int lh_source_compile(const lh_source_problem* P, const lh_source_out
   lh::SrcWorkspace W = lh::src_layout(*P, static_cast<unsigned char*>(workspace));
   if (!workspace || workspace_bytes < W.bytes) return LH_ENOMEM;
   const int64_t n_nodes = (int64_t)P->n_el * P->element_order;
-  const int64_t n_keys = P->n_slices * P->kmax;
   const int NB = P->n_bands;
-  cudaMemsetAsync(W.counts, 0, sizeof(int32_t) * n_keys, s);
+  const int threads = ((5 * P->nch + 31) / 32) * 32;  // of the group kernel: at most 768
+  const size_t gsmem = sizeof(double) * lh::src_row(*P).size * (size_t)lh::src_chunk(*P);
+  cudaMemsetAsync(W.counts, 0, reinterpret_cast<unsigned char*>(W.slice_lo) -
+                                   reinterpret_cast<unsigned char*>(W.counts), s);
   cudaMemsetAsync(W.slice_lo, 0x7f, sizeof(int32_t) * P->n_slices, s);
   cudaMemsetAsync(W.slice_hi, 0xff, sizeof(int32_t) * P->n_slices, s);
-  cudaMemsetAsync(W.deposit, 0, sizeof(double) * n_keys * NB * 5 * P->nch, s);
-  cudaMemsetAsync(W.zero, 0, sizeof(double) * P->n_slices * NB * 5, s);
   cudaMemsetAsync(O->channels, 0, sizeof(float) * 2 * NB * O->capacity * P->nch * P->n_omega, s);
-  int blocks = (int)std::min<int64_t>((n_nodes + 255) / 256, 148 * 32);
-  lh::src_nodes_kernel<<<std::max(blocks, 1), 256, 0, s>>>(*P, W.nodes, W.counts, W.slice_lo,
-                                                          W.slice_hi, status);
-  lh::src_scan_kernel<<<1, 1024, 0, s>>>(n_keys, W.counts, W.offsets, W.cursor, W.groups,
-                                         W.n_groups);
-  lh::src_scatter_kernel<<<std::max(blocks, 1), 256, 0, s>>>(*P, W.nodes, W.cursor, W.order);
-  const size_t gsmem = sizeof(lh::SrcGroupShared) + sizeof(double) * (NB * 45 * P->nch + NB * 20);
-  if (gsmem > 200 * 1024) return LH_EUNSUPPORTED;
-  if (cudaFuncSetAttribute(lh::src_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)gsmem) != cudaSuccess)
-    return LH_ECUDA;
+  lh::src_nodes_kernel<<<(unsigned)((n_nodes + 63) / 64), 64, 0, s>>>(*P, W, status);
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n_nodes + 255) / 256, 148 * 4));
+  lh::src_rows_kernel<<<1 + blocks, 256, 0, s>>>(*P, W);
+  lh::src_scatter_kernel<<<148 * 8, 256, 0, s>>>(*P, W);
   {
     lh::TimedLaunch timed_launch(LH_KT_SRC_GROUP, s);
-    lh::src_group_kernel<<<148 * 4, lh::kSrcThreads, gsmem, s>>>(
-        *P, W.nodes, W.offsets, W.counts, W.order, W.groups, W.n_groups, W.deposit, W.zero);
+    lh::src_group_kernel<<<148 * 8, threads, gsmem, s>>>(*P, W);
   }
-  lh::src_layout_kernel<<<1, 32, 0, s>>>(*P, W.slice_lo, W.slice_hi, W.zero, W.slice_point,
-                                         W.slice_wide, W.centroid, W.n_occ, *O);
-  const int w_block = std::max(1, std::min(lh::kSrcOmegaBlock, 1024 / P->nch));
-  dim3 grid((unsigned)P->n_slices, (unsigned)NB, (unsigned)((P->n_omega + w_block - 1) / w_block));
-  const int threads = ((P->nch * w_block + 31) / 32) * 32;
+  lh::src_layout_kernel<<<1, 32 * NB, 0, s>>>(*P, W, *O);
+  const int pairs = std::max(1, std::min(lh::kSrcPairs, 512 / P->nch));
+  dim3 grid((unsigned)P->n_slices, (unsigned)NB,
+            (unsigned)((P->n_omega + 2 * pairs - 1) / (2 * pairs)));
   {
     lh::TimedLaunch timed_launch(LH_KT_SRC_TRANSFORM, s);
-    lh::src_transform_kernel<<<grid, threads, lh::kSrcStageBytes, s>>>(
-        *P, W.slice_lo, W.slice_hi, W.deposit, W.slice_point, W.slice_wide, W.n_occ, *O, w_block);
+    lh::src_transform_kernel<<<grid, ((P->nch * pairs + 31) / 32) * 32, lh::kSrcTransformBytes,
+                               s>>>(*P, W, *O, pairs);
   }
   return cudaGetLastError() == cudaSuccess ? LH_OK : LH_ECUDA;
 }
