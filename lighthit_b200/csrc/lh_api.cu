@@ -10,11 +10,9 @@
 namespace lh {
 __global__ void flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins,
                                    float* a_rows);
-__global__ void flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* g_bhi,
-                                const __nv_bfloat16* g_blo, int kpad, int n_bins, int n_tile,
-                                int passes);
-size_t flash_tc_smem_bytes(int kpad, int n_tile);
-__global__ void flash_combine_kernel(lh_flash_problem p, lh_flash_nodes nd, lh_flash_batch b);
+size_t flash_tc_smem_bytes(int kpad, int n_tile, bool sorted);
+__global__ void flash_combine_kernel(const lh_flash_problem p, const lh_flash_nodes nd,
+                                     const lh_flash_batch b);
 }  // namespace lh
 
 using namespace lh;
@@ -150,17 +148,22 @@ int lh_flash_transport(const lh_flash_problem* p, const lh_readout_operator* op,
     return check_launch();
   }
   if (op->n_tiles != 1) return LH_EUNSUPPORTED;  // fused path: all bins in one tile
-  size_t smem = flash_tc_smem_bytes(op->k_pad, op->n_tile);
+  // the sort by radial interval needs 12 KB more: operators that leave less are
+  // run in the order of their pairs
+  const bool sorted = flash_tc_smem_bytes(op->k_pad, op->n_tile, true) <= 227 * 1024;
+  size_t smem = flash_tc_smem_bytes(op->k_pad, op->n_tile, sorted);
   if (smem > 227 * 1024) return LH_EUNSUPPORTED;
-  cudaFuncSetAttribute(flash_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+  const FlashTcKernel kernel = flash_tc_kernel_of(p->acc_top + 1);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int grid = (int)(n_pairs < sm_count() ? n_pairs : sm_count());
   const int threads = b->block_threads == 0 ? 512 : b->block_threads;
   if (threads != 256 && threads != 512) return LH_EINVAL;
   {
     lh::TimedLaunch timed_launch(LH_KT_FLASH, s);
-    flash_tc_kernel<<<grid, threads, smem, s>>>(*p, *b, reinterpret_cast<const __nv_bfloat16*>(op->b_hi),
-                                            reinterpret_cast<const __nv_bfloat16*>(op->b_lo),
-                                            op->k_pad, op->n_bins, op->n_tile, passes_of(mode));
+    kernel<<<grid, threads, smem, s>>>(*p, *b, reinterpret_cast<const __nv_bfloat16*>(op->b_hi),
+                                       reinterpret_cast<const __nv_bfloat16*>(op->b_lo),
+                                       op->k_pad, op->n_bins, op->n_tile, passes_of(mode),
+                                       sorted ? 1 : 0);
   }
   return check_launch();
 }

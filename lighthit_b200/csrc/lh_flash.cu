@@ -41,6 +41,7 @@ struct FlashPair {
   double t0;      // absolute order-0 phase time (r / speed inside, t + r / speed outside)
   double q0;      // order-0 bin weight
   double c12, c0, cr;  // t12, t0 and t12 - origin in turns per (rad/ns): t / (2 pi)
+  int64_t pair;   // flash * n_om + OM
   float tt;       // offset in the log-r interval
   float amp12;    // photons * area * efficiency * exp(-mu_a r) / (4 pi r^2)
   float amp0;     // order-0 amplitude
@@ -156,35 +157,39 @@ LH_DEVICE float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// Step 2 for one (pair, omega). Returns the relative spectra of orders 1, 2
-// through rel1/rel2 and writes the absolute spectrum of all orders.
-LH_DEVICE void flash_item(const lh_flash_problem& p, const lh_flash_batch& b, int64_t pair,
-                          int w, FlashPair& s, float2& rel1, float2& rel2) {
-  const double om = p.omega[w];
-  float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f);
+// One degree's cubic coefficients of orders 1 and 2 at one frequency.
+struct FlashCoef {
+  float2 a0, a1, a2, a3;  // order 1: c0..c3
+  float2 b0, b1, b2, b3;  // order 2
+};
+
+// [interval][degree][order][power][omega]: the lanes of a warp (consecutive
+// omega) read consecutive float2, one coalesced segment per coefficient.
+LH_DEVICE FlashCoef flash_coef(const lh_flash_problem& p, int j, int l, int w) {
+  const int W = p.n_omega;
+  const float2* c = reinterpret_cast<const float2*>(p.coef) +
+                    ((int64_t)j * (p.acc_top + 1) + l) * 8 * W + w;
+  return FlashCoef{__ldg(c),         __ldg(c + W),     __ldg(c + 2 * W), __ldg(c + 3 * W),
+                   __ldg(c + 4 * W), __ldg(c + 5 * W), __ldg(c + 6 * W), __ldg(c + 7 * W)};
+}
+
+LH_DEVICE void flash_degree(const FlashCoef& c, float t, float wl, float2& s1, float2& s2) {
+  float vr = fmaf(fmaf(fmaf(c.a0.x, t, c.a1.x), t, c.a2.x), t, c.a3.x);
+  float vi = fmaf(fmaf(fmaf(c.a0.y, t, c.a1.y), t, c.a2.y), t, c.a3.y);
+  s1.x = fmaf(wl, vr, s1.x);
+  s1.y = fmaf(wl, vi, s1.y);
+  vr = fmaf(fmaf(fmaf(c.b0.x, t, c.b1.x), t, c.b2.x), t, c.b3.x);
+  vi = fmaf(fmaf(fmaf(c.b0.y, t, c.b1.y), t, c.b2.y), t, c.b3.y);
+  s2.x = fmaf(wl, vr, s2.x);
+  s2.y = fmaf(wl, vi, s2.y);
+}
+
+// Step 2 for one (pair, omega) from its contracted spectra s1, s2 (zero outside the
+// table): returns the relative spectra of orders 1, 2 through rel1/rel2 and writes
+// the absolute spectrum of all orders.
+LH_DEVICE void flash_item(const lh_flash_problem& p, const lh_flash_batch& b, int w, double om,
+                          FlashPair& s, float2 s1, float2 s2, float2& rel1, float2& rel2) {
   if (s.j >= 0) {
-    const int L = p.acc_top + 1;
-    const int W = p.n_omega;
-    // [interval][degree][order][power][omega]: the lanes of a warp (consecutive
-    // omega) read consecutive float2, one coalesced segment per coefficient
-    const float2* c = reinterpret_cast<const float2*>(p.coef) + (int64_t)s.j * L * 8 * W + w;
-    const float t = s.tt;
-    for (int l = 0; l < L; ++l) {
-      const float2* cl = c + (int64_t)l * 8 * W;
-      const float2 a0 = __ldg(cl), a1 = __ldg(cl + W), a2 = __ldg(cl + 2 * W),
-                   a3 = __ldg(cl + 3 * W);  // order 1: c0..c3
-      const float2 b0 = __ldg(cl + 4 * W), b1 = __ldg(cl + 5 * W), b2 = __ldg(cl + 6 * W),
-                   b3 = __ldg(cl + 7 * W);  // order 2
-      float vr = fmaf(fmaf(fmaf(a0.x, t, a1.x), t, a2.x), t, a3.x);
-      float vi = fmaf(fmaf(fmaf(a0.y, t, a1.y), t, a2.y), t, a3.y);
-      const float wl = s.w[l];
-      s1.x = fmaf(wl, vr, s1.x);
-      s1.y = fmaf(wl, vi, s1.y);
-      vr = fmaf(fmaf(fmaf(b0.x, t, b1.x), t, b2.x), t, b3.x);
-      vi = fmaf(fmaf(fmaf(b0.y, t, b1.y), t, b2.y), t, b3.y);
-      s2.x = fmaf(wl, vr, s2.x);
-      s2.y = fmaf(wl, vi, s2.y);
-    }
     s1.x *= s.amp12; s1.y *= s.amp12;
     s2.x *= s.amp12; s2.y *= s.amp12;
   }
@@ -194,7 +199,7 @@ LH_DEVICE void flash_item(const lh_flash_problem& p, const lh_flash_batch& b, in
   const float2 o0 = make_float2(s.amp0 * e0.x, s.amp0 * e0.y);
   const float2 o1 = cmul(s1, e12), o2 = cmul(s2, e12);
   if (s.valid) {
-    float2* out = reinterpret_cast<float2*>(b.spectrum) + (pair * p.n_omega + w) * 3;
+    float2* out = reinterpret_cast<float2*>(b.spectrum) + (s.pair * p.n_omega + w) * 3;
     out[0] = o0;
     out[1] = o1;
     out[2] = o2;
@@ -211,7 +216,7 @@ LH_DEVICE void flash_item(const lh_flash_problem& p, const lh_flash_batch& b, in
 // Step 3 (order 0 and the mask) for the tile's pairs.
 // `threads`: the first threads of the CTA that take part (0: all).
 LH_DEVICE void flash_tile_order0(const lh_flash_problem& p, const lh_flash_batch& b,
-                                 const FlashPair* sp, int64_t base, int n_bins, int threads = 0) {
+                                 const FlashPair* sp, int n_bins, int threads = 0) {
   const int stride = threads ? threads : (int)blockDim.x;
   if ((n_bins & 3) == 0) {  // rows are 16-byte aligned: four bins per store
     const int quads = n_bins >> 2;
@@ -222,20 +227,20 @@ LH_DEVICE void flash_tile_order0(const lh_flash_problem& p, const lh_flash_batch
       const float q = (float)s.q0;
       const float4 v = make_float4(bin == s.bin0 ? q : 0.f, bin + 1 == s.bin0 ? q : 0.f,
                                    bin + 2 == s.bin0 ? q : 0.f, bin + 3 == s.bin0 ? q : 0.f);
-      *reinterpret_cast<float4*>(b.components + ((base + lp) * 3) * n_bins + bin) = v;
+      *reinterpret_cast<float4*>(b.components + (s.pair * 3) * n_bins + bin) = v;
     }
   } else {
     for (int i = threadIdx.x; i < kFlashPairs * n_bins; i += stride) {
       const int lp = i / n_bins, bin = i % n_bins;
       const FlashPair& s = sp[lp];
       if (!s.valid) continue;
-      b.components[((base + lp) * 3) * n_bins + bin] = (bin == s.bin0) ? (float)s.q0 : 0.f;
+      b.components[(s.pair * 3) * n_bins + bin] = (bin == s.bin0) ? (float)s.q0 : 0.f;
     }
   }
   if (threadIdx.x < kFlashPairs) {
     const FlashPair& s = sp[threadIdx.x];
     if (s.valid) {
-      const int64_t pair = base + threadIdx.x;
+      const int64_t pair = s.pair;
       const double q = ((double)s.charge[0] + (double)s.charge[1]) + (double)s.charge[2];
       for (int o = 0; o < 3; ++o) b.charge[pair * 3 + o] = (double)s.charge[o];
       b.origin[pair] = s.origin;
@@ -247,6 +252,7 @@ LH_DEVICE void flash_tile_order0(const lh_flash_problem& p, const lh_flash_batch
 
 LH_DEVICE void flash_slot_setup(const lh_flash_problem& p, const lh_flash_batch& b, FlashPair& s,
                                 int64_t pair, int64_t n_pairs) {
+  s.pair = pair;
   if (pair < n_pairs) {
     flash_pair_setup(p, b, pair, s);
   } else {
@@ -285,8 +291,12 @@ flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins, f
   const int64_t host_pairs = (int64_t)b.n_flash * p.n_om;
   for (int i = threadIdx.x; i < kFlashPairs * nw; i += blockDim.x) {
     const int lp = i / nw, w = i % nw;
-    float2 r1, r2;
-    flash_item(p, b, base + lp, w, sp[lp], r1, r2);
+    FlashPair& pair = sp[lp];
+    float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f), r1, r2;
+    if (pair.j >= 0)
+      for (int l = 0; l <= p.acc_top; ++l)
+        flash_degree(flash_coef(p, pair.j, l, w), pair.tt, pair.w[l], s1, s2);
+    flash_item(p, b, w, p.omega[w], pair, s1, s2, r1, r2);
     if (base + lp < host_pairs) {
       float* row1 = a_rows + (2 * (base + lp)) * (int64_t)kpad;
       float* row2 = row1 + kpad;
@@ -301,18 +311,49 @@ flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins, f
     }
   }
   __syncthreads();
-  flash_tile_order0(p, b, sp, base, n_bins);
+  flash_tile_order0(p, b, sp, n_bins);
 }
 
 // ---------------------------------------------------------------- fused tcgen05 path
-// 256 threads, one CTA per SM, persistent over tiles. B (the readout operator,
-// hi and lo parts) is loaded once per CTA. Per tile: setup -> spectrum items
-// writing A (bf16 hi/lo) into shared memory -> one thread issues the MMAs ->
-// order-0 rows and mask while the tensor core runs -> TMEM drain.
+// One CTA per SM, each over its share of consecutive pairs. B (the readout
+// operator, hi and lo parts) is loaded once per CTA. The CTA sorts up to
+// kFlashSort pairs at a time by radial interval and takes them in tiles of 64: a
+// thread holds the cubic coefficients of its frequency in registers and runs over
+// neighbouring pairs, reading coefficients only where the interval changes. Per
+// tile: setup -> spectrum items writing A (bf16 hi/lo) into shared memory -> one
+// thread issues the MMAs -> order-0 rows and mask while the tensor core runs ->
+// TMEM drain. A share of few pairs (a single flash) spreads over the SMs pair by
+// pair. kDegrees: acceptance degrees whose coefficients a thread holds (0: any,
+// read for every pair; four degrees or more would not fit beside the rest in the 128
+// registers of a thread).
+//
+// What bounds it: the outputs (65 frequencies x 24 bytes and 480 bins x 4 bytes a
+// pair) take 0.1 ms for 4096 flashes of 48 OMs, the spectra another 0.19 ms that
+// nothing overlaps, since the A tile and the operator leave shared memory for one
+// tile only. With coefficients read for every pair (192 bytes a pair and frequency
+// through L1) the same launch took 0.380 ms, sorted it takes 0.345. A single flash
+// (48 pairs on one CTA before, on 48 now): 21.8 us, now 13.7.
+constexpr int kFlashSort = 2048;        // pairs sorted at a time
+constexpr int kFlashMaxBuckets = 1024;  // radial intervals the sort tells apart
+
+// The pair's radial interval for the sort, in float32: where it is off by one the
+// pair only sits between neighbours of another interval.
+LH_DEVICE int flash_bucket(const lh_flash_problem& p, const lh_flash_batch& b, int64_t pair,
+                           int buckets) {
+  const int64_t f = pair / p.n_om;
+  const int d = (int)(pair - f * p.n_om);
+  const float dx = (float)(p.om_pos[3 * d] - b.pos[3 * f]),
+              dy = (float)(p.om_pos[3 * d + 1] - b.pos[3 * f + 1]),
+              dz = (float)(p.om_pos[3 * d + 2] - b.pos[3 * f + 2]);
+  const int j = bin_right(p.log_r, p.n_radii, 0.5f * __logf(dx * dx + dy * dy + dz * dz)) + 1;
+  return min(max(j, 0), buckets - 1);
+}
+
+template <int kDegrees>
 __global__ void __launch_bounds__(kFlashTcThreads, 1)
 flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __restrict__ g_bhi,
                 const __nv_bfloat16* __restrict__ g_blo, int kpad, int n_bins, int n_tile,
-                int passes) {
+                int passes, int sorted) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t a_bytes = (uint32_t)(kpad / 8) * kAChunk * 2u;
   const uint32_t b_bytes = (uint32_t)n_tile * kpad * 2u;
@@ -324,6 +365,9 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
   FlashPair* sp_buf = reinterpret_cast<FlashPair*>(smem + 2 * a_bytes + 2 * b_bytes);
   uint64_t* bars = reinterpret_cast<uint64_t*>(sp_buf + 2 * kFlashPairs);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 2);
+  uint16_t* s_order = reinterpret_cast<uint16_t*>(bars + 4);  // pairs of the share by interval
+  uint16_t* s_bucket = s_order + kFlashSort;
+  int* s_count = reinterpret_cast<int*>(s_bucket + kFlashSort);  // [buckets]
   uint64_t* bar_b = bars;
   uint64_t* bar_mma = bars + 1;
 
@@ -349,18 +393,57 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
   }
   const uint32_t idesc = instr_desc_bf16_f32(128, n_tile);
   const int64_t n_pairs = (int64_t)flash_count(b) * p.n_om;
-  const int64_t n_tiles = (n_pairs + kFlashPairs - 1) / kFlashPairs;
   const int nw = p.n_omega;
   const int padw = kpad - 2 * nw;
   uint32_t ph_mma = 0;
   bool b_ready = false, failed = false, mma_pending = false;
 
-  if (blockIdx.x < n_tiles) flash_tile_setup(p, b, sp_buf, blockIdx.x * kFlashPairs, n_pairs);
+  // this CTA's share of the pairs
+  const int64_t share = (n_pairs + gridDim.x - 1) / gridDim.x;
+  const int64_t share_begin = min(n_pairs, (int64_t)blockIdx.x * share);
+  const int64_t share_end = min(n_pairs, share_begin + share);
+  const int buckets = min(p.n_radii + 1, kFlashMaxBuckets);
+  const int workers = blockDim.x - 32;
+  // spectrum items: thread (group of pairs, frequency)
+  const int groups = max(1, workers / nw), group = tid / nw;
+  for (int64_t chunk = share_begin; chunk < share_end && !failed; chunk += kFlashSort) {
+  const int in_chunk = (int)min((int64_t)kFlashSort, share_end - chunk);
+  for (int i = tid; sorted && i < buckets; i += blockDim.x) s_count[i] = 0;
   __syncthreads();
+  for (int i = tid; sorted && i < in_chunk; i += blockDim.x) {
+    const int j = flash_bucket(p, b, chunk + i, buckets);
+    s_bucket[i] = (uint16_t)j;
+    atomicAdd(s_count + j, 1);
+  }
+  __syncthreads();
+  if (sorted && warp == 0) {  // exclusive prefix sums
+    int carry = 0;
+    for (int first = 0; first < buckets; first += 32) {
+      const int v = first + lane < buckets ? s_count[first + lane] : 0;
+      int sum = v;
+      for (int off = 1; off < 32; off <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, sum, off);
+        if (lane >= off) sum += up;
+      }
+      if (first + lane < buckets) s_count[first + lane] = carry + sum - v;
+      carry += __shfl_sync(0xffffffffu, sum, 31);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; sorted && i < in_chunk; i += blockDim.x)
+    s_order[atomicAdd(s_count + s_bucket[i], 1)] = (uint16_t)i;
+  __syncthreads();
+  // the pair at place k of the sorted chunk, past its end none
+  auto pair_at = [&](int k) {
+    return k < in_chunk ? chunk + (sorted ? (int)s_order[k] : k) : n_pairs;
+  };
+  const int tiles = (in_chunk + kFlashPairs - 1) / kFlashPairs;
   int cur = 0;
-  for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const int64_t base = tile * kFlashPairs;
+  if (tid < kFlashPairs) flash_slot_setup(p, b, sp_buf[tid], pair_at(tid), n_pairs);
+  __syncthreads();
+  for (int tile = 0; tile < tiles; ++tile) {
     FlashPair* sp = sp_buf + cur * kFlashPairs;  // set up before the barrier closing the last tile
+    const int count = min(kFlashPairs, in_chunk - tile * kFlashPairs);
     for (int i = tid; i < 128 * padw; i += blockDim.x) {
       const int off = a_offset(i / padw, 2 * nw + i % padw);
       s_ahi[off] = __float2bfloat16_rn(0.f);
@@ -369,30 +452,49 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
     // The last warp sets up the next tile's pairs (float64, two per lane) while
     // the other warps compute this tile's spectra, then issues the MMAs while
     // they write the order-0 rows: neither waits behind the other.
-    const int64_t next = tile + gridDim.x;
-    const int workers = blockDim.x - 32;
     if (tid >= workers) {
-      if (next < n_tiles)
+      if (tile + 1 < tiles)
         for (int k = lane; k < kFlashPairs; k += 32)
-          flash_slot_setup(p, b, sp_buf[(cur ^ 1) * kFlashPairs + k], next * kFlashPairs + k,
-                           n_pairs);
-    } else {
-      for (int i = tid; i < kFlashPairs * nw; i += workers) {
-        const int lp = i / nw, w = i % nw;
-        float2 r1, r2;
-        flash_item(p, b, base + lp, w, sp[lp], r1, r2);
-        // K columns (Re, Im) per frequency: one bf16x2 store per row and part
-        const __nv_bfloat162 h1 = __floats2bfloat162_rn(r1.x, r1.y);
-        const __nv_bfloat162 l1 = __floats2bfloat162_rn(r1.x - __low2float(h1),
-                                                        r1.y - __high2float(h1));
-        const __nv_bfloat162 h2 = __floats2bfloat162_rn(r2.x, r2.y);
-        const __nv_bfloat162 l2 = __floats2bfloat162_rn(r2.x - __low2float(h2),
-                                                        r2.y - __high2float(h2));
-        const int o1 = a_offset(2 * lp, 2 * w), o2 = a_offset(2 * lp + 1, 2 * w);
-        *reinterpret_cast<__nv_bfloat162*>(s_ahi + o1) = h1;
-        *reinterpret_cast<__nv_bfloat162*>(s_alo + o1) = l1;
-        *reinterpret_cast<__nv_bfloat162*>(s_ahi + o2) = h2;
-        *reinterpret_cast<__nv_bfloat162*>(s_alo + o2) = l2;
+          flash_slot_setup(p, b, sp_buf[(cur ^ 1) * kFlashPairs + k],
+                           pair_at((tile + 1) * kFlashPairs + k), n_pairs);
+    } else if (group < groups) {
+      const int first = group * count / groups, last = (group + 1) * count / groups;
+      for (int w = tid - group * nw; w < nw; w += workers) {
+        const double om = p.omega[w];
+        constexpr int kHeld = kDegrees > 0 ? kDegrees : 1;
+        FlashCoef held[kHeld];
+        int j_held = -1;
+        for (int lp = first; lp < last; ++lp) {
+          FlashPair& s = sp[lp];
+          float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f), r1, r2;
+          if (s.j >= 0) {
+            if (kDegrees > 0) {
+              if (s.j != j_held) {
+                j_held = s.j;
+#pragma unroll
+                for (int l = 0; l < kHeld; ++l) held[l] = flash_coef(p, j_held, l, w);
+              }
+#pragma unroll
+              for (int l = 0; l < kHeld; ++l) flash_degree(held[l], s.tt, s.w[l], s1, s2);
+            } else {
+              for (int l = 0; l <= p.acc_top; ++l)
+                flash_degree(flash_coef(p, s.j, l, w), s.tt, s.w[l], s1, s2);
+            }
+          }
+          flash_item(p, b, w, om, s, s1, s2, r1, r2);
+          // K columns (Re, Im) per frequency: one bf16x2 store per row and part
+          const __nv_bfloat162 h1 = __floats2bfloat162_rn(r1.x, r1.y);
+          const __nv_bfloat162 l1 = __floats2bfloat162_rn(r1.x - __low2float(h1),
+                                                          r1.y - __high2float(h1));
+          const __nv_bfloat162 h2 = __floats2bfloat162_rn(r2.x, r2.y);
+          const __nv_bfloat162 l2 = __floats2bfloat162_rn(r2.x - __low2float(h2),
+                                                          r2.y - __high2float(h2));
+          const int o1 = a_offset(2 * lp, 2 * w), o2 = a_offset(2 * lp + 1, 2 * w);
+          *reinterpret_cast<__nv_bfloat162*>(s_ahi + o1) = h1;
+          *reinterpret_cast<__nv_bfloat162*>(s_alo + o1) = l1;
+          *reinterpret_cast<__nv_bfloat162*>(s_ahi + o2) = h2;
+          *reinterpret_cast<__nv_bfloat162*>(s_alo + o2) = l2;
+        }
       }
     }
     fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core
@@ -425,7 +527,7 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
         failed = true;
       }
     }
-    if (tid < workers) flash_tile_order0(p, b, sp, base, n_bins, workers);
+    if (tid < workers) flash_tile_order0(p, b, sp, n_bins, workers);
     if (__syncthreads_or(failed)) { failed = true; break; }
     const bool ok = mbar_wait(bar_mma, ph_mma);
     ph_mma ^= 1u;
@@ -433,15 +535,15 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
     tc_fence_after();
     // drain: warp w reads TMEM lanes 32*(w%4).. (rows); the warps with the same
     // lane quarter split the 16-column chunks between them
-    const int q = warp & 3, h = warp >> 2, groups = (int)blockDim.x / 128;
+    const int q = warp & 3, h = warp >> 2, quarters = (int)blockDim.x / 128;
     const int row = q * 32 + lane;
     const int lp = row >> 1, order = 1 + (row & 1);
     const bool valid = sp[lp].valid;
     const int chunks = n_tile / 16;
-    const int per = (chunks + groups - 1) / groups;
+    const int per = (chunks + quarters - 1) / quarters;
     const int c_begin = h * per, c_end = min(chunks, (h + 1) * per);
     const uint32_t lane_addr = tmem + ((uint32_t)(q * 32) << 16);
-    float* dst = b.components + ((base + lp) * 3 + order) * (int64_t)n_bins;
+    float* dst = b.components + (sp[lp].pair * 3 + order) * (int64_t)n_bins;
     const bool vec = (n_bins & 3) == 0;
     // The A tile is free once the MMA has completed: each warp transposes its
     // 32 rows x 16 bins through a 32 x 20-float slice of it, so that four
@@ -465,7 +567,7 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
           const int tlp = trow >> 1, torder = 1 + (trow & 1);
           if (sp[tlp].valid) {
             const float4 x = *reinterpret_cast<const float4*>(stage + r * 20 + 4 * part);
-            *reinterpret_cast<float4*>(b.components + ((base + tlp) * 3 + torder) * (int64_t)n_bins +
+            *reinterpret_cast<float4*>(b.components + (sp[tlp].pair * 3 + torder) * (int64_t)n_bins +
                                        c * 16 + 4 * part) = x;
           }
         }
@@ -480,6 +582,7 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
     __syncthreads();
     cur ^= 1;
   }
+  }  // chunks
   if (failed && tid == 0) atomicOr(reinterpret_cast<unsigned*>(b.status), LH_STATUS_TIMEOUT);
   if (mma_pending) mbar_wait(bar_mma, ph_mma ^ 1u);
   if (tid == blockDim.x - 32 && !b_ready) mbar_wait(bar_b, 0);  // no bulk copy left in flight
@@ -489,27 +592,64 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
 }
 
 // ---------------------------------------------------------------- broadband
+// out[i] = the nodes' values in node order, four at a time where every array is
+// 16-byte aligned. What bounds it is the copy of (nodes + 1) arrays: one float per
+// thread and step kept too few loads on their way (0.175 ms for 337 MB, 501
+// flashes of three nodes; 0.052 ms now, 6.4 TB/s).
+LH_DEVICE void flash_sum_nodes(const float* const* from, int n_nodes, float* out, int64_t n,
+                               int64_t first, int64_t stride) {
+  bool aligned = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  for (int k = 0; k < n_nodes; ++k) aligned &= (reinterpret_cast<uintptr_t>(from[k]) & 15) == 0;
+  int64_t done = 0;
+  if (aligned) {
+    const int64_t quads = n >> 2;
+    done = quads << 2;
+    constexpr int kAhead = 4;  // steps on their way per thread
+    for (int64_t i0 = first; i0 < quads; i0 += kAhead * stride) {
+      float4 v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int k = 0; k < n_nodes; ++k) {
+        const float4* src = reinterpret_cast<const float4*>(from[k]);
+        float4 x[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+          if (i0 + u * stride < quads) x[u] = __ldcs(src + i0 + u * stride);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+          if (i0 + u * stride < quads) {
+            v[u].x += x[u].x;
+            v[u].y += x[u].y;
+            v[u].z += x[u].z;
+            v[u].w += x[u].w;
+          }
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (i0 + u * stride < quads) reinterpret_cast<float4*>(out)[i0 + u * stride] = v[u];
+    }
+  }
+  for (int64_t i = done + first; i < n; i += stride) {
+    float v = 0.f;
+    for (int k = 0; k < n_nodes; ++k) v += from[k][i];
+    out[i] = v;
+  }
+}
+
 // Sum of the node runs of a broadband flash and the mask and range check of
 // the sum (transport.py:1088-1164). Grid-stride over the spectrum and bins
 // (node order fixed: identical results alone or in a batch), then one thread
 // per pair: charge, the absorption-only estimate over the nodes, flags.
-__global__ void flash_combine_kernel(lh_flash_problem p, lh_flash_nodes nd, lh_flash_batch b) {
+__global__ void __launch_bounds__(256)
+flash_combine_kernel(const __grid_constant__ lh_flash_problem p,
+                     const __grid_constant__ lh_flash_nodes nd,
+                     const __grid_constant__ lh_flash_batch b) {
   const int64_t n_pairs = (int64_t)flash_count(b) * p.n_om;
   const int nb = p.n_edges - 1;
   const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t n_spec = n_pairs * p.n_omega * 6;  // floats
-  for (int64_t i = first; i < n_spec; i += stride) {
-    float v = 0.f;
-    for (int n = 0; n < nd.n_nodes; ++n) v += nd.spectrum[n][i];
-    b.spectrum[i] = v;
-  }
-  const int64_t n_comp = n_pairs * 3 * nb;
-  for (int64_t i = first; i < n_comp; i += stride) {
-    float v = 0.f;
-    for (int n = 0; n < nd.n_nodes; ++n) v += nd.components[n][i];
-    b.components[i] = v;
-  }
+  flash_sum_nodes(nd.spectrum, nd.n_nodes, b.spectrum, n_pairs * p.n_omega * 6, first, stride);
+  flash_sum_nodes(nd.components, nd.n_nodes, b.components, n_pairs * 3 * nb, first, stride);
   for (int64_t pair = first; pair < n_pairs; pair += stride) {
     double q[3] = {0.0, 0.0, 0.0};
     for (int n = 0; n < nd.n_nodes; ++n)
@@ -562,9 +702,19 @@ __global__ void flash_combine_kernel(lh_flash_problem p, lh_flash_nodes nd, lh_f
   }
 }
 
-size_t flash_tc_smem_bytes(int kpad, int n_tile) {
+size_t flash_tc_smem_bytes(int kpad, int n_tile, bool sorted) {
   return 2ull * (kpad / 8) * kAChunk * 2 + 2ull * n_tile * kpad * 2 +
-         2 * sizeof(FlashPair) * kFlashPairs + 64;
+         2 * sizeof(FlashPair) * kFlashPairs + 64 +
+         (sorted ? 2 * sizeof(uint16_t) * kFlashSort + sizeof(int) * kFlashMaxBuckets : 0);
+}
+
+// The instance that holds `degrees` acceptance degrees in registers.
+FlashTcKernel flash_tc_kernel_of(int degrees) {
+  switch (degrees) {
+    case 2: return flash_tc_kernel<2>;
+    case 3: return flash_tc_kernel<3>;
+    default: return flash_tc_kernel<0>;
+  }
 }
 
 }  // namespace lh

@@ -110,3 +110,44 @@ def test_flash_against_oracle_fresh_positions(transports, flash_table):
         for o in (1, 2):
             assert (np.abs(c[:, :, o] - r["components_pe"][:, :, o]).max()
                     <= 1e-4 * np.abs(r["components_pe"][:, :, o]).max())
+
+
+@pytest.mark.parametrize("acceptance, count", [
+    (lambda x: .5 + .5 * np.asarray(x), 4),                                  # 2 degrees, 2 pairs per block
+    (lambda x: .45 + .45 * np.asarray(x) + .10 * np.asarray(x) ** 2, 200),   # 3 degrees, a tile and a pair
+    (lambda x: (.5 + .5 * np.asarray(x)) ** 3, 197),                         # 4 degrees: the general loop
+    (lambda x: .45 + .45 * np.asarray(x) + .10 * np.asarray(x) ** 2, 6400)], # two sorts per block
+    ids=["linear-4", "quadratic-200", "cubic-197", "quadratic-6400"])
+def test_flash_degrees_and_shares_match_the_oracle(flash_table, flash_config, acceptance, count):
+    """Coefficients held for 2 and 3 acceptance degrees and read per pair for 4;
+    shares of a block around a tile of 64 pairs and above one sort of 2048: flashes
+    against the oracle (the tolerances of the fixture tests), and bit for bit against
+    the same flash alone."""
+    from dataclasses import replace
+    from lighthit_b200.flash import FlashTransport
+    from lighthit_b200.model import acceptance_coefficients, synthetic_detector
+    from lighthit_b200.workloads import flash_positions
+    from oracle.flash import transport_flash
+    g = np.load(TABLES.parent.parent / "tests" / "golden" / "flash_c1.npz")
+    table = dict(np.load(TABLES / "flash_450nm_2-250m.npz"))
+    ft = FlashTransport(replace(synthetic_detector(), angular_acceptance=acceptance),
+                        flash_config, flash_table, mode="split-bf16")
+    centre = g["om_positions_m"].mean(axis=0)
+    pos = flash_positions(count, centre, seed=count, om_positions=g["om_positions_m"])
+    out = {k: v[[0, count // 2, count - 1]].cpu().numpy() for k, v in ft.run(pos, 1e10).items()
+           if k in ("spectrum", "components", "charge", "origin", "active")}
+    detector = dict(oracle_detector(g), acceptance=acceptance,
+                    alpha=acceptance_coefficients(acceptance, flash_table.degree))
+    for k, i in enumerate((0, count // 2, count - 1)):
+        alone = ft.run(pos[i:i + 1], 1e10)
+        for key, value in out.items():
+            assert np.array_equal(alone[key][0].cpu().numpy(), value[k]), (key, i)
+        r = transport_flash(table, detector, dict(position_m=pos[i], photons=1e10, time_ns=0.0),
+                            oracle_config(g))
+        q, c = r["charge_components_pe"].sum(axis=1), r["components_pe"]
+        assert np.all(np.abs(out["charge"][k].sum(axis=1) - q)
+                      <= CHARGE_RTOL * np.abs(q) + 1e-6 * np.abs(q).max())
+        got = out["components"][k].transpose(0, 2, 1)
+        for o in (1, 2):
+            assert (np.abs(got[:, :, o] - c[:, :, o]).max()
+                    <= BINS_TOL["split-bf16"] * np.abs(c[:, :, o]).max())
