@@ -25,9 +25,9 @@
 //       + (E0 - along sin(th) 2 sin^2(phi/2))^2,
 // E0 = along sin(th) - rho cos(th) formed in float64.
 //
-// Launch: a candidate pass (one thread per (OM, element), warp-aggregated
-// counts per (event, OM)), a scan into per-(event, OM) pair segments and a
-// list of pair chunks (up to 32 pairs), a second candidate pass listing the pairs, then a
+// Launch: a candidate pass (a warp per 32 elements and range of OMs, counts per
+// (event, OM)), a scan into per-(event, OM) pair segments and a
+// list of pair chunks (up to 16 pairs), a pass listing the pairs, then a
 // persistent grid over the chunks: warp 0 forms each pair's frame, the CTA
 // lists the (pair, panel, piece) work, spreads (piece x wavelength node) over
 // its threads, accumulates bins in shared memory and the charge by a block
@@ -39,13 +39,14 @@
 
 namespace lh {
 
-constexpr int kO0Chunk = 32;  // most pairs per chunk
+constexpr int kO0Chunk = 16;  // most pairs per chunk
 // Pairs per chunk: as many as still give this many chunks (16 per SM), 1 to
 // kO0Chunk. A pair's cost varies by orders of magnitude (an OM near the track
 // has its arrivals cut at many bin edges), so chunks of 32 left one shower of
 // 2000 elements x 48 OMs on a few SMs: 2.95 ms against 0.35 ms with this rule;
 // eight showers of 500-50000 elements x 384 OMs: 2.38 against 1.72 ms (1.91 ms
-// with 8 or 64 chunks per SM: too uneven, too many chunk starts).
+// with 8 or 64 chunks per SM: too uneven, too many chunk starts). At most 16, as
+// the last chunks decide when the launch ends: 1.07 against 1.10 ms with 32.
 constexpr int kO0ChunkTarget = 16 * 148;
 constexpr int kO0Threads = 256;
 constexpr int kO0MaxOrder = 64;
@@ -96,24 +97,40 @@ LH_DEVICE bool o0_support(double z, double rho, double length, double beta, doub
   return true;
 }
 
-// _ballistic_interval_numba.py:226-251 (_cone_can_reach_sphere)
-LH_DEVICE bool o0_cone_reaches(double z, double rho, double length, double beta, double radius,
-                               double pmin, double pmax) {
-  if (z <= -radius || beta * pmax <= 1.0) return false;
-  double c_hi = 1.0 / (beta * pmax);
-  double t = (1.0 - c_hi) * (1.0 + c_hi);
-  double s_hi = sqrt(t > 0.0 ? t : 0.0);
-  double c_lo = 1.0 / (beta * pmin);
-  if (c_lo > 1.0) c_lo = 1.0;
-  t = (1.0 - c_lo) * (1.0 + c_lo);
-  double s_lo = sqrt(t > 0.0 ? t : 0.0);
-  double q_hi = rho * c_hi - z * s_hi;
-  double other = rho * c_lo - z * s_lo;
-  double minimum = z >= 0.0 ? q_hi : (q_hi < other ? q_hi : other);
-  double rounding = 16 * 2.220446049250313e-16 * (fabs(z) + rho + length + radius);
+// What the candidate test of one element needs at every OM.
+struct O0Cone {
+  double ux, uy, uz, sx, sy, sz;  // direction, start
+  double length, beta;
+  double c_hi, s_hi, c_lo, s_lo;  // cone angles at the ends of the phase range
+  bool lit;                       // radiates somewhere in the range
+};
+
+LH_DEVICE O0Cone o0_cone(const lh_order0_batch& B, int64_t i, double pmin, double pmax) {
+  O0Cone c;
+  c.beta = B.beta[i];
+  c.length = B.length[i];
+  c.ux = B.direction[3 * i]; c.uy = B.direction[3 * i + 1]; c.uz = B.direction[3 * i + 2];
+  c.sx = B.start[3 * i]; c.sy = B.start[3 * i + 1]; c.sz = B.start[3 * i + 2];
+  c.lit = !(B.c0[i] == 0.0 || c.beta * pmax <= 1.0);
+  c.c_hi = 1.0 / (c.beta * pmax);
+  double t = (1.0 - c.c_hi) * (1.0 + c.c_hi);
+  c.s_hi = sqrt(t > 0.0 ? t : 0.0);
+  c.c_lo = 1.0 / (c.beta * pmin);
+  if (c.c_lo > 1.0) c.c_lo = 1.0;
+  t = (1.0 - c.c_lo) * (1.0 + c.c_lo);
+  c.s_lo = sqrt(t > 0.0 ? t : 0.0);
+  return c;
+}
+
+// _ballistic_interval_numba.py:226-251 (_cone_can_reach_sphere), z > -radius
+LH_DEVICE bool o0_cone_reaches(const O0Cone& c, double z, double rho, double radius) {
+  const double q_hi = rho * c.c_hi - z * c.s_hi;
+  const double other = rho * c.c_lo - z * c.s_lo;
+  const double minimum = z >= 0.0 ? q_hi : (q_hi < other ? q_hi : other);
+  const double rounding = 16 * 2.220446049250313e-16 * (fabs(z) + rho + c.length + radius);
   if (minimum > radius + rounding) return false;
-  double end_z = z - length;
-  if (end_z >= 0.0 && rho * c_lo - end_z * s_lo < -radius - rounding) return false;
+  const double end_z = z - c.length;
+  if (end_z >= 0.0 && rho * c.c_lo - end_z * c.s_lo < -radius - rounding) return false;
   return true;
 }
 
@@ -187,7 +204,14 @@ LH_DEVICE float o0_acceptance(const float* alpha, int n_alpha, float x, float al
   float result = alpha[0] * inv4pi;
   float previous = 1.0f, current = x;
   if (n_alpha > 1) result += 3.0f * alpha[1] * current * inv4pi;
-  for (int ell = 2; ell < n_alpha; ++ell) {
+  if (n_alpha > 2) {  // the usual degree: its factors are constants, not conversions
+    float value = (3 * x * current - previous) * (1.0f / 2);
+    result += 5 * alpha[2] * value * inv4pi;
+    previous = current;
+    current = value;
+  }
+#pragma unroll 1
+  for (int ell = 3; ell < n_alpha; ++ell) {
     float value = ((2 * ell - 1) * x * current - (ell - 1) * previous) * (1.0f / ell);
     result += (2 * ell + 1) * alpha[ell] * value * inv4pi;
     previous = current;
@@ -203,32 +227,25 @@ LH_DEVICE float o0_acceptance(const float* alpha, int n_alpha, float x, float al
 
 
 // interval_candidates (_ballistic_interval_numba.py:449-519) with the sphere
-// always in reach and the axis included: does element i light OM om at all?
-LH_DEVICE bool o0_is_candidate(const lh_order0_optics& O, const lh_order0_batch& B, int om,
-                               int64_t i, double pmin, double pmax, uint32_t& flags) {
+// always in reach and the axis included: does the element light OM om at all?
+// 0: no, 1: yes, 2: if o0_support(z, rho) says so.
+LH_DEVICE int o0_candidate(const lh_order0_optics& O, int om, const O0Cone& c, double& z,
+                           double& rho, uint32_t& flags) {
   const double radius = O.om_radius[om];
-  const double beta = B.beta[i], len = B.length[i];
-  const double ux = B.direction[3 * i], uy = B.direction[3 * i + 1], uz = B.direction[3 * i + 2];
-  const double wx = O.om_pos[3 * om] - B.start[3 * i], wy = O.om_pos[3 * om + 1] - B.start[3 * i + 1],
-               wz = O.om_pos[3 * om + 2] - B.start[3 * i + 2];
-  const double z = wx * ux + wy * uy + wz * uz;
+  const double wx = O.om_pos[3 * om] - c.sx, wy = O.om_pos[3 * om + 1] - c.sy,
+               wz = O.om_pos[3 * om + 2] - c.sz;
+  z = wx * c.ux + wy * c.uy + wz * c.uz;
   const bool sphere = radius > 0.0;
-  if (B.c0[i] == 0.0 || beta * pmax <= 1.0 || (z <= 0.0 && (!sphere || z <= -radius))) return false;
-  const double cx = wy * uz - wz * uy, cy = wz * ux - wx * uz, cz = wx * uy - wy * ux;
-  const double rho_c = sqrt(cx * cx + cy * cy + cz * cz);
-  const double rad = sphere ? radius : 0.0;
-  if (z <= 0.0 && rad == 0.0) return false;
-  if (rho_c == 0.0) {
-    if (rad == 0.0) {
-      if (0.0 < z && z < len) flags |= LH_STATUS_ON_TRACK;
-      return false;
-    }
-    return true;
+  if (!c.lit || (z <= 0.0 && (!sphere || z <= -radius))) return 0;
+  const double cx = wy * c.uz - wz * c.uy, cy = wz * c.ux - wx * c.uz, cz = wx * c.uy - wy * c.ux;
+  rho = sqrt(cx * cx + cy * cy + cz * cz);
+  if (rho == 0.0) {
+    if (sphere) return 1;
+    if (0.0 < z && z < c.length) flags |= LH_STATUS_ON_TRACK;
+    return 0;
   }
-  if (rad == 0.0) return false;  // a point receiver has no first-entry window: no light here
-  if (!o0_cone_reaches(z, rho_c, len, beta, rad, pmin, pmax)) return false;
-  double a, b, c, d;
-  return o0_support(z, rho_c, len, beta, rad, a, b, c, d) && !(a > pmax || b <= pmin);
+  // a point receiver has no first-entry window: no light here
+  return sphere && o0_cone_reaches(c, z, rho, radius) ? 2 : 0;
 }
 
 LH_DEVICE void o0_phase_range(const lh_order0_optics& O, double& pmin, double& pmax) {
@@ -255,52 +272,158 @@ struct O0Work {
   int32_t* cursor;    // [n_events * n_om]
   int32_t* pairs;     // [pair capacity] global element index
   int2* chunks;       // [chunk capacity] (event * n_om + om, chunk)
-  uint32_t* mask;     // [pair capacity / 32] candidate bits of the counting pass
+  uint32_t* mask;     // [n_om][el_words] candidate bits of the counting pass
   int32_t* n_chunks;  // [3]: the chunk count, the next chunk to take, the pairs per chunk
   int64_t pair_capacity, chunk_capacity;
+  int64_t el_words;   // words of 32 elements
 };
 
-// Candidate pairs counted (fill = false) or listed (fill = true) per (event, OM):
-// one thread per (OM, element); a warp's elements are consecutive, so the
-// lanes of one (event, OM) add their count once (warp-aggregated atomics). The
-// counting pass keeps each warp's candidate mask, which the listing pass reads
-// instead of testing the pair again.
-template <bool fill>
-__global__ void order0_candidates_kernel(const lh_order0_optics O, const lh_order0_batch B,
-                                         O0Work W) {
-  double pmin, pmax;
-  o0_phase_range(O, pmin, pmax);
-  const int64_t n_el = B.n_elements;
-  const int64_t total = n_el * O.n_om;
+constexpr int kO0CountWarps = 8;
+
+// The candidates among a word's bits that belong to the event of its lowest one.
+LH_DEVICE uint32_t o0_word_of_event(const lh_order0_batch& B, uint32_t bits, int64_t base,
+                                    int& ev) {
+  ev = o0_event_of(B, base + __ffs(bits) - 1);
+  const int64_t rest = (ev + 1 < B.n_events ? B.element_offset[ev + 1] : B.n_elements) - base;
+  return rest < 32 ? bits & ((1u << rest) - 1u) : bits;
+}
+
+// Candidate pairs counted per (event, OM). A warp takes 32 consecutive elements
+// and a range of up to 32 OMs: each lane keeps its element's geometry in registers.
+// What bounds it is float64 arithmetic, most of it the support window (inverse
+// trigonometry) of the few pairs that the cone test leaves: they wait in a queue
+// until a full warp of them can be tested. With one thread per (OM, element), which
+// read the element and formed its cone again at every OM and tested the window on
+// single lanes, 151000 elements x 384 OMs took 0.383 ms (0.147
+// now).
+__global__ void __launch_bounds__(32 * kO0CountWarps, 3)
+order0_count_kernel(const lh_order0_optics O, const lh_order0_batch B, O0Work W,
+                    int oms_per_warp) {
+  __shared__ uint32_t s_word[kO0CountWarps][32];
+  __shared__ double2 s_zr[kO0CountWarps][64];
+  __shared__ int s_code[kO0CountWarps][64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double pmin = INFINITY, pmax = -INFINITY;
+  for (int k = lane; k < O.n_panel_edges; k += 32) {
+    pmin = fmin(pmin, O.phase[k]);
+    pmax = fmax(pmax, O.phase[k]);
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    pmin = fmin(pmin, __shfl_xor_sync(0xffffffffu, pmin, off));
+    pmax = fmax(pmax, __shfl_xor_sync(0xffffffffu, pmax, off));
+  }
+  const int64_t unit = (int64_t)blockIdx.x * kO0CountWarps + warp;
+  const int64_t range = unit / W.el_words, column = unit - range * W.el_words;
+  const int64_t first = range * oms_per_warp;
+  if (first >= O.n_om) return;
+  const int n_oms = (int)min((int64_t)oms_per_warp, O.n_om - first);
+  const int64_t i = 32 * column + lane;
+  const bool exists = i < B.n_elements;
+  const O0Cone cone = o0_cone(B, exists ? i : B.n_elements - 1, pmin, pmax);
+  // The cone test in float32, positions relative to the first OM. Its distances are
+  // off by less than 32 float32 roundings of the sum of all components, lengths and
+  // radii in them; a pair is refused here only where it misses by more than twice
+  // that (NaN and overflow refuse nothing).
+  const double ox = O.om_pos[0], oy = O.om_pos[1], oz = O.om_pos[2];
+  const float sx = (float)(cone.sx - ox), sy = (float)(cone.sy - oy), sz = (float)(cone.sz - oz);
+  const float ux = (float)cone.ux, uy = (float)cone.uy, uz = (float)cone.uz;
+  const float c_hi = (float)cone.c_hi, s_hi = (float)cone.s_hi, c_lo = (float)cone.c_lo,
+              s_lo = (float)cone.s_lo, length = (float)cone.length;
+  const float margin = 64.f * 5.97e-8f * fmaxf(1.f, fabsf(ux) + fabsf(uy) + fabsf(uz));
+  const float reach = fabsf(sx) + fabsf(sy) + fabsf(sz) + length;
+  float px = 0.f, py = 0.f, pz = 0.f, pr = 0.f;  // lane k: OM first + k
+  if (lane < n_oms) {
+    const int64_t om = first + lane;
+    px = (float)(O.om_pos[3 * om] - ox);
+    py = (float)(O.om_pos[3 * om + 1] - oy);
+    pz = (float)(O.om_pos[3 * om + 2] - oz);
+    pr = (float)O.om_radius[om];
+  }
+  uint32_t* word = s_word[warp];
+  word[lane] = 0;
+  __syncwarp();
+  double2* zr = s_zr[warp];
+  int* code = s_code[warp];
   uint32_t flags = 0;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < total;
-       base += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t item = base + threadIdx.x;
-    const int64_t word = item >> 5;  // blockDim and base are multiples of 32
-    bool keep = false;
-    int key = -1;
-    int64_t i = 0;
-    if (item < total) {
-      const int om = (int)(item / n_el);
-      i = item - (int64_t)om * n_el;
-      keep = fill ? ((W.mask[word] >> (threadIdx.x & 31)) & 1u)
-                  : o0_is_candidate(O, B, om, i, pmin, pmax, flags);
-      if (keep) key = o0_event_of(B, i) * O.n_om + om;
+  int waiting = 0;  // entries in the queue, below 32 between OMs
+  auto test = [&](int at, int count) {
+    const int entry = lane < count ? code[at + lane] : 0;
+    const double2 v = lane < count ? zr[at + lane] : make_double2(1.0, 1.0);
+    const double length = __shfl_sync(0xffffffffu, cone.length, entry & 31);
+    const double beta = __shfl_sync(0xffffffffu, cone.beta, entry & 31);
+    double lo, hi, inner0, inner1;
+    if (lane < count &&
+        o0_support(v.x, v.y, length, beta, O.om_radius[first + (entry >> 5)], lo, hi, inner0,
+                   inner1) &&
+        !(lo > pmax || hi <= pmin))
+      atomicOr(&word[entry >> 5], 1u << (entry & 31));
+    __syncwarp();
+  };
+  for (int k = 0; k < n_oms; ++k) {
+    const float ax = __shfl_sync(0xffffffffu, px, k), ay = __shfl_sync(0xffffffffu, py, k),
+                az = __shfl_sync(0xffffffffu, pz, k), radius = __shfl_sync(0xffffffffu, pr, k);
+    const float wx = ax - sx, wy = ay - sy, wz = az - sz;
+    const float far =
+        radius + (margin * (fabsf(ax) + fabsf(ay) + fabsf(az) + radius + reach) + 1e-15f);
+    const float zf = wx * ux + wy * uy + wz * uz;
+    const float cx = wy * uz - wz * uy, cy = wz * ux - wx * uz, cz = wx * uy - wy * ux;
+    const float rf = sqrtf(cx * cx + cy * cy + cz * cz);
+    const float q_hi = rf * c_hi - zf * s_hi, q_lo = rf * c_lo - zf * s_lo;
+    const bool misses =
+        zf < -far || (q_hi > far && q_lo > far) || q_lo + length * s_lo < -far;
+    const bool open_pair = exists && !(misses && rf < INFINITY);
+    if (!__any_sync(0xffffffffu, open_pair)) continue;
+    double z = 0.0, rho = 0.0;
+    const int state = open_pair ? o0_candidate(O, (int)first + k, cone, z, rho, flags) : 0;
+    const unsigned lit = __ballot_sync(0xffffffffu, state == 1);
+    const unsigned open = __ballot_sync(0xffffffffu, state == 2);
+    if (lane == 0 && lit) atomicOr(&word[k], lit);
+    if (state == 2) {
+      const int at = waiting + __popc(open & ((1u << lane) - 1u));
+      zr[at] = make_double2(z, rho);
+      code[at] = lane | (k << 5);
     }
-    const unsigned active = __ballot_sync(0xffffffffu, keep);
-    if (!fill && (threadIdx.x & 31) == 0 && item < total) W.mask[word] = active;
-    if (keep) {
-      const unsigned peers = __match_any_sync(active, key);
-      const int leader = __ffs(peers) - 1;
-      const int lane = threadIdx.x & 31;
-      const int rank = __popc(peers & ((1u << lane) - 1u));
-      int first = 0;
-      if (lane == leader) first = atomicAdd(fill ? W.cursor + key : W.counts + key, __popc(peers));
-      first = __shfl_sync(peers, first, leader);
-      if (fill && first + rank < W.pair_capacity) W.pairs[first + rank] = (int32_t)i;
+    waiting += __popc(open);
+    __syncwarp();
+    if (waiting >= 32) {
+      waiting -= 32;
+      test(waiting, 32);
     }
   }
-  if (!fill && flags) atomicOr(reinterpret_cast<unsigned*>(B.status), flags);
+  test(0, waiting);
+  if (lane < n_oms) {
+    const int64_t om = first + lane;
+    uint32_t bits = word[lane];
+    W.mask[om * W.el_words + column] = bits;
+    while (bits) {
+      int ev;
+      const uint32_t mine = o0_word_of_event(B, bits, 32 * column, ev);
+      atomicAdd(W.counts + (int64_t)ev * O.n_om + om, __popc(mine));
+      bits ^= mine;
+    }
+  }
+  if (flags) atomicOr(reinterpret_cast<unsigned*>(B.status), flags);
+}
+
+// Lists the candidates: one thread per word of the mask, most of which are empty
+// (0.100 ms
+// with one thread per pair, 0.006 now).
+__global__ void __launch_bounds__(256)
+order0_list_kernel(const lh_order0_optics O, const lh_order0_batch B, O0Work W) {
+  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (item >= W.el_words * O.n_om) return;
+  uint32_t bits = W.mask[item];
+  if (!bits) return;
+  const int om = (int)(item / W.el_words);
+  const int64_t base = 32 * (item - om * W.el_words);
+  while (bits) {  // the candidates of one event at a time
+    int ev;
+    const uint32_t mine = o0_word_of_event(B, bits, base, ev);
+    int32_t at = atomicAdd(W.cursor + (int64_t)ev * O.n_om + om, __popc(mine));
+    for (uint32_t m = mine; m; m &= m - 1, ++at)
+      if (at < W.pair_capacity) W.pairs[at] = (int32_t)(base + __ffs(m) - 1);
+    bits ^= mine;
+  }
 }
 
 // Single CTA: pair offsets per (event, OM), the chunk size and the chunk list.
@@ -379,6 +502,7 @@ __global__ void __launch_bounds__(1024) order0_scan_kernel(int32_t n_keys, O0Wor
 struct O0Rule {
   double x[kO0MaxOrder], w[kO0MaxOrder];
   double sin_psi[kO0MaxOrder], cos_psi[kO0MaxOrder];
+  float2 xw[kO0MaxOrder];  // x, w of the float32 azimuth rule
 };
 
 // A (piece, wavelength node) item as its s-nodes read it.
@@ -432,6 +556,12 @@ LH_DEVICE int o0_block_scan(int v, int& total, int* warp_sums) {
   return inclusive - v + (warp ? warp_sums[warp - 1] : 0);
 }
 
+// What bounds it is the instructions issued (62 % of the slots, the tensor cores have
+// nothing to do, memory is idle): the float32 azimuth nodes and the float64 set-up of
+// each s-node. Constants of the azimuth rule and of the acceptance that were converted
+// from float64 and int at every node, and cuts kept in local memory, took 1.41 ms for
+// 151000 elements x 384 OMs against 1.10 without, 0.226 against 0.183 ms for 2000 x 48.
+// 128 threads (1.43 ms) balance a chunk worse, 80 registers (1.14) hide less.
 __global__ void __launch_bounds__(kO0Threads, 4)
 order0_kernel(const lh_order0_optics O, const lh_order0_batch B, const O0Work W,
               unsigned long long* units) {
@@ -450,11 +580,13 @@ order0_kernel(const lh_order0_optics O, const lh_order0_batch B, const O0Work W,
   for (int k = tid; k < order; k += blockDim.x) {
     S.rule[0].x[k] = O.gauss_x[k];
     S.rule[0].w[k] = O.gauss_w[k];
+    S.rule[0].xw[k] = make_float2((float)O.gauss_x[k], (float)O.gauss_w[k]);
     sincospi(0.5 * O.gauss_x[k], &S.rule[0].sin_psi[k], &S.rule[0].cos_psi[k]);
   }
   for (int k = tid; k < check; k += blockDim.x) {
     S.rule[1].x[k] = O.check_x[k];
     S.rule[1].w[k] = O.check_w[k];
+    S.rule[1].xw[k] = make_float2((float)O.check_x[k], (float)O.check_w[k]);
     sincospi(0.5 * O.check_x[k], &S.rule[1].sin_psi[k], &S.rule[1].cos_psi[k]);
   }
   for (int k = tid; k < O.n_alpha; k += blockDim.x) S.alpha[k] = (float)O.alpha[k];
@@ -591,7 +723,6 @@ order0_kernel(const lh_order0_optics O, const lh_order0_batch B, const O0Work W,
   bool bad_acceptance = false;
   double charge = 0.0, charge_check = 0.0;
   double scuts[kO0MaxSCuts];
-  double phicuts[kO0MaxPhiCuts];
 
   // main-rule items first, then the check rule's: a warp's items share a rule
   const int main_items = n_combos * order;
@@ -749,25 +880,15 @@ order0_kernel(const lh_order0_optics O, const lh_order0_batch B, const O0Work W,
       const double emission = t0 + tau * s - origin;
       const double tmin = emission + o0_entry(Bq, cosine * along + sine * rho) / velocity;
       const double tmax = emission + o0_entry(Bq, cosine * along + sine * rho * cos_half) / velocity;
-      phicuts[0] = 0.0;
-      int nphi = 1;
+      int edge = 0, last_cut = 0;  // the bin edges that cut the azimuth range
       if (rho > 0.0) {
-        const int first_cut = o0_search_right(edges, n_edges, tmin);
-        const int last_cut = o0_search_left(edges, n_edges, tmax);
-        for (int edge = first_cut; edge < last_cut; ++edge) {
-          const double distance = (edges[edge] - emission) * velocity;
-          const double dot = (Bq + distance * distance) / (2 * distance);
-          const double phi = acos(o0_clamp1((dot - cosine * along) / (sine * rho)));
-          const double r = phi / half;
-          if (nphi < kO0MaxPhiCuts - 1) phicuts[nphi] = asin(r < 1.0 ? r : 1.0);
-          ++nphi;
-        }
+        edge = o0_search_right(edges, n_edges, tmin);
+        last_cut = o0_search_left(edges, n_edges, tmax);
       }
-      if (nphi > kO0MaxPhiCuts - 1) {
+      if (last_cut - edge > kO0MaxPhiCuts - 2) {
         flags |= LH_STATUS_OVERFLOW;
         continue;
       }
-      phicuts[nphi++] = kPi / 2;
       // float32 azimuth integrand, entry distance without cancellation
       const float half_f = (float)half;
       const float W2_f = (float)W2, B_f = (float)Bq;
@@ -775,8 +896,19 @@ order0_kernel(const lh_order0_optics O, const lh_order0_batch B, const O0Work W,
       const float Sa = (float)(along * sine);
       const float along_cos = (float)(cosine * along), rho_sin = (float)(sine * rho);
       const float sin2W2 = sin_f * sin_f * W2_f;
-      for (int pp = 0; pp < nphi - 1; ++pp) {
-        const double pa = phicuts[pp], pb = phicuts[pp + 1];
+      double pb = 0.0;
+      for (bool more = true; more; ++edge) {  // piece by piece, cut by cut
+        const double pa = pb;
+        more = edge < last_cut;
+        if (more) {
+          const double distance = (edges[edge] - emission) * velocity;
+          const double dot = (Bq + distance * distance) / (2 * distance);
+          const double phi = acos(o0_clamp1((dot - cosine * along) / (sine * rho)));
+          const double r = phi / half;
+          pb = asin(r < 1.0 ? r : 1.0);
+        } else {
+          pb = kPi / 2;
+        }
         if (pa >= pb) continue;
         const float mid = (float)((pa + pb) / 2), hw = (float)((pb - pa) / 2);
         evaluations += ord;
@@ -785,9 +917,10 @@ order0_kernel(const lh_order0_optics O, const lh_order0_batch B, const O0Work W,
           // arguments lie in [0, pi]: the hardware approximations (absolute error
           // near 2^-21) are well inside the float32 integrand's budget
           float s_eta, c_eta;
-          __sincosf(mid + hw * (float)R.x[jp], &s_eta, &c_eta);
+          const float2 xw = R.xw[jp];
+          __sincosf(mid + hw * xw.x, &s_eta, &c_eta);
           const float phi = half_f * s_eta;
-          const float dphi = half_f * c_eta * hw * (float)R.w[jp];
+          const float dphi = half_f * c_eta * hw * xw.y;
           // sin(phi), cos(phi) from the half angle: 2 sin^2(phi/2) = 1 - cos(phi)
           // without cancellation near phi = 0
           float sh, chh;
@@ -903,7 +1036,8 @@ static O0Work o0_layout(const lh_order0_optics& O, const lh_order0_batch& B, uns
   W.cursor = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * keys));
   W.pairs = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * W.pair_capacity));
   W.chunks = reinterpret_cast<int2*>(take(sizeof(int2) * W.chunk_capacity));
-  W.mask = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * ((W.pair_capacity + 31) / 32)));
+  W.el_words = (B.n_elements + 31) / 32;
+  W.mask = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * W.el_words * O.n_om));
   W.n_chunks = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * 4));
   if (bytes) *bytes = off;
   return W;
@@ -925,11 +1059,14 @@ int order0_launch(const lh_order0_optics& O, const lh_order0_batch& B, cudaStrea
   if (B.bins) cudaMemsetAsync(B.bins, 0, sizeof(double) * (size_t)keys * (B.n_edges - 1), s);
   if (B.n_elements == 0) return cudaGetLastError() == cudaSuccess ? LH_OK : LH_ECUDA;
   cudaMemsetAsync(W.counts, 0, sizeof(int32_t) * keys, s);
-  const int64_t items = B.n_elements * O.n_om;
-  const int blocks = (int)std::min<int64_t>((items + 255) / 256, 148 * 16);
-  order0_candidates_kernel<false><<<blocks, 256, 0, s>>>(O, B, W);
+  // OMs per warp of the counting pass: as many as still give 64 warps per SM
+  const int64_t words = W.el_words * O.n_om;
+  const int oms = (int)std::max<int64_t>(1, std::min<int64_t>(32, words / (148 * 64)));
+  const int64_t warps = W.el_words * ((O.n_om + oms - 1) / oms);
+  order0_count_kernel<<<(unsigned)((warps + kO0CountWarps - 1) / kO0CountWarps),
+                        32 * kO0CountWarps, 0, s>>>(O, B, W, oms);
   order0_scan_kernel<<<1, 1024, 0, s>>>((int32_t)keys, W);
-  order0_candidates_kernel<true><<<blocks, 256, 0, s>>>(O, B, W);
+  order0_list_kernel<<<(unsigned)((words + 255) / 256), 256, 0, s>>>(O, B, W);
   {
     lh::TimedLaunch timed_launch(LH_KT_ORDER0, s);
     order0_kernel<<<148 * 8, kO0Threads, smem, s>>>(

@@ -110,9 +110,9 @@ def test_batched_events_equal_alone_and_ragged():
                   g["rays8_charge"], g["rays8_bins"])
 
 
-@pytest.mark.parametrize("pairs", [1, 4735, 4736, 75776, 80000])
+@pytest.mark.parametrize("pairs", [1, 4735, 4736, 37888, 75776, 80000])
 def test_chunk_sizes(pairs):
-    """Chunks hold 1 pair below 2 x 2368 candidate pairs and 32 from 32 x 2368 on: the
+    """Chunks hold 1 pair below 2 x 2368 candidate pairs and 16 from 16 x 2368 on: the
     same events on both sides of either edge (sums in float64, so to 1e-12)."""
     from lighthit_b200.order0 import order0
     g, el = fixture()
@@ -132,6 +132,42 @@ def test_chunk_sizes(pairs):
         for k, ref in enumerate([alone] + [whole] * copies):
             ref = ref[key][0].cpu().numpy()
             assert np.abs(values[k] - ref).max() <= 1e-12 * max(ref.max(), 1e-30)
+
+
+@pytest.mark.parametrize("sizes", [(1,), (31, 1, 33), (0, 3, 29, 0, 64), (2000,) * 16 + (1337,)])
+def test_candidate_words(sizes):
+    """Candidates are kept in words of 32 elements: words shared by several events,
+    remainders, and a batch large enough for several OMs per warp (5 for 33337
+    elements x 48 OMs, the last range 3). Against the oracle where it is small, else
+    each event alone (sums in float64, so to 1e-12)."""
+    from lighthit_b200.order0 import order0
+    g, el = fixture()
+    opt = optics_of(g)
+    lit = np.argsort(-np.bincount(g["pair_element"], minlength=len(el["beta"])), kind="stable")
+    events = [{k: v[np.sort(lit[:n])] for k, v in el.items()} for n in sizes]
+    out = order0(opt, events, np.repeat(g["origins_ns"][None], len(events), axis=0),
+                 g["edges_ns"])
+    charge, bins = out["charge"].cpu().numpy(), out["bins"].cpu().numpy()
+    det, optics = oracle_args(g)
+    done = {}
+    for k, (n, ev) in enumerate(zip(sizes, events)):
+        if n == 0:
+            assert not charge[k].any() and not bins[k].any()
+            continue
+        if n not in done:
+            if n < 100:
+                po, pe = oracle.candidates(g["positions_m"], g["radii_m"], ev["start_m"],
+                                           ev["direction"], ev["length_m"], ev["coefficient0"],
+                                           ev["beta"], g["phase_nodes"])
+                done[n] = oracle.rays(po, pe, det, ev, optics, g["origins_ns"], g["edges_ns"], 8)
+            else:
+                alone = order0(opt, [ev], g["origins_ns"][None], g["edges_ns"])
+                done[n] = [alone[key][0].cpu().numpy() for key in ("charge", "bins")]
+        if n < 100:
+            check_against(charge[k], bins[k], *done[n])
+        else:
+            for got, ref in zip((charge[k], bins[k]), done[n]):
+                assert np.abs(got - ref).max() <= 1e-12 * ref.max()
 
 
 def test_fine_bins_and_shifted_clock_vs_oracle():
