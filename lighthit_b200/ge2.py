@@ -182,7 +182,8 @@ class Ge2Table:
         return res.cpu().numpy().T
 
     def _prepare(self, sources, positions, looks, out_scale, window, zero_frequency):
-        """Host geometry in the axis frame and the device channels of one problem."""
+        """Host geometry in the axis frame and the channels of one problem: on the
+        device, or a host array that travels with the geometry."""
         import torch
         dev = self.device
         positions = np.atleast_2d(np.asarray(positions, float))
@@ -213,18 +214,21 @@ class Ge2Table:
         reference = float(ref.min())
         ch = sources.channels
         if not isinstance(ch, torch.Tensor):
-            ch = torch.from_numpy(np.ascontiguousarray(np.asarray(ch), dtype=np.complex64))
-        ch = ch.to(dev, torch.complex64)
-        if zero_frequency:
-            ch = ch[..., :1]
+            ch = np.ascontiguousarray(np.asarray(ch), dtype=np.complex64)
+        else:
+            ch = ch.to(dev, torch.complex64)
         if ch.shape[0] != self.n_bands or ch.shape[2] != self.nch or ch.shape[3] < W:
             raise ValueError("source channels do not match the folded kernels")
         shift = ref - reference
         if np.any(shift != 0):  # align every band to the earliest emission reference
+            if not isinstance(ch, torch.Tensor):
+                ch = _lib.upload(ch, torch.complex64, dev)
+            ch = ch[..., :W]
             ph = _lib.upload(np.exp(1j * np.outer(shift, self.omega[:ch.shape[3]])),
                              torch.complex64, dev)
             ch = ch * ph[:, None, None, :]
-        ch = torch.view_as_real(ch.contiguous()).contiguous()
+        if isinstance(ch, torch.Tensor):
+            ch = ch.resolve_conj().contiguous()  # a zero-frequency problem reads the first column
         scale = np.asarray(out_scale, float)
         if scale.ndim == 1:
             scale = np.repeat(scale[None, :], self.n_bands, axis=0)
@@ -239,7 +243,13 @@ class Ge2Table:
         for key in ("pts", "rec", "lk", "scale"):
             offs[key] = at
             at += 8 * q[key].size
-        return _lib.Ge2Problem(len(q["pts"]), offs["pts"], q["ch"].data_ptr(),
+        channels = None
+        if not isinstance(q["ch"], np.ndarray):
+            channels = q["ch"].data_ptr()
+        elif q["ch"].size:
+            channels = at + -at % 256
+            at = channels + q["ch"].nbytes
+        return _lib.Ge2Problem(len(q["pts"]), offs["pts"], channels,
                                int(q["ch"].shape[3]), q["W"], q["n_om"], offs["rec"],
                                offs["lk"], offs["scale"], q["low"], q["high"], q["reference"],
                                result_ptr), at
@@ -264,9 +274,14 @@ class Ge2Table:
         if not items:
             return []
         prepared = [self._prepare(*it, zero_frequency) for it in items]
-        host = np.concatenate([np.concatenate([q[k].ravel() for k in ("pts", "rec", "lk", "scale")])
-                               for q in prepared])
-        d_geom = _lib.upload(host, torch.float64, dev)
+        parts, words = [], 0  # in the order of _problem
+        for q in prepared:
+            parts += [q[k] for k in ("pts", "rec", "lk", "scale")]
+            words += sum(a.size for a in parts[-4:])
+            if isinstance(q["ch"], np.ndarray) and q["ch"].size:  # on a 256-byte boundary
+                parts += [np.zeros(-words % 32), q["ch"].ravel().view(np.float64)]
+                words += parts[-2].size + parts[-1].size
+        d_geom, _ = _lib.upload_parts(parts, torch.float64, dev)
         sizes = [q["n_om"] * q["W"] for q in prepared]
         result = torch.empty(max(sum(sizes), 1), dtype=torch.complex128, device=dev)
         probs = (_lib.Ge2Problem * len(prepared))()

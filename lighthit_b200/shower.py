@@ -826,7 +826,7 @@ class ShowerTransport:
                 centroid = np.stack([np.bincount(inverse, weights=share * coords[:, k],
                                                  minlength=groups) for k in range(3)], axis=1)
                 order = np.argsort(inverse, kind="stable")  # group sums in point order
-                starts = np.searchsorted(inverse[order], np.arange(groups))
+                starts = np.cumsum(count) - count  # every group has points
                 summed = np.add.reduceat(ev.zero_ch[b][order].astype(complex), starts, axis=0)
                 c_points.append(centre + centroid[:, :1] * axis + centroid[:, 1:2] * e1
                                 + centroid[:, 2:3] * e2)

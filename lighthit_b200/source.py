@@ -229,9 +229,10 @@ class SourceCompiler:
         n_slices = int(zb.max()) + 3
         dev = self.device
         if device_elements is None:
-            arrays = {k: _lib.upload(v, torch.float64, dev)
-                      for k, v in dict(start=start, direction=direction, length=length, c0=c0,
-                                       c2=c2, beta=beta, t0=t0, t1=t1).items()}
+            host = dict(start=start, direction=direction, length=length, c0=c0, c2=c2,
+                        beta=beta, t0=t0, t1=t1)
+            flat, at = _lib.upload_parts(list(host.values()), torch.float64, dev)
+            arrays = {k: flat[lo:hi] for k, lo, hi in zip(host, at, at[1:])}
         else:
             d = device_elements
             arrays = dict(start=d["start_m"], direction=d["direction"], length=d["length_m"],

@@ -151,3 +151,25 @@ def test_flash_degrees_and_shares_match_the_oracle(flash_table, flash_config, ac
         for o in (1, 2):
             assert (np.abs(got[:, :, o] - c[:, :, o]).max()
                     <= BINS_TOL["split-bf16"] * np.abs(c[:, :, o]).max())
+
+
+@pytest.mark.parametrize("count", [1, 137])
+def test_flash_run_on_a_stream_and_response_equal_the_default(transports, flash_golden, count):
+    """Inputs travel on the launching stream, and one flash's outputs in one buffer: a
+    run on another stream, a response of it and ``transport`` give the same values."""
+    import torch
+    from lighthit_b200.model import IsotropicFlash
+    from lighthit_b200.workloads import flash_positions
+    g = flash_golden
+    ft = transports["split-bf16"]
+    pos = flash_positions(count, g["om_positions_m"].mean(axis=0), seed=3,
+                          om_positions=g["om_positions_m"])
+    times = np.linspace(0.0, 40.0, count)
+    here = ft.run(pos, 1e10, times)
+    there = ft.run(pos, 1e10, times, stream=torch.cuda.Stream())
+    for key in ("spectrum", "components", "charge", "origin", "active"):
+        assert torch.equal(here[key], there[key]), key
+    a = ft.response(there, count - 1)
+    b = ft.transport(IsotropicFlash.monochromatic(pos[-1], 1e10, 450.0, time_ns=times[-1]))
+    for key in ("spectrum_pe", "components_pe", "charge_components_pe", "time_origin_ns", "active"):
+        assert np.array_equal(getattr(a, key), getattr(b, key)), key
