@@ -99,6 +99,27 @@ LH_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit_ns = kW
   return false;
 }
 
+// mbar_wait of a whole warp, with one outcome for all its lanes.
+LH_DEVICE bool warp_wait(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
+// A barrier of a group of kThreads threads in whole warps (the group's number picks
+// the barrier); true when `flag` holds on any.
+template <int kThreads>
+LH_DEVICE bool group_sync_or(int group, bool flag) {
+  int any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %2, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, %3, p;\n\t"
+      "selp.b32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(1 + group), "r"((int)flag), "n"(kThreads)
+      : "memory");
+  return any != 0;
+}
+
 // Untiled bulk copy global -> shared, completion counted on an mbarrier.
 // Both addresses 16-byte aligned, size a multiple of 16.
 LH_DEVICE void bulk_g2s(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {

@@ -26,7 +26,7 @@ namespace lh {
 constexpr int kFlashPairs = 64;  // pairs per tile -> 128 readout rows
 constexpr int kMaxAcc = 8;       // highest acceptance degree handled
 constexpr int kFlashThreads = 256;    // plain path
-constexpr int kFlashTcThreads = 512;  // fused path: 16 warps hide the table-load latency
+constexpr int kFlashTcThreads = 512;  // fused path: 11 warps of spectra, 4 of drain, 1 of MMAs
 // A tile of the fused path: K-major, no swizzle, [k/8][row][k%8] with each
 // 8-column chunk of the 128 rows padded by 16 bytes (2064 B apart, the MMA's
 // leading byte offset). A warp stores 32 consecutive columns of one row: the
@@ -47,9 +47,9 @@ struct FlashPair {
   float amp0;     // order-0 amplitude
   int j;          // log-r interval, -1 outside the table's radial range
   int bin0;       // order-0 bin, -1 outside the window
-  int valid;      // pair exists
-  int inside;
-  int flags;      // bit 1: unsafe (outside range, bound above threshold); bit 2: coincident
+  uint8_t valid;  // pair exists
+  uint8_t inside;
+  uint8_t flags;  // bit 1: unsafe (outside range, bound above threshold); bit 2: coincident
   float w[kMaxAcc + 1];  // alpha_l P_l(cos) / (4 pi)
   float charge[3];
 };
@@ -214,13 +214,12 @@ LH_DEVICE void flash_item(const lh_flash_problem& p, const lh_flash_batch& b, in
 }
 
 // Step 3 (order 0 and the mask) for the tile's pairs.
-// `threads`: the first threads of the CTA that take part (0: all).
+// The calling thread is number `index` of the `stride` (at least 64) that take part.
 LH_DEVICE void flash_tile_order0(const lh_flash_problem& p, const lh_flash_batch& b,
-                                 const FlashPair* sp, int n_bins, int threads = 0) {
-  const int stride = threads ? threads : (int)blockDim.x;
+                                 const FlashPair* sp, int n_bins, int index, int stride) {
   if ((n_bins & 3) == 0) {  // rows are 16-byte aligned: four bins per store
     const int quads = n_bins >> 2;
-    for (int i = threadIdx.x; i < kFlashPairs * quads; i += stride) {
+    for (int i = index; i < kFlashPairs * quads; i += stride) {
       const int lp = i / quads, bin = (i % quads) * 4;
       const FlashPair& s = sp[lp];
       if (!s.valid) continue;
@@ -230,15 +229,15 @@ LH_DEVICE void flash_tile_order0(const lh_flash_problem& p, const lh_flash_batch
       *reinterpret_cast<float4*>(b.components + (s.pair * 3) * n_bins + bin) = v;
     }
   } else {
-    for (int i = threadIdx.x; i < kFlashPairs * n_bins; i += stride) {
+    for (int i = index; i < kFlashPairs * n_bins; i += stride) {
       const int lp = i / n_bins, bin = i % n_bins;
       const FlashPair& s = sp[lp];
       if (!s.valid) continue;
       b.components[(s.pair * 3) * n_bins + bin] = (bin == s.bin0) ? (float)s.q0 : 0.f;
     }
   }
-  if (threadIdx.x < kFlashPairs) {
-    const FlashPair& s = sp[threadIdx.x];
+  if (index < kFlashPairs) {
+    const FlashPair& s = sp[index];
     if (s.valid) {
       const int64_t pair = s.pair;
       const double q = ((double)s.charge[0] + (double)s.charge[1]) + (double)s.charge[2];
@@ -311,28 +310,32 @@ flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins, f
     }
   }
   __syncthreads();
-  flash_tile_order0(p, b, sp, n_bins);
+  flash_tile_order0(p, b, sp, n_bins, threadIdx.x, blockDim.x);
 }
 
 // ---------------------------------------------------------------- fused tcgen05 path
 // One CTA per SM, each over its share of consecutive pairs. B (the readout
 // operator, hi and lo parts) is loaded once per CTA. The CTA sorts up to
-// kFlashSort pairs at a time by radial interval and takes them in tiles of 64: a
-// thread holds the cubic coefficients of its frequency in registers and runs over
-// neighbouring pairs, reading coefficients only where the interval changes. Per
-// tile: setup -> spectrum items writing A (bf16 hi/lo) into shared memory -> one
-// thread issues the MMAs -> order-0 rows and mask while the tensor core runs ->
-// TMEM drain. A share of few pairs (a single flash) spreads over the SMs pair by
-// pair. kDegrees: acceptance degrees whose coefficients a thread holds (0: any,
-// read for every pair; four degrees or more would not fit beside the rest in the 128
-// registers of a thread).
+// kFlashSort pairs at a time by radial interval and takes them in tiles of 64 as a
+// pipeline of warp roles: the first warps hold the cubic coefficients of their
+// frequency in registers, run over neighbouring pairs (reading coefficients only
+// where the interval changes) and write A (bf16 hi/lo) into shared memory; the last
+// warp issues the MMAs into one of two accumulators; four warps write the order-0
+// rows, drain the accumulator and set up the pairs of the tile after next, while the
+// first warps compute the next tile. They wait only for the MMAs, since A is there
+// once. A share of few pairs (a single flash) spreads over the SMs pair by pair.
+// kDegrees: acceptance degrees whose coefficients a thread holds (0: any, read for
+// every pair; four degrees or more would not fit beside the rest in the 128 registers
+// of a thread).
 //
 // What bounds it: the outputs (65 frequencies x 24 bytes and 480 bins x 4 bytes a
-// pair) take 0.1 ms for 4096 flashes of 48 OMs, the spectra another 0.19 ms that
-// nothing overlaps, since the A tile and the operator leave shared memory for one
-// tile only. With coefficients read for every pair (192 bytes a pair and frequency
-// through L1) the same launch took 0.380 ms, sorted it takes 0.345. A single flash
-// (48 pairs on one CTA before, on 48 now): 21.8 us, now 13.7.
+// pair) take 0.10 ms for 4096 flashes of 48 OMs. The launch took 0.380 ms with
+// coefficients read for every pair (192 bytes a pair and frequency through L1), 0.345
+// with pairs sorted and all warps in step, 0.304 with roles: now the spectra (11
+// warps of latency chains, 40 % of the issue slots) and the drains take about as long
+// as each other. 576 threads leave 96 registers each (0.376), eight draining warps
+// leave three groups of frequencies (0.293, but 0.166 for 3 x 501 flashes against
+// 0.148). One flash: 21.8 us on one SM, now 13.9 on 48. 137 flashes: 25.4, now 22.2.
 constexpr int kFlashSort = 2048;        // pairs sorted at a time
 constexpr int kFlashMaxBuckets = 1024;  // radial intervals the sort tells apart
 
@@ -349,115 +352,28 @@ LH_DEVICE int flash_bucket(const lh_flash_problem& p, const lh_flash_batch& b, i
   return min(max(j, 0), buckets - 1);
 }
 
+// The spectra of a chunk's tiles, written as A rows (order 1, order 2 of each pair):
+// thread (group of pairs, frequency).
 template <int kDegrees>
-__global__ void __launch_bounds__(kFlashTcThreads, 1)
-flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __restrict__ g_bhi,
-                const __nv_bfloat16* __restrict__ g_blo, int kpad, int n_bins, int n_tile,
-                int passes, int sorted) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  const uint32_t a_bytes = (uint32_t)(kpad / 8) * kAChunk * 2u;
-  const uint32_t b_bytes = (uint32_t)n_tile * kpad * 2u;
-  __nv_bfloat16* s_ahi = reinterpret_cast<__nv_bfloat16*>(smem);
-  __nv_bfloat16* s_alo = reinterpret_cast<__nv_bfloat16*>(smem + a_bytes);
-  __nv_bfloat16* s_bhi = reinterpret_cast<__nv_bfloat16*>(smem + 2 * a_bytes);
-  __nv_bfloat16* s_blo = reinterpret_cast<__nv_bfloat16*>(smem + 2 * a_bytes + b_bytes);
-  // two pair buffers: the next tile's setup runs while this tile's MMA is in flight
-  FlashPair* sp_buf = reinterpret_cast<FlashPair*>(smem + 2 * a_bytes + 2 * b_bytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sp_buf + 2 * kFlashPairs);
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 2);
-  uint16_t* s_order = reinterpret_cast<uint16_t*>(bars + 4);  // pairs of the share by interval
-  uint16_t* s_bucket = s_order + kFlashSort;
-  int* s_count = reinterpret_cast<int*>(s_bucket + kFlashSort);  // [buckets]
-  uint64_t* bar_b = bars;
-  uint64_t* bar_mma = bars + 1;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool need_lo_b = passes >= 2;
-  if (tid == 0) {
-    mbar_init(bar_b, 1);
-    mbar_init(bar_mma, 1);
-    fence_barrier_init();
-  }
-  if (warp == 0) {
-    tmem_alloc(s_tmem, 256);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *s_tmem;
-  if (tid == 0) {
-    mbar_expect_tx(bar_b, b_bytes * (need_lo_b ? 2u : 1u));
-    bulk_g2s(s_bhi, g_bhi, b_bytes, bar_b);
-    if (need_lo_b) bulk_g2s(s_blo, g_blo, b_bytes, bar_b);
-  }
-  const uint32_t idesc = instr_desc_bf16_f32(128, n_tile);
-  const int64_t n_pairs = (int64_t)flash_count(b) * p.n_om;
-  const int nw = p.n_omega;
-  const int padw = kpad - 2 * nw;
-  uint32_t ph_mma = 0;
-  bool b_ready = false, failed = false, mma_pending = false;
-
-  // this CTA's share of the pairs
-  const int64_t share = (n_pairs + gridDim.x - 1) / gridDim.x;
-  const int64_t share_begin = min(n_pairs, (int64_t)blockIdx.x * share);
-  const int64_t share_end = min(n_pairs, share_begin + share);
-  const int buckets = min(p.n_radii + 1, kFlashMaxBuckets);
-  const int workers = blockDim.x - 32;
-  // spectrum items: thread (group of pairs, frequency)
+LH_DEVICE void flash_spectra(const lh_flash_problem& p, const lh_flash_batch& b,
+                             FlashPair* sp_buf, __nv_bfloat16* s_ahi, __nv_bfloat16* s_alo,
+                             uint64_t* bar_pairs, uint64_t* bar_a, uint64_t* bar_mma, int workers,
+                             int n_bins, int in_chunk, int64_t tiles_before, bool& failed) {
+  const int tid = threadIdx.x, nw = p.n_omega;
   const int groups = max(1, workers / nw), group = tid / nw;
-  for (int64_t chunk = share_begin; chunk < share_end && !failed; chunk += kFlashSort) {
-  const int in_chunk = (int)min((int64_t)kFlashSort, share_end - chunk);
-  for (int i = tid; sorted && i < buckets; i += blockDim.x) s_count[i] = 0;
-  __syncthreads();
-  for (int i = tid; sorted && i < in_chunk; i += blockDim.x) {
-    const int j = flash_bucket(p, b, chunk + i, buckets);
-    s_bucket[i] = (uint16_t)j;
-    atomicAdd(s_count + j, 1);
-  }
-  __syncthreads();
-  if (sorted && warp == 0) {  // exclusive prefix sums
-    int carry = 0;
-    for (int first = 0; first < buckets; first += 32) {
-      const int v = first + lane < buckets ? s_count[first + lane] : 0;
-      int sum = v;
-      for (int off = 1; off < 32; off <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, sum, off);
-        if (lane >= off) sum += up;
-      }
-      if (first + lane < buckets) s_count[first + lane] = carry + sum - v;
-      carry += __shfl_sync(0xffffffffu, sum, 31);
-    }
-  }
-  __syncthreads();
-  for (int i = tid; sorted && i < in_chunk; i += blockDim.x)
-    s_order[atomicAdd(s_count + s_bucket[i], 1)] = (uint16_t)i;
-  __syncthreads();
-  // the pair at place k of the sorted chunk, past its end none
-  auto pair_at = [&](int k) {
-    return k < in_chunk ? chunk + (sorted ? (int)s_order[k] : k) : n_pairs;
-  };
   const int tiles = (in_chunk + kFlashPairs - 1) / kFlashPairs;
-  int cur = 0;
-  if (tid < kFlashPairs) flash_slot_setup(p, b, sp_buf[tid], pair_at(tid), n_pairs);
-  __syncthreads();
   for (int tile = 0; tile < tiles; ++tile) {
-    FlashPair* sp = sp_buf + cur * kFlashPairs;  // set up before the barrier closing the last tile
+    const int64_t at = tiles_before + tile;
+    FlashPair* sp = sp_buf + (at & 1) * kFlashPairs;
     const int count = min(kFlashPairs, in_chunk - tile * kFlashPairs);
-    for (int i = tid; i < 128 * padw; i += blockDim.x) {
-      const int off = a_offset(i / padw, 2 * nw + i % padw);
-      s_ahi[off] = __float2bfloat16_rn(0.f);
-      s_alo[off] = __float2bfloat16_rn(0.f);
+    // this tile's pairs are there, and the tensor core has read the last tile's A
+    bool ok = warp_wait(bar_pairs + (at & 1), (uint32_t)(at >> 1) & 1u);
+    if (ok && at > 0) ok = warp_wait(bar_mma + ((at - 1) & 1), (uint32_t)((at - 1) >> 1) & 1u);
+    if (!ok) {
+      failed = true;
+      return;
     }
-    // The last warp sets up the next tile's pairs (float64, two per lane) while
-    // the other warps compute this tile's spectra, then issues the MMAs while
-    // they write the order-0 rows: neither waits behind the other.
-    if (tid >= workers) {
-      if (tile + 1 < tiles)
-        for (int k = lane; k < kFlashPairs; k += 32)
-          flash_slot_setup(p, b, sp_buf[(cur ^ 1) * kFlashPairs + k],
-                           pair_at((tile + 1) * kFlashPairs + k), n_pairs);
-    } else if (group < groups) {
+    if (group < groups) {
       const int first = group * count / groups, last = (group + 1) * count / groups;
       for (int w = tid - group * nw; w < nw; w += workers) {
         const double om = p.omega[w];
@@ -498,97 +414,252 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
       }
     }
     fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core
-    __syncthreads();
-    if (tid == workers) {
-      bool ok = true;
-      if (!b_ready) {
-        ok = mbar_wait(bar_b, 0);
-        b_ready = true;
-      }
-      if (ok) {
-        tc_fence_after();
-        const int ksteps = kpad / 16;
-        const uint32_t lbo_a = kAChunk * 2u, lbo_b = (uint32_t)n_tile * 16u;
-        int first = 1;
-        for (int pass = 0; pass < passes; ++pass) {
-          const __nv_bfloat16* pa = (pass == 2) ? s_alo : s_ahi;
-          const __nv_bfloat16* pb = (pass == 1) ? s_blo : s_bhi;
-          for (int kk = 0; kk < ksteps; ++kk) {
-            uint64_t da = smem_desc_kmajor(reinterpret_cast<const uint8_t*>(pa) + kk * 2 * lbo_a,
-                                           lbo_a, 128);
-            uint64_t db = smem_desc_kmajor(reinterpret_cast<const uint8_t*>(pb) + kk * 2 * lbo_b,
-                                           lbo_b, 128);
-            tc_mma_bf16(tmem, da, db, idesc, first ? 0u : 1u);
-            first = 0;
-          }
-        }
-        tc_commit(bar_mma);
-      } else {
-        failed = true;
-      }
+    __syncwarp();
+    if ((tid & 31) == 0) mbar_arrive(bar_a + (at & 1));
+    if (tile + 1 == tiles) {  // nothing left to compute: the order-0 rows of the last tile
+      if (!warp_wait(bar_a + (at & 1), (uint32_t)(at >> 1) & 1u)) failed = true;
+      else flash_tile_order0(p, b, sp, n_bins, tid, workers);
     }
-    if (tid < workers) flash_tile_order0(p, b, sp, n_bins, workers);
-    if (__syncthreads_or(failed)) { failed = true; break; }
-    const bool ok = mbar_wait(bar_mma, ph_mma);
-    ph_mma ^= 1u;
-    if (__syncthreads_or(!ok)) { failed = true; mma_pending = true; break; }
-    tc_fence_after();
-    // drain: warp w reads TMEM lanes 32*(w%4).. (rows); the warps with the same
-    // lane quarter split the 16-column chunks between them
-    const int q = warp & 3, h = warp >> 2, quarters = (int)blockDim.x / 128;
-    const int row = q * 32 + lane;
-    const int lp = row >> 1, order = 1 + (row & 1);
-    const bool valid = sp[lp].valid;
-    const int chunks = n_tile / 16;
-    const int per = (chunks + quarters - 1) / quarters;
-    const int c_begin = h * per, c_end = min(chunks, (h + 1) * per);
-    const uint32_t lane_addr = tmem + ((uint32_t)(q * 32) << 16);
-    float* dst = b.components + (sp[lp].pair * 3 + order) * (int64_t)n_bins;
-    const bool vec = (n_bins & 3) == 0;
-    // The A tile is free once the MMA has completed: each warp transposes its
-    // 32 rows x 16 bins through a 32 x 20-float slice of it, so that four
-    // lanes store one row's 64 bytes and a store instruction covers eight rows
-    // (full 32-byte sectors) instead of 32 rows at a 16-byte stride.
-    float* stage = reinterpret_cast<float*>(smem) + warp * 32 * 20;
-    const bool staged = vec && 2u * a_bytes >= (blockDim.x / 32) * 32u * 20u * sizeof(float);
-    for (int c = c_begin; c < c_end; ++c) {
-      float v[16];
-      tmem_ld16(lane_addr + (uint32_t)(c * 16), v);
-      if (staged && c * 16 + 16 <= n_bins) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<float4*>(stage + lane * 20 + 4 * i) =
-              make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        __syncwarp();
-#pragma unroll
-        for (int it = 0; it < 4; ++it) {
-          const int r = it * 8 + (lane >> 2), part = lane & 3;
-          const int trow = q * 32 + r;
-          const int tlp = trow >> 1, torder = 1 + (trow & 1);
-          if (sp[tlp].valid) {
-            const float4 x = *reinterpret_cast<const float4*>(stage + r * 20 + 4 * part);
-            *reinterpret_cast<float4*>(b.components + (sp[tlp].pair * 3 + torder) * (int64_t)n_bins +
-                                       c * 16 + 4 * part) = x;
-          }
-        }
-        __syncwarp();
-      } else if (valid) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (c * 16 + i < n_bins) dst[c * 16 + i] = v[i];
-      }
-    }
-    tc_fence_before();
-    __syncthreads();
-    cur ^= 1;
   }
-  }  // chunks
-  if (failed && tid == 0) atomicOr(reinterpret_cast<unsigned*>(b.status), LH_STATUS_TIMEOUT);
-  if (mma_pending) mbar_wait(bar_mma, ph_mma ^ 1u);
-  if (tid == blockDim.x - 32 && !b_ready) mbar_wait(bar_b, 0);  // no bulk copy left in flight
+}
+
+// One tile's MMAs (one thread): hi x hi, hi x lo, lo x hi over the K steps.
+LH_DEVICE void flash_mma(uint32_t d, const __nv_bfloat16* s_ahi, const __nv_bfloat16* s_alo,
+                         const __nv_bfloat16* s_bhi, const __nv_bfloat16* s_blo, int kpad,
+                         int n_tile, int passes) {
+  const uint32_t idesc = instr_desc_bf16_f32(128, n_tile);
+  const int ksteps = kpad / 16;
+  const uint32_t lbo_a = kAChunk * 2u, lbo_b = (uint32_t)n_tile * 16u;
+  int first = 1;
+  for (int pass = 0; pass < passes; ++pass) {
+    const __nv_bfloat16* pa = (pass == 2) ? s_alo : s_ahi;
+    const __nv_bfloat16* pb = (pass == 1) ? s_blo : s_bhi;
+    for (int kk = 0; kk < ksteps; ++kk) {
+      uint64_t da = smem_desc_kmajor(reinterpret_cast<const uint8_t*>(pa) + kk * 2 * lbo_a,
+                                     lbo_a, 128);
+      uint64_t db = smem_desc_kmajor(reinterpret_cast<const uint8_t*>(pb) + kk * 2 * lbo_b,
+                                     lbo_b, 128);
+      tc_mma_bf16(d, da, db, idesc, first ? 0u : 1u);
+      first = 0;
+    }
+  }
+}
+
+// One warp's 32 rows of the accumulator -> components. Four lanes exchange their
+// rows' 16 bins, so that they store one row's 64 bytes together and a store
+// instruction covers eight rows in whole sectors instead of 32 rows in parts.
+LH_DEVICE void flash_drain(const lh_flash_batch& b, const FlashPair* sp, uint32_t d, int quarter,
+                           int n_bins, int n_tile) {
+  const int lane = threadIdx.x & 31;
+  const int row = quarter * 32 + lane;
+  if (!__any_sync(0xffffffffu, sp[row >> 1].valid)) return;
+  const uint32_t addr = d + ((uint32_t)(quarter * 32) << 16);
+  const bool vec = (n_bins & 3) == 0;
+  const bool upper = lane & 2, odd = lane & 1;
+  for (int c = 0; c < n_tile; c += 16) {
+    float v[16];
+    tmem_ld16(addr + (uint32_t)c, v);
+    if (vec && c + 16 <= n_bins) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {  // parts 2, 3 of the lower lanes <-> 0, 1 of the upper
+        const float got = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[8 + i], 2);
+        if (upper) v[i] = got; else v[8 + i] = got;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // parts 1, 3 of the even lanes <-> 0, 2 of the odd
+        const float got0 = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[4 + i], 1);
+        const float got1 = __shfl_xor_sync(0xffffffffu, odd ? v[8 + i] : v[12 + i], 1);
+        if (odd) { v[i] = got0; v[8 + i] = got1; } else { v[4 + i] = got0; v[12 + i] = got1; }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {  // part lane & 3 of row 4 (lane / 4) + j
+        const int r = quarter * 32 + (lane & ~3) + j;
+        const FlashPair& s = sp[r >> 1];
+        if (s.valid)
+          *reinterpret_cast<float4*>(b.components + (s.pair * 3 + 1 + (r & 1)) * (int64_t)n_bins +
+                                     c + 4 * (lane & 3)) =
+              make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      }
+    } else if (sp[row >> 1].valid) {
+      float* dst = b.components + (sp[row >> 1].pair * 3 + 1 + (row & 1)) * (int64_t)n_bins;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (c + i < n_bins) dst[c + i] = v[i];
+    }
+  }
+}
+
+template <int kDegrees>
+__global__ void __launch_bounds__(kFlashTcThreads, 1)
+flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __restrict__ g_bhi,
+                const __nv_bfloat16* __restrict__ g_blo, int kpad, int n_bins, int n_tile,
+                int passes, int sorted) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t a_bytes = (uint32_t)(kpad / 8) * kAChunk * 2u;
+  const uint32_t b_bytes = (uint32_t)n_tile * kpad * 2u;
+  __nv_bfloat16* s_ahi = reinterpret_cast<__nv_bfloat16*>(smem);
+  __nv_bfloat16* s_alo = reinterpret_cast<__nv_bfloat16*>(smem + a_bytes);
+  __nv_bfloat16* s_bhi = reinterpret_cast<__nv_bfloat16*>(smem + 2 * a_bytes);
+  __nv_bfloat16* s_blo = reinterpret_cast<__nv_bfloat16*>(smem + 2 * a_bytes + b_bytes);
+  // two pair buffers: a tile's drain sets up the pairs of the tile after next
+  FlashPair* sp_buf = reinterpret_cast<FlashPair*>(smem + 2 * a_bytes + 2 * b_bytes);
+  uint64_t* bar_b = reinterpret_cast<uint64_t*>(sp_buf + 2 * kFlashPairs);
+  // for even and odd tiles: pairs set up, A written, accumulators complete. Each
+  // completes once per tile, and only after all its waiters of the tile two before.
+  uint64_t* bar_pairs = bar_b + 1;
+  uint64_t* bar_a = bar_b + 3;
+  uint64_t* bar_mma = bar_b + 5;
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar_b + 7);
+  uint16_t* s_order = reinterpret_cast<uint16_t*>(bar_b + 8);  // pairs of the share by interval
+  uint16_t* s_bucket = s_order + kFlashSort;
+  int* s_count = reinterpret_cast<int*>(s_bucket + kFlashSort);  // [buckets]
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // roles: spectra (the first warps), drain (four warps), MMA (the last warp)
+  const int mma_warp = (int)(blockDim.x >> 5) - 1, drain_warp = mma_warp - 4;
+  const int workers = 32 * drain_warp;
+  const bool need_lo_b = passes >= 2;
+  if (tid == 0) {
+    mbar_init(bar_b, 1);
+    for (int k = 0; k < 2; ++k) {
+      mbar_init(bar_pairs + k, 4);
+      mbar_init(bar_a + k, drain_warp);
+      mbar_init(bar_mma + k, 1);
+    }
+    fence_barrier_init();
+  }
+  const uint32_t d_stride = n_tile <= 128 ? 128u : 256u;  // TMEM columns between accumulators
+  if (warp == 0) {
+    tmem_alloc(s_tmem, 2 * d_stride);
+    tmem_relinquish();
+  }
+  const int64_t n_pairs = (int64_t)flash_count(b) * p.n_om;
+  const int nw = p.n_omega;
+  const int padw = kpad - 2 * nw;
+  for (int i = tid; i < 128 * padw; i += blockDim.x) {  // columns that no spectrum fills
+    const int off = a_offset(i / padw, 2 * nw + i % padw);
+    s_ahi[off] = __float2bfloat16_rn(0.f);
+    s_alo[off] = __float2bfloat16_rn(0.f);
+  }
+  fence_proxy_async();
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 256);
+  tc_fence_after();
+  const uint32_t tmem = *s_tmem;
+  if (tid == 0) {
+    mbar_expect_tx(bar_b, b_bytes * (need_lo_b ? 2u : 1u));
+    bulk_g2s(s_bhi, g_bhi, b_bytes, bar_b);
+    if (need_lo_b) bulk_g2s(s_blo, g_blo, b_bytes, bar_b);
+  }
+  bool b_ready = false, failed = false;
+  int64_t issued = -1;  // the MMA warp's last tile
+
+  // this CTA's share of the pairs
+  const int64_t share = (n_pairs + gridDim.x - 1) / gridDim.x;
+  const int64_t share_begin = min(n_pairs, (int64_t)blockIdx.x * share);
+  const int64_t share_end = min(n_pairs, share_begin + share);
+  const int buckets = min(p.n_radii + 1, kFlashMaxBuckets);
+  int64_t tiles_before = 0;  // tiles of the chunks before: the barriers' phases go on
+  for (int64_t chunk = share_begin; chunk < share_end && !failed; chunk += kFlashSort) {
+    const int in_chunk = (int)min((int64_t)kFlashSort, share_end - chunk);
+    for (int i = tid; sorted && i < buckets; i += blockDim.x) s_count[i] = 0;
+    __syncthreads();
+    for (int i = tid; sorted && i < in_chunk; i += blockDim.x) {
+      const int j = flash_bucket(p, b, chunk + i, buckets);
+      s_bucket[i] = (uint16_t)j;
+      atomicAdd(s_count + j, 1);
+    }
+    __syncthreads();
+    if (sorted && warp == 0) {  // exclusive prefix sums
+      int carry = 0;
+      for (int first = 0; first < buckets; first += 32) {
+        const int v = first + lane < buckets ? s_count[first + lane] : 0;
+        int sum = v;
+        for (int off = 1; off < 32; off <<= 1) {
+          const int up = __shfl_up_sync(0xffffffffu, sum, off);
+          if (lane >= off) sum += up;
+        }
+        if (first + lane < buckets) s_count[first + lane] = carry + sum - v;
+        carry += __shfl_sync(0xffffffffu, sum, 31);
+      }
+    }
+    __syncthreads();
+    for (int i = tid; sorted && i < in_chunk; i += blockDim.x)
+      s_order[atomicAdd(s_count + s_bucket[i], 1)] = (uint16_t)i;
+    __syncthreads();
+    // the pair at place k of the sorted chunk, past its end none
+    auto pair_at = [&](int k) {
+      return k < in_chunk ? chunk + (sorted ? (int)s_order[k] : k) : n_pairs;
+    };
+    const int tiles = (in_chunk + kFlashPairs - 1) / kFlashPairs;
+    // the first two tiles' pairs
+    if (tid < 2 * kFlashPairs && tid / kFlashPairs < tiles)
+      flash_slot_setup(p, b,
+                       sp_buf[((tiles_before + tid / kFlashPairs) & 1) * kFlashPairs +
+                              tid % kFlashPairs],
+                       pair_at(tid), n_pairs);
+    __syncthreads();
+    if (warp < drain_warp) {
+      flash_spectra<kDegrees>(p, b, sp_buf, s_ahi, s_alo, bar_pairs, bar_a, bar_mma, workers,
+                              n_bins, in_chunk, tiles_before, failed);
+    } else if (warp == mma_warp) {
+      for (int tile = 0; tile < tiles && !failed; ++tile) {
+        const int64_t at = tiles_before + tile;
+        const uint32_t parity = (uint32_t)(at >> 1) & 1u;
+        if (!b_ready) {
+          b_ready = true;
+          if (!warp_wait(bar_b, 0)) failed = true;
+        }
+        if (!failed && !warp_wait(bar_a + (at & 1), parity)) failed = true;
+        if (failed) break;
+        tc_fence_after();
+        if (lane == 0) {
+          flash_mma(tmem + (uint32_t)(at & 1) * d_stride, s_ahi, s_alo, s_bhi, s_blo, kpad,
+                    n_tile, passes);
+          tc_commit(bar_mma + (at & 1));
+        }
+        __syncwarp();
+        issued = at;
+      }
+    } else {
+      const int index = tid - 32 * drain_warp;
+      if (lane == 0)
+        for (int k = 0; k < min(2, tiles); ++k) mbar_arrive(bar_pairs + ((tiles_before + k) & 1));
+      for (int tile = 0; tile < tiles; ++tile) {
+        const int64_t at = tiles_before + tile;
+        const uint32_t parity = (uint32_t)(at >> 1) & 1u;
+        FlashPair* sp = sp_buf + (at & 1) * kFlashPairs;
+        bool ok = warp_wait(bar_pairs + (at & 1), parity) && warp_wait(bar_a + (at & 1), parity);
+        if (ok && tile + 1 < tiles) flash_tile_order0(p, b, sp, n_bins, index, 128);
+        ok = ok && warp_wait(bar_mma + (at & 1), parity);
+        if (ok) {
+          tc_fence_after();
+          flash_drain(b, sp, tmem + (uint32_t)(at & 1) * d_stride, warp & 3, n_bins, n_tile);
+          tc_fence_before();
+        }
+        if (group_sync_or<128>(0, !ok)) {  // all four warps are done with the pairs, or none goes on
+          failed = true;
+          break;
+        }
+        if (tile + 2 < tiles) {
+          if (index < kFlashPairs)
+            flash_slot_setup(p, b, sp[index], pair_at((tile + 2) * kFlashPairs + index), n_pairs);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_pairs + (at & 1));
+        }
+      }
+    }
+    failed = __syncthreads_or(failed);
+    tiles_before += tiles;
+  }
+  if (failed && tid == 0) atomicOr(reinterpret_cast<unsigned*>(b.status), LH_STATUS_TIMEOUT);
+  if (warp == mma_warp) {  // nothing in flight when the CTA ends
+    if (issued >= 0) mbar_wait(bar_mma + (issued & 1), (uint32_t)(issued >> 1) & 1u);
+    if (!b_ready) mbar_wait(bar_b, 0);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 2 * d_stride);
 }
 
 // ---------------------------------------------------------------- broadband

@@ -810,25 +810,6 @@ LH_DEVICE bool elect_one() {
   return mine != 0;
 }
 
-// mbar_wait of a whole warp, with one outcome for all its lanes.
-LH_DEVICE bool warp_wait(uint64_t* bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
-}
-
-// A barrier of the four warps of an epilogue group; true when `flag` holds on any.
-LH_DEVICE bool group_sync_or(int group, bool flag) {
-  int any;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %2, 0;\n\t"
-      "barrier.cta.red.or.pred q, %1, 128, p;\n\t"
-      "selp.b32 %0, 1, 0, q;\n\t}"
-      : "=r"(any)
-      : "r"(1 + group), "r"((int)flag)
-      : "memory");
-  return any != 0;
-}
-
 struct Ge2TcBars {
   uint64_t a_full[kTcAStages], a_empty[kTcAStages];
   uint64_t b_full[kTcBStages], b_empty[kTcBStages];
@@ -902,14 +883,14 @@ ge2_tc_kernel(const lh_ge2_table T, const Ge2TcArgs G) {
         const int lam = m_ok ? m / W : 0, wq = m_ok ? m % W : 0;
         // the table of the item before has been read; a wait that gave up ends
         // all four warps here
-        if (group_sync_or(g, failed)) { failed = true; break; }
+        if (group_sync_or<128>(g, failed)) { failed = true; break; }
         for (int e = quarter * 32 + lane; e < P * NB; e += 128) {
           // places past the last pair repeat the first: computed, not written
           const int band = e / P, i = e - band * P;
           const Ge2TcEntry& q = G.entries[t.first + g * P + (i < cnt ? i : 0)];
           table[e] = q.rows + band * q.band_bytes;
         }
-        group_sync_or(g, false);
+        group_sync_or<128>(g, false);
         const char* const* mine = table + lam * P;
         const uint32_t wq_bytes = (uint32_t)wq * (uint32_t)sizeof(float2);
         float acc_re[P], acc_im[P];

@@ -173,3 +173,24 @@ def test_flash_run_on_a_stream_and_response_equal_the_default(transports, flash_
     b = ft.transport(IsotropicFlash.monochromatic(pos[-1], 1e10, 450.0, time_ns=times[-1]))
     for key in ("spectrum_pe", "components_pe", "charge_components_pe", "time_origin_ns", "active"):
         assert np.array_equal(getattr(a, key), getattr(b, key)), key
+
+
+@pytest.mark.parametrize("count", [1, 137, 200])
+def test_flash_block_sizes_agree(transports, flash_golden, count):
+    """256 threads leave three warps for the spectra, 512 eleven: the same values bit
+    for bit, for one tile per block and for two."""
+    import torch
+    from lighthit_b200.workloads import flash_positions
+    g = flash_golden
+    ft = transports["split-bf16"]
+    pos = torch.tensor(flash_positions(count, g["om_positions_m"].mean(axis=0), seed=5,
+                                       om_positions=g["om_positions_m"]), device=ft.device)
+    photons = torch.full((count,), 1e10, dtype=torch.float64, device=ft.device)
+    times = torch.linspace(0.0, 40.0, count, dtype=torch.float64, device=ft.device)
+    out = {}
+    for threads in (256, 512):
+        out[threads] = ft.allocate(count)
+        ft.launch(pos, photons, times, out[threads], block_threads=threads)
+    torch.cuda.synchronize()
+    for key in ("spectrum", "components", "charge", "origin", "active"):
+        assert torch.equal(out[256][key], out[512][key]), key
