@@ -438,10 +438,13 @@ o1_tile_scan_kernel(int32_t* tile, int64_t n_tiles, int32_t* count) {
 LH_DEVICE void o1_write_pencil(const double* a, lh_order1_pencil_table& Pn, int q);
 
 // finish_pencils (_prompt_numba.py:2247-2354) for slots with a positive weight,
-// compacted into the pencil table in slot order: one CTA per tile, each thread
-// over kO1Tile / kO1FinishThreads consecutive slots, ranks by a CTA scan plus
-// the tile's offset. Slot order follows the keys, so pencils of a cell are
-// neighbours in the table.
+// compacted into the pencil table in slot order: one CTA per tile ranks its used
+// slots (a CTA scan plus the tile's offset), lists them, and takes one per thread.
+// Slot order follows the keys, so pencils of a cell are neighbours in the table.
+// What bounds it is the float64 chain of a pencil (an eigenbasis with sincos and
+// atan2). Used slots are few in a hundred: with each thread finishing its own slots,
+// round by round, a warp ran that chain 16 times for a lane or two each (82.7 us for
+// 94509 pencils in 2.1M slots, 53.3 from the list).
 // Screen tables (the coarse charge screen) take their parents first: parent
 // rows [0, n_parents) record their row per slot in `slot_row`; child rows
 // follow from `base_count` and look up their parent's row by its key.
@@ -455,6 +458,8 @@ o1_finish_kernel(const long long* keys, int64_t capacity, const double* rows,
   constexpr int warps = kO1FinishThreads / 32;
   static_assert(per <= 32 && per * warps == 128, "one 32-bit mask per thread, 4 counts per lane");
   __shared__ int before[per * warps];  // used slots ahead of each (round, warp) in the tile
+  __shared__ uint16_t list[kO1Tile];   // the used slots in slot order
+  __shared__ int in_tile;
   const int64_t n = *count;
   const int64_t base = base_count ? *base_count : 0;
   if (base + n > Pn.capacity) {  // the caller redoes the stage with a larger table
@@ -488,24 +493,30 @@ o1_finish_kernel(const long long* keys, int64_t capacity, const double* rows,
       if (lane >= off) inclusive += up;
     }
     int running = inclusive - sum;
+    if (lane == 31) in_tile = inclusive;
     for (int i = 0; i < 4; ++i) {
       before[4 * lane + i] = running;
       running += v[i];
     }
   }
   __syncthreads();
-  if (!used) return;
   const unsigned lower = (1u << lane) - 1u;
+#pragma unroll
   for (int j = 0; j < per; ++j) {
-    const unsigned b = __ballot_sync(__activemask(), (used >> j) & 1u);
-    if (!((used >> j) & 1u)) continue;
-    const int64_t slot = tile0 + (int64_t)j * kO1FinishThreads;
-    // rank order = slot order: a cell's pencils are neighbours in the table, so
-    // that the 32 pencils of a stage-B warp share their groups (about four items
-    // per group against one for a random order) and the warp sums them before
-    // the atomics
-    const int row = (int)(base + tile_offset[blockIdx.x] + before[j * warps + warp] +
-                          __popc(b & lower));
+    const unsigned b = __ballot_sync(0xffffffffu, (used >> j) & 1u);
+    if ((used >> j) & 1u)
+      list[before[j * warps + warp] + __popc(b & lower)] =
+          (uint16_t)(j * kO1FinishThreads + threadIdx.x);
+  }
+  __syncthreads();
+  // rank order = slot order: a cell's pencils are neighbours in the table, so that
+  // the 32 pencils of a stage-B warp share their groups (about four items per group
+  // against one for a random order) and the warp sums them before the atomics
+  const int64_t tile = blockIdx.x * (int64_t)kO1Tile;
+  const int64_t row0 = base + tile_offset[blockIdx.x];
+  for (int i = threadIdx.x; i < in_tile; i += kO1FinishThreads) {
+    const int64_t slot = tile + list[i];
+    const int row = (int)(row0 + i);
     o1_write_pencil(rows + slot * kO1Moments, Pn, row);
     if (slot_row) slot_row[slot] = row;
     if (Pn.parent) {
