@@ -24,9 +24,9 @@
 // (OM, pencil) computes the pencil's geometry against the OM and adds its
 // moments into that OM's group table (atomics); one CTA per OM sorts its
 // group keys in shared memory (bitonic) and emits its batches; a persistent
-// grid of CTAs takes batches from the global list, builds each batch's path
-// grid and profile in shared memory and deposits its panels; one CTA per OM
-// finishes the bins with the prefix pass. Everything is float64, as the
+// grid of warps takes batches from the global list, builds each batch's path
+// grid and profile and deposits its panels (batches too long for a warp go to
+// CTAs); one CTA per OM finishes the bins by prefix scans. Everything is float64, as the
 // deposit's global quadratic coefficients in t cancel strongly.
 #include <algorithm>
 
