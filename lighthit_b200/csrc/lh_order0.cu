@@ -285,7 +285,8 @@ LH_DEVICE uint32_t o0_word_of_event(const lh_order0_batch& B, uint32_t bits, int
                                     int& ev) {
   ev = o0_event_of(B, base + __ffs(bits) - 1);
   const int64_t rest = (ev + 1 < B.n_events ? B.element_offset[ev + 1] : B.n_elements) - base;
-  return rest < 32 ? bits & ((1u << rest) - 1u) : bits;
+  const uint32_t mine = rest < 32 ? (rest > 0 ? bits & ((1u << rest) - 1u) : 0u) : bits;
+  return mine | (bits & (0u - bits));  // at least one, whatever the offsets
 }
 
 // Candidate pairs counted per (event, OM). A warp takes 32 consecutive elements
