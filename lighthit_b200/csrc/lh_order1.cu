@@ -318,7 +318,10 @@ o1_ring_kernel(const lh_order1_config C, const lh_order1_elements E,
   }
 }
 
-constexpr int kO1Tile = 4096;          // ring-table slots per compaction CTA
+// Ring-table slots per compaction CTA. The fullest tile decides when the finish ends:
+// 35.3 us for the screen's passes with 4096, 24.6 with 2048 and with 1024, whose counts
+// of 16.8M slots take longer (8 showers: 0.25, 0.18 and 0.28 ms).
+constexpr int kO1Tile = 2048;
 constexpr int kO1FinishThreads = 256;  // kO1Tile / kO1FinishThreads consecutive slots each
 
 LH_DEVICE bool o1_slot_used(const long long* keys, const double* rows, int64_t slot) {
@@ -444,7 +447,7 @@ LH_DEVICE void o1_write_pencil(const double* a, lh_order1_pencil_table& Pn, int 
 // What bounds it is the float64 chain of a pencil (an eigenbasis with sincos and
 // atan2). Used slots are few in a hundred: with each thread finishing its own slots,
 // round by round, a warp ran that chain 16 times for a lane or two each (82.7 us for
-// 94509 pencils in 2.1M slots, 53.3 from the list).
+// 94509 pencils in 2.1M slots, 44.4 from the list).
 // Screen tables (the coarse charge screen) take their parents first: parent
 // rows [0, n_parents) record their row per slot in `slot_row`; child rows
 // follow from `base_count` and look up their parent's row by its key.
@@ -456,7 +459,8 @@ o1_finish_kernel(const long long* keys, int64_t capacity, const double* rows,
                  int32_t* status) {
   constexpr int per = kO1Tile / kO1FinishThreads;  // rounds of 256 consecutive slots
   constexpr int warps = kO1FinishThreads / 32;
-  static_assert(per <= 32 && per * warps == 128, "one 32-bit mask per thread, 4 counts per lane");
+  constexpr int counts = per * warps / 32;  // (round, warp) counts per lane of the scan
+  static_assert(per <= 32 && per * warps % 32 == 0, "one 32-bit mask per thread");
   __shared__ int before[per * warps];  // used slots ahead of each (round, warp) in the tile
   __shared__ uint16_t list[kO1Tile];   // the used slots in slot order
   __shared__ int in_tile;
@@ -481,10 +485,10 @@ o1_finish_kernel(const long long* keys, int64_t capacity, const double* rows,
     if (lane == 0) before[j * warps + warp] = __popc(b);
   }
   __syncthreads();
-  if (warp == 0) {  // exclusive scan of the 128 (round, warp) counts in slot order
-    int v[4], sum = 0;
-    for (int i = 0; i < 4; ++i) {
-      v[i] = before[4 * lane + i];
+  if (warp == 0) {  // exclusive scan of the (round, warp) counts in slot order
+    int v[counts], sum = 0;
+    for (int i = 0; i < counts; ++i) {
+      v[i] = before[counts * lane + i];
       sum += v[i];
     }
     int inclusive = sum;
@@ -494,8 +498,8 @@ o1_finish_kernel(const long long* keys, int64_t capacity, const double* rows,
     }
     int running = inclusive - sum;
     if (lane == 31) in_tile = inclusive;
-    for (int i = 0; i < 4; ++i) {
-      before[4 * lane + i] = running;
+    for (int i = 0; i < counts; ++i) {
+      before[counts * lane + i] = running;
       running += v[i];
     }
   }
