@@ -590,6 +590,7 @@ constexpr int kTcGroups = 3;                  // most pair groups per tile
 constexpr int kTcEpiWarps = 4 * kTcGroups;    // one warp per group and lane quarter
 constexpr int kTcBuildWarps = 3;
 constexpr int kTcThreads = 32 * (kTcEpiWarps + kTcBuildWarps + 1);  // 16 warps: 128 registers each
+constexpr size_t kTcSmem = 227 * 1024;        // most shared memory of a CTA
 
 // One (OM, point) pair in range.
 struct __align__(16) Ge2TcEntry {
@@ -613,14 +614,26 @@ struct Ge2TcArgs {
   int row_bytes;                // between channel rows, the same in every problem
 };
 
+size_t ge2_tc_smem_bytes(int pairs, int n_bands, int parts);
+
+// Shared memory of ge2_tc_tiles_kernel: the starts of the intervals' pairs and tiles.
+static size_t ge2_tc_tiles_smem(int n_intervals) {
+  return sizeof(int32_t) * 2 * ((size_t)n_intervals + 1);
+}
+
 // Whether a table takes the tensor-core path; `pairs` per group: 16 where the
 // widest degree's rows x 16 fit an accumulator's columns, else 8 (up to 9 rows).
+// The rings and the table of the pairs' channels, 8 bytes per pair and band, have to
+// fit shared memory (up to 60 bands with 16 pairs, 121 with 8), and so do the starts
+// of the intervals (up to 29000); other tables take the CUDA cores.
 bool ge2_tc_supported(const lh_ge2_table& T, int& halves, int& pairs) {
   const int M = T.n_bands * T.n_omega;
   const int rows_max = 2 * std::min(T.degree, T.max_m) + 1;
   halves = (M + 127) / 128;
   pairs = rows_max * 16 <= kTcCols ? 16 : 8;
-  return M <= 256 && 4 * T.n_pairs <= kTcK && ((rows_max * pairs + 15) & ~15) <= kTcCols;
+  return M <= 256 && 4 * T.n_pairs <= kTcK && ((rows_max * pairs + 15) & ~15) <= kTcCols &&
+         ge2_tc_smem_bytes(pairs, T.n_bands, kTcParts) <= kTcSmem &&
+         ge2_tc_tiles_smem(T.n_intervals) <= kTcSmem - 64;  // one static int beside it
 }
 
 size_t ge2_tc_block_bytes(const lh_ge2_table& T, int halves) {
@@ -1294,7 +1307,12 @@ static int ge2_tc_class_launch(const lh_ge2_table& T, const lh_ge2_problem* P, i
   cudaMemsetAsync(counts, 0, sizeof(int32_t) * (T.n_intervals + 1), s);
   const unsigned bucket_blocks = (unsigned)std::min<int64_t>((max_pairs + 255) / 256, 148 * 4);
   ge2_tc_bucket_kernel<<<dim3(bucket_blocks, count), 256, 0, s>>>(slots, A, T.nch, counts, nullptr);
-  ge2_tc_tiles_kernel<<<1, 256, sizeof(int32_t) * 2 * (T.n_intervals + 1), s>>>(
+  const size_t tiles_smem = ge2_tc_tiles_smem(T.n_intervals);
+  if (tiles_smem > 47 * 1024 &&  // a static int lies beside it
+      cudaFuncSetAttribute(ge2_tc_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)tiles_smem) != cudaSuccess)
+    return LH_ECUDA;
+  ge2_tc_tiles_kernel<<<1, 256, tiles_smem, s>>>(
       T.n_intervals, group_pairs, halves, counts, tiles, n_tiles,
       kernel_units() ? kernel_units() + LH_KT_GE2_TC : nullptr);
   ge2_tc_bucket_kernel<<<dim3(bucket_blocks, count), 256, 0, s>>>(slots, A, T.nch, counts, entries);
@@ -1311,7 +1329,6 @@ static int ge2_tc_class_launch(const lh_ge2_table& T, const lh_ge2_problem* P, i
   G.halves = halves;
   const size_t smem = ge2_tc_smem_bytes(group_pairs, T.n_bands, passes > 1 ? kTcParts : 1);
   auto* kernel = group_pairs == 16 ? ge2_tc_kernel<16> : ge2_tc_kernel<8>;
-  if (smem > 227 * 1024) return LH_EUNSUPPORTED;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return LH_ECUDA;

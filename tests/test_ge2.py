@@ -220,3 +220,63 @@ def test_tensor_core_tile_edges(n_points):
     assert int(table.status.item()) == 0
     for got, ref in zip(out, expected):
         assert np.abs(got.cpu().numpy().T - ref).max() <= GE2_TOL * np.abs(ref).max()
+
+
+def folded_of(n_bands, n_intervals, n_omega, *, degree=1, seed=5):
+    """Seeded folded kernels of one (lambda, mu) pair over 2-150 m."""
+    rng = np.random.default_rng(seed)
+    shape = (n_bands, n_intervals, degree + 1, 1, 4, n_omega)
+    return dict(coefficients=rng.normal(size=shape) + 1j * rng.normal(size=shape),
+                log_r=np.linspace(np.log(2.0), np.log(150.0), n_intervals + 1),
+                omega=np.linspace(0.0, 0.5, n_omega), absorption=np.full(n_bands, 0.02),
+                speed=np.full(n_bands, 0.218), degree=degree, acceptance_degree=0,
+                pair_lambda=np.array([0]), pair_mu=np.array([0]), phase="flight")
+
+
+def test_tensor_core_shapes_by_their_shared_memory():
+    """The pairs' channel pointers of every band, and the starts of every interval, lie
+    in shared memory: tables with more take the CUDA cores, others the tensor cores
+    (16 pairs per group up to azimuthal degree 2, 8 above)."""
+    import ctypes
+    from lighthit_b200 import _lib
+
+    def packed(n_bands, n_intervals=47, n_omega=1, max_m=2):
+        one = ctypes.c_void_p(16)  # only its presence is looked at
+        return int(_lib.load().lh_ge2_tc_pack_bytes(_lib.Ge2Table(
+            n_bands, n_intervals, 8, 2, max_m, 6, 39, n_omega, one, one, one, one, one, one, one,
+            one, one, one, 2, 1)))
+
+    for n_bands, max_m, takes in ((1, 2, True), (60, 2, True), (61, 2, False), (256, 2, False),
+                                  (61, 4, True), (121, 4, True), (122, 4, False)):
+        assert (packed(n_bands, max_m=max_m) > 0) == takes, (n_bands, max_m)
+    for n_intervals, takes in ((6000, True), (6200, True), (29000, True), (29100, False)):
+        assert (packed(3, n_intervals, 65) > 0) == takes, n_intervals
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_bands, n_intervals", [(60, 7), (64, 7), (2, 6200)])
+def test_many_bands_and_many_intervals_match_the_oracle(n_bands, n_intervals):
+    """Tables on both sides of the shared-memory limit of the channel pointers, and
+    one whose interval starts pass 48 KB: split-BF16 applies against the float64
+    oracle, on whichever cores they take."""
+    from lighthit_b200.ge2 import AxialSources, Ge2Table
+    g, _, frame = fixture()
+    t = folded_of(n_bands, n_intervals, 4 if n_bands > 2 else 3)
+    W = len(t["omega"])
+    table = Ge2Table(t, [1.0], source_degree=1, azimuthal_degree=1)
+    assert (table.tc_packed() is not None) == (n_bands != 64)
+    rng = np.random.default_rng(n_bands)
+    pts = points(g, frame, "zero")[:20]
+    ch = (rng.normal(size=(n_bands, 20, 4, W))
+          + 1j * rng.normal(size=(n_bands, 20, 4, W))).astype(np.complex64)
+    src = AxialSources(pts, ch, np.zeros(n_bands),
+                       (frame["centre"], frame["first"], frame["second"], frame["axis"]), 1, 1)
+    oms = np.arange(0, 48, 5)
+    out = table.apply_batch([(src, g["om_positions_m"][oms], g["om_looks"][oms],
+                              g["om_area_m2"][oms], g["radial_window_m"])], mode="split-bf16")[0]
+    assert table.status is None or int(table.status.item()) == 0
+    ref = oracle_apply(t, dict(points_m=pts, channels=ch, reference_ns=np.zeros(n_bands),
+                               frame=frame, degree=1, azimuthal_degree=1),
+                       g["om_positions_m"][oms], g["om_looks"][oms], [1.0], g["om_area_m2"][oms],
+                       g["radial_window_m"], fast=True)
+    assert np.abs(out.cpu().numpy().T - ref).max() <= GE2_TOL * np.abs(ref).max()
