@@ -153,11 +153,11 @@ int lh_flash_transport(const lh_flash_problem* p, const lh_readout_operator* op,
   const bool sorted = flash_tc_smem_bytes(op->k_pad, op->n_tile, true) <= 227 * 1024;
   size_t smem = flash_tc_smem_bytes(op->k_pad, op->n_tile, sorted);
   if (smem > 227 * 1024) return LH_EUNSUPPORTED;
-  const FlashTcKernel kernel = flash_tc_kernel_of(p->acc_top + 1);
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int grid = (int)(n_pairs < sm_count() ? n_pairs : sm_count());
   const int threads = b->block_threads == 0 ? 512 : b->block_threads;
   if (threads != 256 && threads != 512) return LH_EINVAL;
+  const FlashTcKernel kernel = flash_tc_kernel_of(p->acc_top + 1, threads);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int grid = (int)(n_pairs < sm_count() ? n_pairs : sm_count());
   {
     lh::TimedLaunch timed_launch(LH_KT_FLASH, s);
     kernel<<<grid, threads, smem, s>>>(*p, *b, reinterpret_cast<const __nv_bfloat16*>(op->b_hi),

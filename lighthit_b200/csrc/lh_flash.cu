@@ -324,9 +324,9 @@ flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins, f
 // rows, drain the accumulator and set up the pairs of the tile after next, while the
 // first warps compute the next tile. They wait only for the MMAs, since A is there
 // once. A share of few pairs (a single flash) spreads over the SMs pair by pair.
-// kDegrees: acceptance degrees whose coefficients a thread holds (0: any, read for
-// every pair; four degrees or more would not fit beside the rest in the 128 registers
-// of a thread).
+// kDegrees: acceptance degrees whose coefficients a thread holds, two or three (four or
+// more would not fit beside the rest in the 128 registers of a thread; flash_step_kernel
+// takes those).
 //
 // What bounds it: the outputs (65 frequencies x 24 bytes and 480 bins x 4 bytes a
 // pair) take 0.10 ms for 4096 flashes of 48 OMs. The launch took 0.380 ms with
@@ -338,6 +338,8 @@ flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins, f
 // 0.148). One flash: 21.8 us on one SM, now 13.9 on 48. 137 flashes: 25.4, now 22.2.
 constexpr int kFlashSort = 2048;        // pairs sorted at a time
 constexpr int kFlashMaxBuckets = 1024;  // radial intervals the sort tells apart
+constexpr int kFlashRun = 4;            // pairs that share coefficients not held
+constexpr int kFlashDense = 2;          // pairs per interval from which runs share them
 
 // The pair's radial interval for the sort, in float32: where it is off by one the
 // pair only sits between neighbours of another interval.
@@ -352,15 +354,103 @@ LH_DEVICE int flash_bucket(const lh_flash_problem& p, const lh_flash_batch& b, i
   return min(max(j, 0), buckets - 1);
 }
 
-// The spectra of a chunk's tiles, written as A rows (order 1, order 2 of each pair):
-// thread (group of pairs, frequency).
+// One (pair, frequency) from its contracted spectra: the outputs and the A rows of
+// orders 1 and 2, K columns (Re, Im) per frequency, one bf16x2 store per row and part.
+LH_DEVICE void flash_rows(const lh_flash_problem& p, const lh_flash_batch& b, int w, double om,
+                          FlashPair& s, float2 s1, float2 s2, int lp, __nv_bfloat16* s_ahi,
+                          __nv_bfloat16* s_alo) {
+  float2 r1, r2;
+  flash_item(p, b, w, om, s, s1, s2, r1, r2);
+  const __nv_bfloat162 h1 = __floats2bfloat162_rn(r1.x, r1.y);
+  const __nv_bfloat162 l1 = __floats2bfloat162_rn(r1.x - __low2float(h1),
+                                                  r1.y - __high2float(h1));
+  const __nv_bfloat162 h2 = __floats2bfloat162_rn(r2.x, r2.y);
+  const __nv_bfloat162 l2 = __floats2bfloat162_rn(r2.x - __low2float(h2),
+                                                  r2.y - __high2float(h2));
+  const int o1 = a_offset(2 * lp, 2 * w), o2 = a_offset(2 * lp + 1, 2 * w);
+  *reinterpret_cast<__nv_bfloat162*>(s_ahi + o1) = h1;
+  *reinterpret_cast<__nv_bfloat162*>(s_alo + o1) = l1;
+  *reinterpret_cast<__nv_bfloat162*>(s_ahi + o2) = h2;
+  *reinterpret_cast<__nv_bfloat162*>(s_alo + o2) = l2;
+}
+
+// A tile's spectra, written as A rows (order 1, order 2 of each pair), by the first
+// `team` threads: thread (group of pairs, frequency). kDegrees: acceptance degrees whose
+// coefficients a thread holds, reading them again where the interval changes (0: any
+// number, read for every pair).
+template <int kDegrees>
+LH_DEVICE void flash_tile_spectra(const lh_flash_problem& p, const lh_flash_batch& b,
+                                  FlashPair* sp, __nv_bfloat16* s_ahi, __nv_bfloat16* s_alo,
+                                  int count, int team) {
+  const int tid = threadIdx.x, nw = p.n_omega;
+  const int groups = max(1, team / nw), group = tid / nw;
+  if (group >= groups) return;
+  const int first = group * count / groups, last = (group + 1) * count / groups;
+  for (int w = tid - group * nw; w < nw; w += team) {
+    const double om = p.omega[w];
+    constexpr int kHeld = kDegrees > 0 ? kDegrees : 1;
+    FlashCoef held[kHeld];
+    int j_held = -1;
+    for (int lp = first; lp < last; ++lp) {
+      FlashPair& s = sp[lp];
+      float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f);
+      if (s.j >= 0) {
+        if (kDegrees > 0) {
+          if (s.j != j_held) {
+            j_held = s.j;
+#pragma unroll
+            for (int l = 0; l < kHeld; ++l) held[l] = flash_coef(p, j_held, l, w);
+          }
+#pragma unroll
+          for (int l = 0; l < kHeld; ++l) flash_degree(held[l], s.tt, s.w[l], s1, s2);
+        } else {
+          for (int l = 0; l <= p.acc_top; ++l)
+            flash_degree(flash_coef(p, s.j, l, w), s.tt, s.w[l], s1, s2);
+        }
+      }
+      flash_rows(p, b, w, om, s, s1, s2, lp, s_ahi, s_alo);
+    }
+  }
+}
+
+// The same by runs of kFlashRun neighbouring pairs and one frequency: a degree's
+// coefficients are read once for the run's pairs of one interval.
+LH_DEVICE void flash_tile_runs(const lh_flash_problem& p, const lh_flash_batch& b, FlashPair* sp,
+                               __nv_bfloat16* s_ahi, __nv_bfloat16* s_alo, int count, int team) {
+  const int nw = p.n_omega, runs = (count + kFlashRun - 1) / kFlashRun;
+  for (int i = threadIdx.x; i < runs * nw; i += team) {
+    const int run = i / nw, w = i - run * nw;
+    FlashPair* q = sp + run * kFlashRun;  // slots past the count hold no pair
+    float2 s1[kFlashRun], s2[kFlashRun];
+#pragma unroll
+    for (int k = 0; k < kFlashRun; ++k) s1[k] = s2[k] = make_float2(0.f, 0.f);
+    for (int l = 0; l <= p.acc_top; ++l) {
+      FlashCoef c;
+      int j_held = -1;
+#pragma unroll
+      for (int k = 0; k < kFlashRun; ++k) {
+        if (q[k].j < 0) continue;
+        if (q[k].j != j_held) {
+          j_held = q[k].j;
+          c = flash_coef(p, j_held, l, w);
+        }
+        flash_degree(c, q[k].tt, q[k].w[l], s1[k], s2[k]);
+      }
+    }
+    const double om = p.omega[w];
+#pragma unroll
+    for (int k = 0; k < kFlashRun; ++k)
+      flash_rows(p, b, w, om, q[k], s1[k], s2[k], run * kFlashRun + k, s_ahi, s_alo);
+  }
+}
+
+// The spectra warps' way through a chunk's tiles.
 template <int kDegrees>
 LH_DEVICE void flash_spectra(const lh_flash_problem& p, const lh_flash_batch& b,
                              FlashPair* sp_buf, __nv_bfloat16* s_ahi, __nv_bfloat16* s_alo,
                              uint64_t* bar_pairs, uint64_t* bar_a, uint64_t* bar_mma, int workers,
                              int n_bins, int in_chunk, int64_t tiles_before, bool& failed) {
-  const int tid = threadIdx.x, nw = p.n_omega;
-  const int groups = max(1, workers / nw), group = tid / nw;
+  const int tid = threadIdx.x;
   const int tiles = (in_chunk + kFlashPairs - 1) / kFlashPairs;
   for (int tile = 0; tile < tiles; ++tile) {
     const int64_t at = tiles_before + tile;
@@ -373,46 +463,7 @@ LH_DEVICE void flash_spectra(const lh_flash_problem& p, const lh_flash_batch& b,
       failed = true;
       return;
     }
-    if (group < groups) {
-      const int first = group * count / groups, last = (group + 1) * count / groups;
-      for (int w = tid - group * nw; w < nw; w += workers) {
-        const double om = p.omega[w];
-        constexpr int kHeld = kDegrees > 0 ? kDegrees : 1;
-        FlashCoef held[kHeld];
-        int j_held = -1;
-        for (int lp = first; lp < last; ++lp) {
-          FlashPair& s = sp[lp];
-          float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f), r1, r2;
-          if (s.j >= 0) {
-            if (kDegrees > 0) {
-              if (s.j != j_held) {
-                j_held = s.j;
-#pragma unroll
-                for (int l = 0; l < kHeld; ++l) held[l] = flash_coef(p, j_held, l, w);
-              }
-#pragma unroll
-              for (int l = 0; l < kHeld; ++l) flash_degree(held[l], s.tt, s.w[l], s1, s2);
-            } else {
-              for (int l = 0; l <= p.acc_top; ++l)
-                flash_degree(flash_coef(p, s.j, l, w), s.tt, s.w[l], s1, s2);
-            }
-          }
-          flash_item(p, b, w, om, s, s1, s2, r1, r2);
-          // K columns (Re, Im) per frequency: one bf16x2 store per row and part
-          const __nv_bfloat162 h1 = __floats2bfloat162_rn(r1.x, r1.y);
-          const __nv_bfloat162 l1 = __floats2bfloat162_rn(r1.x - __low2float(h1),
-                                                          r1.y - __high2float(h1));
-          const __nv_bfloat162 h2 = __floats2bfloat162_rn(r2.x, r2.y);
-          const __nv_bfloat162 l2 = __floats2bfloat162_rn(r2.x - __low2float(h2),
-                                                          r2.y - __high2float(h2));
-          const int o1 = a_offset(2 * lp, 2 * w), o2 = a_offset(2 * lp + 1, 2 * w);
-          *reinterpret_cast<__nv_bfloat162*>(s_ahi + o1) = h1;
-          *reinterpret_cast<__nv_bfloat162*>(s_alo + o1) = l1;
-          *reinterpret_cast<__nv_bfloat162*>(s_ahi + o2) = h2;
-          *reinterpret_cast<__nv_bfloat162*>(s_alo + o2) = l2;
-        }
-      }
-    }
+    flash_tile_spectra<kDegrees>(p, b, sp, s_ahi, s_alo, count, workers);
     fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core
     __syncwarp();
     if ((tid & 31) == 0) mbar_arrive(bar_a + (at & 1));
@@ -445,18 +496,18 @@ LH_DEVICE void flash_mma(uint32_t d, const __nv_bfloat16* s_ahi, const __nv_bflo
   }
 }
 
-// One warp's 32 rows of the accumulator -> components. Four lanes exchange their
+// One warp's 32 rows and columns [begin, end) of the accumulator -> components. Four lanes exchange their
 // rows' 16 bins, so that they store one row's 64 bytes together and a store
 // instruction covers eight rows in whole sectors instead of 32 rows in parts.
 LH_DEVICE void flash_drain(const lh_flash_batch& b, const FlashPair* sp, uint32_t d, int quarter,
-                           int n_bins, int n_tile) {
+                           int n_bins, int begin, int end) {
   const int lane = threadIdx.x & 31;
   const int row = quarter * 32 + lane;
   if (!__any_sync(0xffffffffu, sp[row >> 1].valid)) return;
   const uint32_t addr = d + ((uint32_t)(quarter * 32) << 16);
   const bool vec = (n_bins & 3) == 0;
   const bool upper = lane & 2, odd = lane & 1;
-  for (int c = 0; c < n_tile; c += 16) {
+  for (int c = begin; c < end; c += 16) {
     float v[16];
     tmem_ld16(addr + (uint32_t)c, v);
     if (vec && c + 16 <= n_bins) {
@@ -489,30 +540,86 @@ LH_DEVICE void flash_drain(const lh_flash_batch& b, const FlashPair* sp, uint32_
   }
 }
 
+// Shared memory of a fused CTA.
+struct FlashSmem {
+  uint32_t b_bytes;
+  __nv_bfloat16 *ahi, *alo, *bhi, *blo;
+  FlashPair* pairs;  // two tiles' pairs
+  // operator loaded; then for even and odd tiles: pairs set up, A written, accumulators
+  // complete. Each completes once per tile, and only after all its waiters of the tile
+  // two before.
+  uint64_t *bar_b, *bar_pairs, *bar_a, *bar_mma;
+  uint32_t* tmem;
+  uint16_t *order, *bucket;  // pairs of the share by interval
+  int* count;                // [buckets]
+};
+
+LH_DEVICE FlashSmem flash_smem(uint8_t* smem, int kpad, int n_tile) {
+  FlashSmem S;
+  const uint32_t a_bytes = (uint32_t)(kpad / 8) * kAChunk * 2u;
+  S.b_bytes = (uint32_t)n_tile * kpad * 2u;
+  S.ahi = reinterpret_cast<__nv_bfloat16*>(smem);
+  S.alo = reinterpret_cast<__nv_bfloat16*>(smem + a_bytes);
+  S.bhi = reinterpret_cast<__nv_bfloat16*>(smem + 2 * a_bytes);
+  S.blo = reinterpret_cast<__nv_bfloat16*>(smem + 2 * a_bytes + S.b_bytes);
+  S.pairs = reinterpret_cast<FlashPair*>(smem + 2 * a_bytes + 2 * S.b_bytes);
+  S.bar_b = reinterpret_cast<uint64_t*>(S.pairs + 2 * kFlashPairs);
+  S.bar_pairs = S.bar_b + 1;
+  S.bar_a = S.bar_b + 3;
+  S.bar_mma = S.bar_b + 5;
+  S.tmem = reinterpret_cast<uint32_t*>(S.bar_b + 7);
+  S.order = reinterpret_cast<uint16_t*>(S.bar_b + 8);
+  S.bucket = S.order + kFlashSort;
+  S.count = reinterpret_cast<int*>(S.bucket + kFlashSort);
+  return S;
+}
+
+// The whole CTA: lists the `in_chunk` pairs from `chunk` on by radial interval. The
+// barriers are the CTA's whether it sorts or not.
+LH_DEVICE void flash_sort(const lh_flash_problem& p, const lh_flash_batch& b, const FlashSmem& S,
+                          int64_t chunk, int in_chunk, bool sorted) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int buckets = min(p.n_radii + 1, kFlashMaxBuckets);
+  for (int i = tid; sorted && i < buckets; i += blockDim.x) S.count[i] = 0;
+  __syncthreads();
+  for (int i = tid; sorted && i < in_chunk; i += blockDim.x) {
+    const int j = flash_bucket(p, b, chunk + i, buckets);
+    S.bucket[i] = (uint16_t)j;
+    atomicAdd(S.count + j, 1);
+  }
+  __syncthreads();
+  if (sorted && tid < 32) {  // exclusive prefix sums
+    int carry = 0;
+    for (int first = 0; first < buckets; first += 32) {
+      const int v = first + lane < buckets ? S.count[first + lane] : 0;
+      int sum = v;
+      for (int off = 1; off < 32; off <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, sum, off);
+        if (lane >= off) sum += up;
+      }
+      if (first + lane < buckets) S.count[first + lane] = carry + sum - v;
+      carry += __shfl_sync(0xffffffffu, sum, 31);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; sorted && i < in_chunk; i += blockDim.x)
+    S.order[atomicAdd(S.count + S.bucket[i], 1)] = (uint16_t)i;
+  __syncthreads();
+}
+
 template <int kDegrees>
 __global__ void __launch_bounds__(kFlashTcThreads, 1)
 flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __restrict__ g_bhi,
                 const __nv_bfloat16* __restrict__ g_blo, int kpad, int n_bins, int n_tile,
                 int passes, int sorted) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  const uint32_t a_bytes = (uint32_t)(kpad / 8) * kAChunk * 2u;
-  const uint32_t b_bytes = (uint32_t)n_tile * kpad * 2u;
-  __nv_bfloat16* s_ahi = reinterpret_cast<__nv_bfloat16*>(smem);
-  __nv_bfloat16* s_alo = reinterpret_cast<__nv_bfloat16*>(smem + a_bytes);
-  __nv_bfloat16* s_bhi = reinterpret_cast<__nv_bfloat16*>(smem + 2 * a_bytes);
-  __nv_bfloat16* s_blo = reinterpret_cast<__nv_bfloat16*>(smem + 2 * a_bytes + b_bytes);
-  // two pair buffers: a tile's drain sets up the pairs of the tile after next
-  FlashPair* sp_buf = reinterpret_cast<FlashPair*>(smem + 2 * a_bytes + 2 * b_bytes);
-  uint64_t* bar_b = reinterpret_cast<uint64_t*>(sp_buf + 2 * kFlashPairs);
-  // for even and odd tiles: pairs set up, A written, accumulators complete. Each
-  // completes once per tile, and only after all its waiters of the tile two before.
-  uint64_t* bar_pairs = bar_b + 1;
-  uint64_t* bar_a = bar_b + 3;
-  uint64_t* bar_mma = bar_b + 5;
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bar_b + 7);
-  uint16_t* s_order = reinterpret_cast<uint16_t*>(bar_b + 8);  // pairs of the share by interval
-  uint16_t* s_bucket = s_order + kFlashSort;
-  int* s_count = reinterpret_cast<int*>(s_bucket + kFlashSort);  // [buckets]
+  const FlashSmem S = flash_smem(smem, kpad, n_tile);
+  const uint32_t b_bytes = S.b_bytes;
+  __nv_bfloat16 *s_ahi = S.ahi, *s_alo = S.alo, *s_bhi = S.bhi, *s_blo = S.blo;
+  // a tile's drain sets up the pairs of the tile after next
+  FlashPair* sp_buf = S.pairs;
+  uint64_t *bar_b = S.bar_b, *bar_pairs = S.bar_pairs, *bar_a = S.bar_a, *bar_mma = S.bar_mma;
+  uint32_t* s_tmem = S.tmem;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // roles: spectra (the first warps), drain (four warps), MMA (the last warp)
@@ -558,38 +665,13 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
   const int64_t share = (n_pairs + gridDim.x - 1) / gridDim.x;
   const int64_t share_begin = min(n_pairs, (int64_t)blockIdx.x * share);
   const int64_t share_end = min(n_pairs, share_begin + share);
-  const int buckets = min(p.n_radii + 1, kFlashMaxBuckets);
   int64_t tiles_before = 0;  // tiles of the chunks before: the barriers' phases go on
   for (int64_t chunk = share_begin; chunk < share_end && !failed; chunk += kFlashSort) {
     const int in_chunk = (int)min((int64_t)kFlashSort, share_end - chunk);
-    for (int i = tid; sorted && i < buckets; i += blockDim.x) s_count[i] = 0;
-    __syncthreads();
-    for (int i = tid; sorted && i < in_chunk; i += blockDim.x) {
-      const int j = flash_bucket(p, b, chunk + i, buckets);
-      s_bucket[i] = (uint16_t)j;
-      atomicAdd(s_count + j, 1);
-    }
-    __syncthreads();
-    if (sorted && warp == 0) {  // exclusive prefix sums
-      int carry = 0;
-      for (int first = 0; first < buckets; first += 32) {
-        const int v = first + lane < buckets ? s_count[first + lane] : 0;
-        int sum = v;
-        for (int off = 1; off < 32; off <<= 1) {
-          const int up = __shfl_up_sync(0xffffffffu, sum, off);
-          if (lane >= off) sum += up;
-        }
-        if (first + lane < buckets) s_count[first + lane] = carry + sum - v;
-        carry += __shfl_sync(0xffffffffu, sum, 31);
-      }
-    }
-    __syncthreads();
-    for (int i = tid; sorted && i < in_chunk; i += blockDim.x)
-      s_order[atomicAdd(s_count + s_bucket[i], 1)] = (uint16_t)i;
-    __syncthreads();
+    flash_sort(p, b, S, chunk, in_chunk, sorted);
     // the pair at place k of the sorted chunk, past its end none
     auto pair_at = [&](int k) {
-      return k < in_chunk ? chunk + (sorted ? (int)s_order[k] : k) : n_pairs;
+      return k < in_chunk ? chunk + (sorted ? (int)S.order[k] : k) : n_pairs;
     };
     const int tiles = (in_chunk + kFlashPairs - 1) / kFlashPairs;
     // the first two tiles' pairs
@@ -634,7 +716,7 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
         ok = ok && warp_wait(bar_mma + (at & 1), parity);
         if (ok) {
           tc_fence_after();
-          flash_drain(b, sp, tmem + (uint32_t)(at & 1) * d_stride, warp & 3, n_bins, n_tile);
+          flash_drain(b, sp, tmem + (uint32_t)(at & 1) * d_stride, warp & 3, n_bins, 0, n_tile);
           tc_fence_before();
         }
         if (group_sync_or<128>(0, !ok)) {  // all four warps are done with the pairs, or none goes on
@@ -660,6 +742,127 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 2 * d_stride);
+}
+
+// The CTA in step: all warps but the last form a tile's spectra (the last sets up the
+// next tile's pairs meanwhile, then issues the MMAs), all write its order-0 rows and all
+// drain it. It stays for what the roles slow down:
+//  * CTAs of 256 threads, where the roles leave three warps for the spectra: 4000 flashes
+//    of 48 OMs with 3 degrees take 0.339 ms against 0.507 (2: 0.305, 0.490), 137 flashes
+//    25.6 us against 36.3;
+//  * degrees that are not held, whose spectra outweigh the drains: 4000 flashes with 5
+//    degrees take 0.391 ms against 0.466 (9: 0.528, 0.673), with 256 threads 0.511 against
+//    1.25; 137 flashes with 4 degrees 26.3 us against 28.5.
+// Degrees not held are read once per run of pairs where an interval has two pairs or
+// more on average (700 flashes, 5 degrees: 84.9 us against 89.2 read for every pair; 137,
+// one pair per interval, the other way round: 34 against 29).
+template <int kDegrees>
+__global__ void __launch_bounds__(kFlashTcThreads, 1)
+flash_step_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __restrict__ g_bhi,
+                  const __nv_bfloat16* __restrict__ g_blo, int kpad, int n_bins, int n_tile,
+                  int passes, int sorted) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const FlashSmem S = flash_smem(smem, kpad, n_tile);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int workers = blockDim.x - 32;
+  if (tid == 0) {
+    mbar_init(S.bar_b, 1);
+    mbar_init(S.bar_mma, 1);
+    fence_barrier_init();
+  }
+  const uint32_t columns = n_tile <= 128 ? 128u : 256u;
+  if (warp == 0) {
+    tmem_alloc(S.tmem, columns);
+    tmem_relinquish();
+  }
+  const int padw = kpad - 2 * p.n_omega;
+  for (int i = tid; i < 128 * padw; i += blockDim.x) {  // columns that no spectrum fills
+    const int off = a_offset(i / padw, 2 * p.n_omega + i % padw);
+    S.ahi[off] = __float2bfloat16_rn(0.f);
+    S.alo[off] = __float2bfloat16_rn(0.f);
+  }
+  fence_proxy_async();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *S.tmem;
+  if (tid == 0) {
+    mbar_expect_tx(S.bar_b, S.b_bytes * (passes >= 2 ? 2u : 1u));
+    bulk_g2s(S.bhi, g_bhi, S.b_bytes, S.bar_b);
+    if (passes >= 2) bulk_g2s(S.blo, g_blo, S.b_bytes, S.bar_b);
+  }
+  const int64_t n_pairs = (int64_t)flash_count(b) * p.n_om;
+  const int64_t share = (n_pairs + gridDim.x - 1) / gridDim.x;
+  const int64_t share_begin = min(n_pairs, (int64_t)blockIdx.x * share);
+  const int64_t share_end = min(n_pairs, share_begin + share);
+  // the drain: warp w reads TMEM lanes 32 (w % 4).., the warps of one lane quarter
+  // split the 16-column pieces between them
+  const int pieces = (n_tile / 16 + (int)blockDim.x / 128 - 1) / ((int)blockDim.x / 128) * 16;
+  const int c_begin = min((warp >> 2) * pieces, n_tile), c_end = min(c_begin + pieces, n_tile);
+  bool b_ready = false, failed = false, issued = false;
+  uint32_t phase = 0;  // of the accumulator: one tile each
+  for (int64_t chunk = share_begin; chunk < share_end && !failed; chunk += kFlashSort) {
+    const int in_chunk = (int)min((int64_t)kFlashSort, share_end - chunk);
+    flash_sort(p, b, S, chunk, in_chunk, sorted);
+    auto pair_at = [&](int k) {
+      return k < in_chunk ? chunk + (sorted ? (int)S.order[k] : k) : n_pairs;
+    };
+    const int tiles = (in_chunk + kFlashPairs - 1) / kFlashPairs;
+    const bool dense = sorted && in_chunk >= kFlashDense * p.n_radii;
+    if (tid < kFlashPairs) flash_slot_setup(p, b, S.pairs[tid], pair_at(tid), n_pairs);
+    __syncthreads();
+    for (int tile = 0; tile < tiles; ++tile) {
+      FlashPair* sp = S.pairs + (tile & 1) * kFlashPairs;
+      const int count = min(kFlashPairs, in_chunk - tile * kFlashPairs);
+      if (tid >= workers) {
+        if (tile + 1 < tiles)
+          for (int k = lane; k < kFlashPairs; k += 32)
+            flash_slot_setup(p, b, S.pairs[((tile + 1) & 1) * kFlashPairs + k],
+                             pair_at((tile + 1) * kFlashPairs + k), n_pairs);
+      } else if (kDegrees == 0 && dense) {
+        flash_tile_runs(p, b, sp, S.ahi, S.alo, count, workers);
+      } else {
+        flash_tile_spectra<kDegrees>(p, b, sp, S.ahi, S.alo, count, workers);
+      }
+      fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core
+      __syncthreads();
+      if (tid >= workers) {
+        if (!b_ready) {
+          b_ready = true;
+          if (!warp_wait(S.bar_b, 0)) failed = true;
+        }
+        if (!failed) {
+          tc_fence_after();
+          if (lane == 0) {
+            flash_mma(tmem, S.ahi, S.alo, S.bhi, S.blo, kpad, n_tile, passes);
+            tc_commit(S.bar_mma);
+          }
+          __syncwarp();
+          issued = true;
+        }
+      } else {
+        flash_tile_order0(p, b, sp, n_bins, tid, workers);
+      }
+      failed = __syncthreads_or(failed);
+      if (failed) break;  // nothing was issued for this tile
+      failed = __syncthreads_or(!mbar_wait(S.bar_mma, phase));
+      if (failed) break;
+      issued = false;
+      phase ^= 1u;
+      tc_fence_after();
+      flash_drain(b, sp, tmem, warp & 3, n_bins, c_begin, c_end);
+      tc_fence_before();
+      __syncthreads();
+    }
+  }
+  if (failed && tid == 0) atomicOr(reinterpret_cast<unsigned*>(b.status), LH_STATUS_TIMEOUT);
+  if (warp == (int)(blockDim.x >> 5) - 1) {  // nothing in flight when the CTA ends
+    if (issued) mbar_wait(S.bar_mma, phase);
+    if (!b_ready) mbar_wait(S.bar_b, 0);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, columns);
 }
 
 // ---------------------------------------------------------------- broadband
@@ -779,12 +982,13 @@ size_t flash_tc_smem_bytes(int kpad, int n_tile, bool sorted) {
          (sorted ? 2 * sizeof(uint16_t) * kFlashSort + sizeof(int) * kFlashMaxBuckets : 0);
 }
 
-// The instance that holds `degrees` acceptance degrees in registers.
-FlashTcKernel flash_tc_kernel_of(int degrees) {
+// The instance for a CTA of `threads` and `degrees` acceptance degrees: roles where two
+// or three degrees are held by a CTA of 512, else in step.
+FlashTcKernel flash_tc_kernel_of(int degrees, int threads) {
   switch (degrees) {
-    case 2: return flash_tc_kernel<2>;
-    case 3: return flash_tc_kernel<3>;
-    default: return flash_tc_kernel<0>;
+    case 2: return threads == 512 ? flash_tc_kernel<2> : flash_step_kernel<2>;
+    case 3: return threads == 512 ? flash_tc_kernel<3> : flash_step_kernel<3>;
+    default: return flash_step_kernel<0>;
   }
 }
 

@@ -27,10 +27,10 @@ __global__ void readout_tc_kernel(const __nv_bfloat16* a_hi, const __nv_bfloat16
                                   int passes, RowMap map, float* out, int32_t* status);
 size_t readout_tc_smem_bytes(int kpad, int n_tile);
 
-// flash_tc_kernel (lh_flash.cu): problem, batch, readout operator (hi, lo), k_pad,
+// flash_tc_kernel and flash_step_kernel (lh_flash.cu): problem, batch, readout operator (hi, lo), k_pad,
 // bins, tile width, MMA passes, whether the CTA sorts its pairs.
 using FlashTcKernel = void (*)(lh_flash_problem, lh_flash_batch, const __nv_bfloat16*,
                                const __nv_bfloat16*, int, int, int, int, int);
-FlashTcKernel flash_tc_kernel_of(int degrees);
+FlashTcKernel flash_tc_kernel_of(int degrees, int threads);
 
 }  // namespace lh

@@ -194,3 +194,43 @@ def test_flash_block_sizes_agree(transports, flash_golden, count):
     torch.cuda.synchronize()
     for key in ("spectrum", "components", "charge", "origin", "active"):
         assert torch.equal(out[256][key], out[512][key]), key
+
+
+@pytest.mark.parametrize("power, count", [(1, 1), (1, 301), (2, 137), (2, 700), (3, 1), (3, 295),
+                                          (3, 297), (4, 137), (8, 65), (8, 700)])
+def test_flash_degrees_block_sizes_and_runs_agree(flash_table, flash_config, power, count):
+    """Acceptances of 2 to 9 degrees, shares of less and of more than two pairs per
+    interval (from about 296 flashes on, runs of pairs share coefficients that are not
+    held): 256 and 512 threads give the same bits, and the plain path the same spectra
+    (float32 sums of up to 9 degrees in the same order: 1e-6 of a flash's largest)."""
+    from dataclasses import replace
+
+    import torch
+    from lighthit_b200.flash import FlashTransport
+    from lighthit_b200.model import synthetic_detector
+    from lighthit_b200.workloads import flash_positions
+    det = replace(synthetic_detector(),
+                  angular_acceptance=lambda x: (.5 + .5 * np.asarray(x)) ** power)
+    ft = FlashTransport(det, flash_config, flash_table, mode="split-bf16")
+    plain = FlashTransport(det, flash_config, flash_table, mode="fp32")
+    assert ft.top == power
+    pos = torch.tensor(flash_positions(count, det.positions_m.mean(axis=0), seed=count + power,
+                                       om_positions=det.positions_m), device=ft.device)
+    photons = torch.full((count,), 1e10, dtype=torch.float64, device=ft.device)
+    times = torch.linspace(0.0, 40.0, count, dtype=torch.float64, device=ft.device)
+    out = {}
+    for threads in (256, 512):
+        out[threads] = ft.allocate(count)
+        ft.launch(pos, photons, times, out[threads], block_threads=threads)
+    ref = plain.launch(pos, photons, times, plain.allocate(count))
+    torch.cuda.synchronize()
+    assert not int(out[512]["status"][0]) and not int(out[256]["status"][0])
+    for key in ("spectrum", "components", "charge", "origin", "active"):
+        assert torch.equal(out[256][key], out[512][key]), key
+    for key in ("origin", "active"):
+        assert torch.equal(out[512][key], ref[key]), key
+    largest = ref["spectrum"].abs().amax(dim=(1, 2, 3), keepdim=True)
+    assert bool(((out[512]["spectrum"] - ref["spectrum"]).abs() <= 1e-6 * largest).all())
+    bins = ref["components"].abs().amax(dim=(1, 3), keepdim=True)
+    assert bool(((out[512]["components"] - ref["components"]).abs()
+                 <= 2 * BINS_TOL["split-bf16"] * bins).all())
