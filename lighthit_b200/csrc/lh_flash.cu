@@ -275,6 +275,10 @@ LH_DEVICE void flash_tile_setup(const lh_flash_problem& p, const lh_flash_batch&
 // ---------------------------------------------------------------- plain path
 // One block per tile; readout rows go to a row-major fp32 workspace that
 // readout_fp32_kernel consumes.
+// A launch of few flashes is one chain of coefficient loads per thread: kPlainDegrees
+// degrees' loads are on their way together (one flash of 3 degrees: 42.2 us with the
+// loads of one degree at a time, 39.2 with four; 30 flashes 175 and 171).
+constexpr int kPlainDegrees = 4;
 __global__ void __launch_bounds__(kFlashThreads)
 flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins, float* a_rows) {
   __shared__ FlashPair sp[kFlashPairs];
@@ -293,8 +297,15 @@ flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins, f
     FlashPair& pair = sp[lp];
     float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f), r1, r2;
     if (pair.j >= 0)
-      for (int l = 0; l <= p.acc_top; ++l)
-        flash_degree(flash_coef(p, pair.j, l, w), pair.tt, pair.w[l], s1, s2);
+      for (int l0 = 0; l0 <= p.acc_top; l0 += kPlainDegrees) {
+        FlashCoef c[kPlainDegrees];
+#pragma unroll
+        for (int k = 0; k < kPlainDegrees; ++k)
+          if (l0 + k <= p.acc_top) c[k] = flash_coef(p, pair.j, l0 + k, w);
+#pragma unroll
+        for (int k = 0; k < kPlainDegrees; ++k)
+          if (l0 + k <= p.acc_top) flash_degree(c[k], pair.tt, pair.w[l0 + k], s1, s2);
+      }
     flash_item(p, b, w, p.omega[w], pair, s1, s2, r1, r2);
     if (base + lp < host_pairs) {
       float* row1 = a_rows + (2 * (base + lp)) * (int64_t)kpad;
