@@ -280,3 +280,29 @@ def test_many_bands_and_many_intervals_match_the_oracle(n_bands, n_intervals):
                        g["om_positions_m"][oms], g["om_looks"][oms], [1.0], g["om_area_m2"][oms],
                        g["radial_window_m"], fast=True)
     assert np.abs(out.cpu().numpy().T - ref).max() <= GE2_TOL * np.abs(ref).max()
+
+
+@pytest.mark.gpu
+def test_channel_rows_beyond_32_bit_offsets():
+    """Channels cut from a buffer whose rows lie so far apart that a point's block passes
+    4 GB: its last row is read at its own offset, not at that modulo 2^32."""
+    import torch
+    from lighthit_b200.ge2 import AxialSources, Ge2Table
+    g, _, frame = fixture()
+    t = folded_of(1, 7, 3)
+    table = Ge2Table(t, [1.0], source_degree=1, azimuthal_degree=1)
+    rng = np.random.default_rng(3)
+    values = (rng.normal(size=(1, 1, 4, 3)) + 1j * rng.normal(size=(1, 1, 4, 3))).astype(np.complex64)
+    stored = torch.empty((1, 1, 4, 180_000_000), dtype=torch.complex64, device=table.device)
+    stored[..., :3] = torch.from_numpy(values).to(table.device)
+    basis = (frame["centre"], frame["first"], frame["second"], frame["axis"])
+    pts = points(g, frame, "zero")[:1]
+    item = (AxialSources(pts, stored, np.zeros(1), basis, 1, 1), g["om_positions_m"][:1],
+            g["om_looks"][:1], g["om_area_m2"][:1], g["radial_window_m"])
+    out = table.apply_batch([item], mode="split-bf16")[0].cpu().numpy().T
+    assert table.tc_packed() is not None and int(table.status.item()) == 0
+    ref = oracle_apply(t, dict(points_m=pts, channels=values, reference_ns=np.zeros(1),
+                               frame=frame, degree=1, azimuthal_degree=1), g["om_positions_m"][:1],
+                       g["om_looks"][:1], [1.0], g["om_area_m2"][:1], g["radial_window_m"],
+                       fast=True)
+    assert np.abs(out - ref).max() <= GE2_TOL * np.abs(ref).max()
