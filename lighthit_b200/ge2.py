@@ -214,11 +214,17 @@ class Ge2Table:
         reference = float(ref.min())
         ch = sources.channels
         if not isinstance(ch, torch.Tensor):
-            ch = np.ascontiguousarray(np.asarray(ch), dtype=np.complex64)
-        else:
-            ch = ch.to(dev, torch.complex64)
+            ch = np.asarray(ch)
         if ch.shape[0] != self.n_bands or ch.shape[2] != self.nch or ch.shape[3] < W:
             raise ValueError("source channels do not match the folded kernels")
+        if not isinstance(ch, torch.Tensor):
+            # a zero-frequency problem takes only its column: 1/65 of the copies (three
+            # problems of 140 points: 2.31 ms with whole rows, TODO with the column)
+            ch = np.ascontiguousarray(ch[..., :1] if zero_frequency else ch, dtype=np.complex64)
+        else:
+            if zero_frequency and not ch.is_contiguous():
+                ch = ch[..., :1]  # copied below: the column alone
+            ch = ch.to(dev, torch.complex64)
         shift = ref - reference
         if np.any(shift != 0):  # align every band to the earliest emission reference
             if not isinstance(ch, torch.Tensor):
@@ -228,7 +234,7 @@ class Ge2Table:
                              torch.complex64, dev)
             ch = ch * ph[:, None, None, :]
         if isinstance(ch, torch.Tensor):
-            ch = ch.resolve_conj().contiguous()  # a zero-frequency problem reads the first column
+            ch = ch.resolve_conj().contiguous()  # zero frequency: a whole one is read in place
         scale = np.asarray(out_scale, float)
         if scale.ndim == 1:
             scale = np.repeat(scale[None, :], self.n_bands, axis=0)

@@ -306,3 +306,33 @@ def test_channel_rows_beyond_32_bit_offsets():
                        g["om_looks"][:1], [1.0], g["om_area_m2"][:1], g["radial_window_m"],
                        fast=True)
     assert np.abs(out - ref).max() <= GE2_TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("kind", ["host", "host slice", "contiguous", "point slice"])
+@pytest.mark.parametrize("shifted", [False, True])
+def test_zero_frequency_problems_copy_one_column(kind, shifted):
+    """What a zero-frequency problem takes of its channels: the first frequency alone
+    wherever they have to be copied (host arrays, a slice of a larger buffer, bands
+    aligned to one reference), the caller's own tensor where it is contiguous."""
+    import torch
+    from lighthit_b200.ge2 import AxialSources, Ge2Table
+    g, t, frame = fixture()
+    table = Ge2Table(t, g["alpha"], source_degree=8, azimuthal_degree=2, device="cpu")
+    rng = np.random.default_rng(12)
+    full = (rng.normal(size=(3, 9, 39, 65)) + 1j * rng.normal(size=(3, 9, 39, 65))).astype(
+        np.complex64)
+    kept = full if kind in ("host", "contiguous") else full[:, :5]
+    channels = kept if kind.startswith("host") else torch.from_numpy(full)[:, :kept.shape[1]]
+    refs = np.array([0.0, 0.2, 0.1]) if shifted else np.zeros(3)
+    src = AxialSources(points(g, frame, "zero")[:kept.shape[1]], channels, refs,
+                       (frame["centre"], frame["first"], frame["second"], frame["axis"]), 8, 2)
+    q = table._prepare(src, g["om_positions_m"], g["om_looks"], g["om_area_m2"],
+                       g["radial_window_m"], True)
+    got = q["ch"] if isinstance(q["ch"], np.ndarray) else q["ch"].numpy()
+    if kind == "contiguous" and not shifted:
+        assert q["ch"].data_ptr() == channels.data_ptr()
+    else:
+        assert got.shape[3] == 1 and got.flags.c_contiguous
+    assert q["W"] == 1
+    # at the first frequency (zero) the bands' alignment is the identity
+    assert np.array_equal(got[..., 0], kept[..., 0])
