@@ -318,6 +318,27 @@ def stream_ptr(stream):
     return C.c_void_p(stream.cuda_stream) if stream is not None else None
 
 
+def hand_over(stream, device, tensors=()):
+    """Before a launch on ``stream``: it comes after what the current stream has uploaded
+    or cleared for it, and ``tensors``, allocated on the current stream, are not used for
+    anything else while it runs. Nothing to do for the current stream itself."""
+    import torch
+    if stream is None or stream == torch.cuda.current_stream(device):
+        return
+    stream.wait_stream(torch.cuda.current_stream(device))
+    for t in tensors:
+        if t is not None:
+            t.record_stream(stream)
+
+
+def hand_back(stream, device):
+    """After a launch on ``stream``: what the current stream reads of it (a status word)
+    comes after it."""
+    import torch
+    if stream is not None:
+        torch.cuda.current_stream(device).wait_stream(stream)
+
+
 def kernel_timing(enable=True):
     """Start (clearing the record) or stop the library's kernel timing."""
     check(load().lh_kernel_timing(int(bool(enable))), "lh_kernel_timing")

@@ -205,7 +205,7 @@ class FlashTransport:
              np.zeros(F) if time_ns is None
              else np.broadcast_to(np.asarray(time_ns, float), (F,))), self.device, stream)
         out = self.allocate(F)
-        _follow_current(stream, self.device)
+        _lib.hand_over(stream, self.device)  # the outputs are cleared on the current stream
         self.launch(pos, ph, t, out, mode=mode, stream=stream)
         torch.cuda.synchronize(self.device)
         self.raise_for_status(out)
@@ -308,14 +308,6 @@ def _upload_flashes(parts, device, stream):
             for a, (lo, hi) in zip(parts, spans)]
 
 
-def _follow_current(stream, device):
-    """Outputs are allocated and cleared on the current stream: a launch on another
-    ``stream`` comes after that."""
-    import torch
-    if stream is not None:
-        stream.wait_stream(torch.cuda.current_stream(device))
-
-
 def flash_node_photons(nodes_nm, weights_nm, photons, spectral_shape):
     """``_flash_nodes`` (``transport.py:1049-1059``): photons of each flash at each
     wavelength node, ``photons * weight * shape / (weight . shape)`` ((node, flash))."""
@@ -386,10 +378,10 @@ class BroadbandFlashTransport:
         outs = []
         for ft, photons_n in zip(self.node, ph):
             outs.append(ft.allocate(F))
-            _follow_current(stream, dev)
+            _lib.hand_over(stream, dev)
             ft.launch(pos, photons_n, t, outs[-1], stream=stream)
         out = self.node[0].allocate(F)
-        _follow_current(stream, dev)
+        _lib.hand_over(stream, dev)
         out["origin"] = outs[0]["origin"]  # every node run wrote the common clock
         nd = _lib.FlashNodes()
         nd.n_nodes = len(self.node)

@@ -257,13 +257,17 @@ class SourceCompiler:
         own_status = status is None
         if own_status:
             status = torch.zeros(1, dtype=torch.int32, device=dev)
+        _lib.hand_over(stream, dev, (*arrays.values(), points, channels, n_points,
+                                     self._workspace, status))
         sp = _lib.stream_ptr(stream or torch.cuda.current_stream(dev))
         _lib.check(lib.lh_source_compile(C.byref(p), C.byref(out), self._workspace.data_ptr(),
                                          self._workspace.numel(), status.data_ptr(), sp),
                    "lh_source_compile")
         self._keep = arrays
-        if own_status and check and int(status.item()) & _lib.LH_STATUS_OVERFLOW:
-            raise ValueError("element nodes fall outside the source lattice")
+        if own_status and check:
+            _lib.hand_back(stream, dev)
+            if int(status.item()) & _lib.LH_STATUS_OVERFLOW:
+                raise ValueError("element nodes fall outside the source lattice")
         return points, channels, n_points, reference, frame
 
     def _compile_per_band(self, elements, beta, frame, *, stream, check, status):
