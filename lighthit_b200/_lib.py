@@ -289,13 +289,13 @@ def upload_parts(parts, dtype, device):
     through one pinned buffer and one asynchronous copy; returns it and the offsets."""
     import numpy as np
     import torch
-    sizes = [int(np.size(a)) for a in parts]
-    offsets = np.zeros(len(parts) + 1, np.int64)
-    offsets[1:] = np.cumsum(sizes)
-    host = torch.empty(int(offsets[-1]), dtype=dtype, pin_memory=torch.device(device).type == "cuda")
-    flat = host.numpy()
-    for a, lo, hi in zip(parts, offsets[:-1], offsets[1:]):
-        flat[lo:hi] = np.ravel(a)
+    flat = [a.ravel() if isinstance(a, np.ndarray) else np.ravel(a) for a in parts]
+    offsets = [0]
+    for a in flat:
+        offsets.append(offsets[-1] + a.size)
+    host = torch.empty(offsets[-1], dtype=dtype, pin_memory=torch.device(device).type == "cuda")
+    if flat:
+        np.concatenate(flat, out=host.numpy(), casting="unsafe")
     return host.to(device, non_blocking=True), offsets
 
 
