@@ -24,14 +24,21 @@ import numpy as np
 __all__ = ["ShowerRequest", "ShowerServer", "shower_footprint_bytes"]
 
 
+# a chord node of the source compile at its largest shape (153 channels, degree 16,
+# 8 bands: 341 float64 values), with its key and its places in the lists
+SOURCE_NODE_BYTES = 8 * (153 + 8 * 17 + 8 + 4 + 8 * 5) + 20
+
+
 def shower_footprint_bytes(n_elements, n_om):
     """Device bytes one shower holds while in flight (tables excluded): element
     copies, ring-node tables of the pencil compression (23 moments per slot),
-    pencil rows, and per-OM group tables of the grouped order 1."""
+    pencil rows, per-OM group tables of the grouped order 1, and the source
+    compile's rows of its (at most two) chord nodes per element. The compile's
+    lattice follows the shower's length, not its elements, and is not in it."""
     nodes = 192 * max(int(n_elements), 1)
     slots = 1 << int(np.ceil(np.log2(max(nodes, 4096))))
     return int(12 * 8 * n_elements + slots * 24 * 8 + nodes * 20 * 8
-               + n_om * 8192 * 27 * 8)
+               + n_om * 8192 * 27 * 8 + 2 * SOURCE_NODE_BYTES * n_elements)
 
 
 def _element_count(source):

@@ -135,3 +135,29 @@ def test_prime_refuses_once_requests_are_queued():
     gate.set()
     srv.drain(1, timeout=30)
     srv.close()
+
+
+@pytest.mark.parametrize("order", [1, 2])
+def test_footprint_grows_by_what_an_element_adds_to_the_source_compile(order):
+    """Between element counts of one ring-table size the footprint grows by at least an
+    element's copy, its ring nodes' pencil rows and what it adds to the workspace of the
+    source compile at its largest shape."""
+    import ctypes
+    from lighthit_b200 import _lib
+    from lighthit_b200.serve_shower import shower_footprint_bytes
+
+    def workspace(n):
+        P, one = _lib.SourceProblem(), ctypes.c_void_p(16)
+        for k in ("start", "direction", "length", "c0", "c2", "beta", "t0", "t1", "omega"):
+            setattr(P, k, one)
+        P.n_el, P.element_order, P.n_omega = n, order, 65
+        P.n_bands, P.degree, P.max_m, P.nch = 8, 16, 4, 153
+        P.cell_m, P.stencil_m, P.stencil_threshold_m, P.time_step_ns = 0.25, 0.2, 0.03, 0.02
+        P.n_slices, P.kmax = 30, 1300
+        return int(_lib.load().lh_source_workspace_bytes(ctypes.byref(P)))
+
+    low, high = 23000, 43000  # 2^22 < 192 x both <= 2^23
+    grown = workspace(high) - workspace(low)
+    assert grown > 0
+    assert (shower_footprint_bytes(high, 384) - shower_footprint_bytes(low, 384)
+            >= grown + (high - low) * (12 * 8 + 192 * 20 * 8))
