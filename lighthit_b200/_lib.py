@@ -304,13 +304,16 @@ def fetch(tensors):
     pinned memory asynchronously on the current stream, then the stream is
     synchronised once (instead of one blocking read per tensor)."""
     import torch
-    hosts = []
+    hosts, device = [], None
     for t in tensors:
-        h = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
-        h.copy_(t, non_blocking=True)
-        hosts.append(h)
-    if hosts:
-        torch.cuda.current_stream(tensors[0].device).synchronize()
+        if t.device.type != "cuda":  # there already
+            hosts.append(t)
+            continue
+        device = t.device
+        hosts.append(torch.empty(t.shape, dtype=t.dtype, pin_memory=True))
+        hosts[-1].copy_(t, non_blocking=True)
+    if device is not None:
+        torch.cuda.current_stream(device).synchronize()
     return [h.numpy() for h in hosts]
 
 

@@ -29,3 +29,32 @@ def test_node_photons_split_the_flash_by_weight_and_shape():
         flash_node_photons(nodes, weights, photons, lambda x: np.zeros_like(x))
     with pytest.raises(ValueError):
         flash_node_photons(nodes, weights, photons, lambda x: -np.ones_like(x))
+
+
+def test_response_of_outputs_kept_on_the_host():
+    """A batch's outputs moved to host memory give the flash's response, in arrays of
+    their own."""
+    import torch
+    from lighthit_b200.flash import FlashTransport
+    from lighthit_b200.model import synthetic_detector
+    g = np.load(GOLDEN / "flash_c1.npz")
+    ft = FlashTransport.__new__(FlashTransport)  # no device: only what a response reads
+    ft.detector, ft.wavelength_nm, ft.mode = synthetic_detector(), 450.0, "fp32"
+    ft.config = type("Config", (), dict(omega_per_ns=g["omega_per_ns"],
+                                        relative_time_edges_ns=g["edges_ns"]))()
+    D, W, B = len(ft.detector), len(g["omega_per_ns"]), len(g["edges_ns"]) - 1
+    rng = np.random.default_rng(4)
+    out = dict(spectrum=torch.from_numpy((rng.normal(size=(2, D, W, 3)) + 1j).astype(np.complex64)),
+               components=torch.from_numpy(rng.normal(size=(2, D, 3, B)).astype(np.float32)),
+               charge=torch.from_numpy(rng.normal(size=(2, D, 3))),
+               origin=torch.from_numpy(rng.normal(size=(2, D))),
+               active=torch.from_numpy(rng.integers(0, 2, (2, D)).astype(np.uint8)))
+    r = ft.response(out, 1)
+    assert np.array_equal(r.spectrum_pe, out["spectrum"][1].numpy().transpose(1, 0, 2))
+    assert np.array_equal(r.components_pe, out["components"][1].numpy().transpose(0, 2, 1))
+    assert np.array_equal(r.charge_components_pe, out["charge"][1].numpy())
+    assert np.array_equal(r.time_origin_ns, out["origin"][1].numpy())
+    assert np.array_equal(r.active, out["active"][1].numpy().astype(bool))
+    r.charge_components_pe[:] = 0
+    r.time_origin_ns[:] = 0
+    assert np.all(out["charge"][1].numpy() != 0) and np.all(out["origin"][1].numpy() != 0)
