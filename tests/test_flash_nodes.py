@@ -41,7 +41,8 @@ def test_response_of_outputs_kept_on_the_host():
     ft = FlashTransport.__new__(FlashTransport)  # no device: only what a response reads
     ft.detector, ft.wavelength_nm, ft.mode = synthetic_detector(), 450.0, "fp32"
     ft.config = type("Config", (), dict(omega_per_ns=g["omega_per_ns"],
-                                        relative_time_edges_ns=g["edges_ns"]))()
+                                        relative_time_edges_ns=g["edges_ns"],
+                                        radial_range_m=(2.0, 250.0)))()
     D, W, B = len(ft.detector), len(g["omega_per_ns"]), len(g["edges_ns"]) - 1
     rng = np.random.default_rng(4)
     out = dict(spectrum=torch.from_numpy((rng.normal(size=(2, D, W, 3)) + 1j).astype(np.complex64)),
