@@ -336,3 +336,54 @@ def test_zero_frequency_problems_copy_one_column(kind, shifted):
     assert q["W"] == 1
     # at the first frequency (zero) the bands' alignment is the identity
     assert np.array_equal(got[..., 0], kept[..., 0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("group, fill, groups", [(16, 100, 2), (16, 160, 3), (8, 50, 2), (8, 110, 3)])
+def test_tensor_core_tiles_of_several_groups(group, fill, groups):
+    """Launches of enough pairs make tiles of two and of three groups (16 pairs each, or 8
+    above azimuthal degree 2): intervals that hold every remainder of such tiles, in one
+    problem of a batch whose other problem fills the launch. Against the float64 oracle,
+    and bit for bit against the same problem alone, whose tiles are one group."""
+    from lighthit_b200.ge2 import AxialSources, Ge2Table
+    g, t, frame = fixture()
+    if group == 16:
+        degree, azimuthal, alpha = 8, 2, g["alpha"]
+    else:
+        degree, azimuthal, alpha = 4, 4, [1.0]
+        t = folded_of(3, 20, 65, degree=degree)
+    table = Ge2Table(t, alpha, source_degree=degree, azimuthal_degree=azimuthal)
+    rng = np.random.default_rng(group + fill)
+    basis = (frame["centre"], frame["first"], frame["second"], frame["axis"])
+    log_r, om = np.asarray(t["log_r"], float), g["om_positions_m"][7]
+
+    def sources(intervals):
+        step = log_r[1] - log_r[0]
+        r = np.exp(log_r[intervals] + step * rng.uniform(0.1, 0.9, len(intervals)))
+        u = rng.normal(size=(len(intervals), 3))
+        pts = om + r[:, None] * u / np.linalg.norm(u, axis=1)[:, None]
+        shape = (3, len(pts), table.nch, 65)
+        ch = (rng.normal(size=shape) + 1j * rng.normal(size=shape)).astype(np.complex64)
+        return AxialSources(pts, ch, np.zeros(3), basis, degree, azimuthal)
+
+    full = 3 * group  # pairs of a tile of three groups
+    counts = [1, group - 1, group, group + 1, 2 * group, 2 * group + 1, full - 1, full, full + 1]
+    window = (float(np.exp(log_r[0])), float(np.exp(log_r[-1])))
+    edges = sources(np.repeat(np.arange(3, 3 + len(counts)), counts))
+    filler = sources(np.full(fill, 15))
+    one, many = np.array([7]), np.full(48, 7)  # 48 OMs at one place: 48 x fill pairs
+    # a tile takes as many groups as leave every SM two work items (tile, half)
+    pairs = sum(counts) + 48 * fill
+    assert 148 * groups * group <= pairs and (groups == 3 or pairs < 148 * full)
+    items = [(s, g["om_positions_m"][k], g["om_looks"][k], g["om_area_m2"][k], window)
+             for s, k in ((edges, one), (filler, many))]
+    out = [r.cpu().numpy() for r in table.apply_batch(items, mode="split-bf16")]
+    assert table.tc_packed() is not None and int(table.status.item()) == 0
+    alone = table.apply_batch(items[:1], mode="split-bf16")[0].cpu().numpy()
+    assert np.array_equal(out[0], alone)
+    for got, (s, pos, looks, area, _) in zip(out, items):
+        ref = oracle_apply(t, dict(points_m=s.points_m, channels=s.channels,
+                                   reference_ns=np.zeros(3), frame=frame, degree=degree,
+                                   azimuthal_degree=azimuthal), pos, looks, alpha, area, window,
+                           fast=True)
+        assert np.abs(got.T - ref).max() <= GE2_TOL * np.abs(ref).max()
