@@ -325,10 +325,13 @@ def hand_over(stream, device, tensors=()):
     """Before a launch on ``stream``: it comes after what the current stream has uploaded
     or cleared for it, and ``tensors``, allocated on the current stream, are not used for
     anything else while it runs. Nothing to do for the current stream itself."""
-    import torch
-    if stream is None or stream == torch.cuda.current_stream(device):
+    if stream is None:
         return
-    stream.wait_stream(torch.cuda.current_stream(device))
+    import torch
+    current = torch.cuda.current_stream(device)
+    if stream == current:
+        return
+    stream.wait_stream(current)
     for t in tensors:
         if t is not None:
             t.record_stream(stream)
@@ -337,8 +340,8 @@ def hand_over(stream, device, tensors=()):
 def hand_back(stream, device):
     """After a launch on ``stream``: what the current stream reads of it (a status word)
     comes after it."""
-    import torch
     if stream is not None:
+        import torch
         torch.cuda.current_stream(device).wait_stream(stream)
 
 

@@ -311,8 +311,9 @@ class Ge2Table:
         if self._workspace is None or self._workspace.numel() < need:
             self._workspace = torch.empty(need, dtype=torch.uint8, device=dev)
         status = (torch.zeros(1, dtype=torch.int32, device=dev) if packed is not None else None)
-        _lib.hand_over(stream, dev, [d_geom, result, status, self._workspace, packed]
-                       + [q["ch"] for q in prepared if isinstance(q["ch"], torch.Tensor)])
+        if stream is not None:
+            _lib.hand_over(stream, dev, [d_geom, result, status, self._workspace, packed]
+                           + [q["ch"] for q in prepared if isinstance(q["ch"], torch.Tensor)])
         if packed is not None:
             _lib.check(lib.lh_ge2_apply_batch_tc(self.struct, probs, n, _lib.MODES[mode],
                                                  packed.data_ptr(), self._workspace.data_ptr(),

@@ -226,8 +226,9 @@ def order0(optics: Order0Optics, events, origins=None, edges=None, *, stream=Non
         raise ValueError("order-0 problem rejected by the device library")
     workspace = optics.workspace(need)
     b.workspace, b.workspace_bytes = workspace.data_ptr(), workspace.numel()
-    _lib.hand_over(stream, dev, (batch._flat, batch._t["offsets"], origins_t, edges_t, charge,
-                                 bins, charge_check, status, workspace))
+    if stream is not None:
+        _lib.hand_over(stream, dev, (batch._flat, batch._t["offsets"], origins_t, edges_t, charge,
+                                     bins, charge_check, status, workspace))
     s = _lib.stream_ptr(stream or torch.cuda.current_stream(dev))
     _lib.check(lib.lh_order0(optics.struct, b, s), "lh_order0")
     result = dict(charge=charge, bins=bins, status=status, charge_check=charge_check,

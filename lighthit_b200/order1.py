@@ -331,7 +331,9 @@ def pencils(tables: Order1Tables, elements, cone_cos, *, stream=None, status=Non
         table.count.zero_()  # stage A writes no count for no elements (a reused table)
     ws = tables.workspace(n_sub, 0)
     st = status if status is not None else torch.zeros(1, dtype=torch.int32, device=dev)
-    _lib.hand_over(stream, dev, (*keep.values(), ws, st, table._buffer, table.count, table.parent))
+    if stream is not None:
+        _lib.hand_over(stream, dev, (*keep.values(), ws, st, table._buffer, table.count,
+                                     table.parent))
     sp = _lib.stream_ptr(stream or torch.cuda.current_stream(dev))
     _lib.check(_lib.load().lh_order1_pencils(tables.struct, el, table.struct,
                                              table.count.data_ptr(), ws.data_ptr(), ws.numel(),
@@ -370,7 +372,8 @@ def grouped(tables: Order1Tables, table: "PencilTable", work, origins, *, n_penc
             if tables.compute_bins else None)
     ws = tables.workspace(0, len(work))
     st = status if status is not None else torch.zeros(1, dtype=torch.int32, device=dev)
-    _lib.hand_over(stream, dev, (work_t, origins_t, charge, bins, ws, st))
+    if stream is not None:
+        _lib.hand_over(stream, dev, (work_t, origins_t, charge, bins, ws, st))
     sp = _lib.stream_ptr(stream or torch.cuda.current_stream(dev))
     _lib.check(_lib.load().lh_order1_grouped(tables.struct, table.struct, n_p, count_ptr,
                                              work_t.data_ptr(), len(work), origins_t.data_ptr(),

@@ -257,8 +257,9 @@ class SourceCompiler:
         own_status = status is None
         if own_status:
             status = torch.zeros(1, dtype=torch.int32, device=dev)
-        _lib.hand_over(stream, dev, (*arrays.values(), points, channels, n_points,
-                                     self._workspace, status))
+        if stream is not None:
+            _lib.hand_over(stream, dev, (*arrays.values(), points, channels, n_points,
+                                         self._workspace, status))
         sp = _lib.stream_ptr(stream or torch.cuda.current_stream(dev))
         _lib.check(lib.lh_source_compile(C.byref(p), C.byref(out), self._workspace.data_ptr(),
                                          self._workspace.numel(), status.data_ptr(), sp),
