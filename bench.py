@@ -58,10 +58,10 @@ MAX_BATCH = 8
 N_FLASH = 4096
 # DRAM bytes (read + write) of one 4096-flash flash_tc_kernel launch, measured with
 # ncu on a B200 (profiles/flash_tc_kernel_4096flashes.txt).
-FLASH_TC_TRAFFIC = 636_147_456
-# DRAM bytes of one o1_group_kernel launch per (OM, pencil) evaluation, from the
-# ncu capture of profiles/order1_kernels_16showers_c2.txt (296 MB for 9472 x 256
-# threads over (OM, pencil) items), or None when not captured.
+FLASH_TC_TRAFFIC = 648_097_024
+# DRAM bytes of one o1_group_kernel launch per (OM, pencil) evaluation, or None: a
+# launch reads its pencils once (26-28 MB, profiles/order1_kernels_4showers_c2.txt)
+# whatever the number of OMs.
 O1_GROUP_TRAFFIC_PER_ITEM = None
 PENCIL_BYTES = 20 * 8  # one float64 pencil record read per (OM, pencil) evaluation
 

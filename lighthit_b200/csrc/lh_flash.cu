@@ -16,8 +16,8 @@
 //     the demodulated (relative) spectrum of orders 1 and 2 as readout rows;
 //  3. readout of the rows (see lh_readout.cu) and the order-0 bin rows,
 //     charge (spectrum at the first frequency) and the active mask.
-// flash_tc_kernel fuses 1-3 in one persistent kernel: the readout rows are
-// written straight into shared memory as the tensor-core A tile.
+// flash_tc_kernel and flash_step_kernel fuse 1-3 in one persistent kernel: the readout
+// rows are written straight into shared memory as the tensor-core A tile.
 #include "lh_common.cuh"
 #include "lh_readout.cuh"
 
@@ -26,7 +26,7 @@ namespace lh {
 constexpr int kFlashPairs = 64;  // pairs per tile -> 128 readout rows
 constexpr int kMaxAcc = 8;       // highest acceptance degree handled
 constexpr int kFlashThreads = 256;    // plain path
-constexpr int kFlashTcThreads = 512;  // fused path: 11 warps of spectra, 4 of drain, 1 of MMAs
+constexpr int kFlashTcThreads = 512;  // fused path; with roles 11 warps of spectra, 4 of drain, 1 of MMAs
 // A tile of the fused path: K-major, no swizzle, [k/8][row][k%8] with each
 // 8-column chunk of the 128 rows padded by 16 bytes (2064 B apart, the MMA's
 // leading byte offset). A warp stores 32 consecutive columns of one row: the

@@ -52,7 +52,7 @@ constexpr int kO0Threads = 256;
 constexpr int kO0MaxOrder = 64;
 constexpr int kO0MaxPanels = 128;
 constexpr int kO0MaxSCuts = 64;
-constexpr int kO0MaxPhiCuts = 32;
+constexpr int kO0MaxPhiCuts = 32;  // more cuts are refused (LH_STATUS_OVERFLOW), as the header says
 constexpr int kO0MaxAlpha = 8;
 
 struct O0Pair {
