@@ -349,7 +349,6 @@ flash_plain_kernel(lh_flash_problem p, lh_flash_batch b, int kpad, int n_bins, f
 // 0.148). One flash: 21.8 us on one SM, now 13.9 on 48. 137 flashes: 25.4, now 22.2.
 constexpr int kFlashSort = 2048;        // pairs sorted at a time
 constexpr int kFlashMaxBuckets = 1024;  // radial intervals the sort tells apart
-constexpr int kFlashRun = 4;            // pairs that share coefficients not held
 constexpr int kFlashDense = 2;          // pairs per interval from which runs share them
 
 // The pair's radial interval for the sort, in float32: where it is off by one the
@@ -386,9 +385,9 @@ LH_DEVICE void flash_rows(const lh_flash_problem& p, const lh_flash_batch& b, in
 }
 
 // A tile's spectra, written as A rows (order 1, order 2 of each pair), by the first
-// `team` threads: thread (group of pairs, frequency). kDegrees: acceptance degrees whose
-// coefficients a thread holds, reading them again where the interval changes (0: any
-// number, read for every pair).
+// `team` threads, each one frequency of a range of pairs. kDegrees: acceptance degrees
+// whose coefficients a thread holds, reading them again where the interval changes (0:
+// any number, read for every pair).
 template <int kDegrees>
 LH_DEVICE void flash_tile_spectra(const lh_flash_problem& p, const lh_flash_batch& b,
                                   FlashPair* sp, __nv_bfloat16* s_ahi, __nv_bfloat16* s_alo,
@@ -424,23 +423,26 @@ LH_DEVICE void flash_tile_spectra(const lh_flash_problem& p, const lh_flash_batc
   }
 }
 
-// The same by runs of kFlashRun neighbouring pairs and one frequency: a degree's
-// coefficients are read once for the run's pairs of one interval.
+// The same for any number of degrees, by runs of kRun neighbouring pairs and one
+// frequency: a degree's coefficients are read once for the run's pairs of one interval.
+template <int kRun>
 LH_DEVICE void flash_tile_runs(const lh_flash_problem& p, const lh_flash_batch& b, FlashPair* sp,
                                __nv_bfloat16* s_ahi, __nv_bfloat16* s_alo, int count, int team) {
-  const int nw = p.n_omega, runs = (count + kFlashRun - 1) / kFlashRun;
+  const int nw = p.n_omega, runs = (count + kRun - 1) / kRun;
   for (int i = threadIdx.x; i < runs * nw; i += team) {
     const int run = i / nw, w = i - run * nw;
-    FlashPair* q = sp + run * kFlashRun;  // slots past the count hold no pair
-    float2 s1[kFlashRun], s2[kFlashRun];
+    FlashPair* q = sp + run * kRun;
+    // slots past the count hold no pair; only with a run of 3 may they pass the tile's 64
+    const int n = kFlashPairs % kRun ? min(kRun, kFlashPairs - run * kRun) : kRun;
+    float2 s1[kRun], s2[kRun];
 #pragma unroll
-    for (int k = 0; k < kFlashRun; ++k) s1[k] = s2[k] = make_float2(0.f, 0.f);
+    for (int k = 0; k < kRun; ++k) s1[k] = s2[k] = make_float2(0.f, 0.f);
     for (int l = 0; l <= p.acc_top; ++l) {
       FlashCoef c;
       int j_held = -1;
 #pragma unroll
-      for (int k = 0; k < kFlashRun; ++k) {
-        if (q[k].j < 0) continue;
+      for (int k = 0; k < kRun; ++k) {
+        if (k >= n || q[k].j < 0) continue;
         if (q[k].j != j_held) {
           j_held = q[k].j;
           c = flash_coef(p, j_held, l, w);
@@ -450,8 +452,8 @@ LH_DEVICE void flash_tile_runs(const lh_flash_problem& p, const lh_flash_batch& 
     }
     const double om = p.omega[w];
 #pragma unroll
-    for (int k = 0; k < kFlashRun; ++k)
-      flash_rows(p, b, w, om, q[k], s1[k], s2[k], run * kFlashRun + k, s_ahi, s_alo);
+    for (int k = 0; k < kRun; ++k)
+      if (k < n) flash_rows(p, b, w, om, q[k], s1[k], s2[k], run * kRun + k, s_ahi, s_alo);
   }
 }
 
@@ -762,11 +764,13 @@ flash_tc_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __res
 //    of 48 OMs with 3 degrees take 0.339 ms against 0.507 (2: 0.305, 0.490), 137 flashes
 //    25.6 us against 36.3;
 //  * degrees that are not held, whose spectra outweigh the drains: 4000 flashes with 5
-//    degrees take 0.391 ms against 0.466 (9: 0.528, 0.673), with 256 threads 0.511 against
-//    1.25; 137 flashes with 4 degrees 26.3 us against 28.5.
-// Degrees not held are read once per run of pairs where an interval has two pairs or
-// more on average (700 flashes, 5 degrees: 84.9 us against 89.2 read for every pair; 137,
-// one pair per interval, the other way round: 34 against 29).
+//    degrees take 0.392 ms against 0.466 (9: 0.525, 0.673), with 256 threads 0.513 against
+//    1.25; 137 flashes with 4 degrees 26.4 us against 28.4.
+// Degrees not held are read for every pair, or once per run of pairs where an interval
+// has kFlashDense pairs or more on average: with 5 degrees and 512 threads 29.1 against
+// 31.1 us at one pair per interval (137 flashes), 46.0 and 45.7 at two (300), 89.4 and
+// 81.9 at 4.7 (700). Runs of 3 make three rounds of 480 threads over a tile, runs of 4 five
+// of 224: the fewest (512 threads with runs of 4: 84.8).
 template <int kDegrees>
 __global__ void __launch_bounds__(kFlashTcThreads, 1)
 flash_step_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __restrict__ g_bhi,
@@ -830,10 +834,12 @@ flash_step_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __r
           for (int k = lane; k < kFlashPairs; k += 32)
             flash_slot_setup(p, b, S.pairs[((tile + 1) & 1) * kFlashPairs + k],
                              pair_at((tile + 1) * kFlashPairs + k), n_pairs);
-      } else if (kDegrees == 0 && dense) {
-        flash_tile_runs(p, b, sp, S.ahi, S.alo, count, workers);
-      } else {
+      } else if (kDegrees > 0 || !dense) {
         flash_tile_spectra<kDegrees>(p, b, sp, S.ahi, S.alo, count, workers);
+      } else if (workers >= 256) {
+        flash_tile_runs<3>(p, b, sp, S.ahi, S.alo, count, workers);
+      } else {
+        flash_tile_runs<4>(p, b, sp, S.ahi, S.alo, count, workers);
       }
       fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core
       __syncthreads();
