@@ -385,15 +385,15 @@ LH_DEVICE void flash_rows(const lh_flash_problem& p, const lh_flash_batch& b, in
 }
 
 // A tile's spectra, written as A rows (order 1, order 2 of each pair), by the first
-// `team` threads, each one frequency of a range of pairs. kDegrees: acceptance degrees
+// `team` threads, each one frequency of a range of pairs: the thread's `group` of the
+// `groups` that the team makes (formed once per launch). kDegrees: acceptance degrees
 // whose coefficients a thread holds, reading them again where the interval changes (0:
 // any number, read for every pair).
 template <int kDegrees>
 LH_DEVICE void flash_tile_spectra(const lh_flash_problem& p, const lh_flash_batch& b,
                                   FlashPair* sp, __nv_bfloat16* s_ahi, __nv_bfloat16* s_alo,
-                                  int count, int team) {
+                                  int count, int team, int groups, int group) {
   const int tid = threadIdx.x, nw = p.n_omega;
-  const int groups = max(1, team / nw), group = tid / nw;
   if (group >= groups) return;
   const int first = group * count / groups, last = (group + 1) * count / groups;
   for (int w = tid - group * nw; w < nw; w += team) {
@@ -463,7 +463,8 @@ LH_DEVICE void flash_spectra(const lh_flash_problem& p, const lh_flash_batch& b,
                              FlashPair* sp_buf, __nv_bfloat16* s_ahi, __nv_bfloat16* s_alo,
                              uint64_t* bar_pairs, uint64_t* bar_a, uint64_t* bar_mma, int workers,
                              int n_bins, int in_chunk, int64_t tiles_before, bool& failed) {
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, nw = p.n_omega;
+  const int groups = max(1, workers / nw), group = tid / nw;
   const int tiles = (in_chunk + kFlashPairs - 1) / kFlashPairs;
   for (int tile = 0; tile < tiles; ++tile) {
     const int64_t at = tiles_before + tile;
@@ -476,7 +477,7 @@ LH_DEVICE void flash_spectra(const lh_flash_problem& p, const lh_flash_batch& b,
       failed = true;
       return;
     }
-    flash_tile_spectra<kDegrees>(p, b, sp, s_ahi, s_alo, count, workers);
+    flash_tile_spectra<kDegrees>(p, b, sp, s_ahi, s_alo, count, workers, groups, group);
     fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core
     __syncwarp();
     if ((tid & 31) == 0) mbar_arrive(bar_a + (at & 1));
@@ -814,6 +815,7 @@ flash_step_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __r
   // split the 16-column pieces between them
   const int pieces = (n_tile / 16 + (int)blockDim.x / 128 - 1) / ((int)blockDim.x / 128) * 16;
   const int c_begin = min((warp >> 2) * pieces, n_tile), c_end = min(c_begin + pieces, n_tile);
+  const int groups = max(1, workers / p.n_omega), group = tid / p.n_omega;
   bool b_ready = false, failed = false, issued = false;
   uint32_t phase = 0;  // of the accumulator: one tile each
   for (int64_t chunk = share_begin; chunk < share_end && !failed; chunk += kFlashSort) {
@@ -835,7 +837,7 @@ flash_step_kernel(lh_flash_problem p, lh_flash_batch b, const __nv_bfloat16* __r
             flash_slot_setup(p, b, S.pairs[((tile + 1) & 1) * kFlashPairs + k],
                              pair_at((tile + 1) * kFlashPairs + k), n_pairs);
       } else if (kDegrees > 0 || !dense) {
-        flash_tile_spectra<kDegrees>(p, b, sp, S.ahi, S.alo, count, workers);
+        flash_tile_spectra<kDegrees>(p, b, sp, S.ahi, S.alo, count, workers, groups, group);
       } else if (workers >= 256) {
         flash_tile_runs<3>(p, b, sp, S.ahi, S.alo, count, workers);
       } else {
